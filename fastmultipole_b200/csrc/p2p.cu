@@ -198,44 +198,47 @@ __device__ __forceinline__ int chan_row(int a) {
   return KIND == FMM_POINT_SOURCE ? a : (GS ? a + 1 : a + 4);
 }
 
-// one source body (x, y, z, s0, s1, s2) on one target; same arithmetic as interact()
-template <class R, int KIND, bool PS, bool GS, bool HS, int NA>
-__device__ __forceinline__ void pair1(R tx, R ty, R tz, R sx, R sy, R sz, R s0, R s1, R s2, R (&a)[NA]) {
-  R dx = tx - sx, dy = ty - sy, dz = tz - sz;
-  R r2 = dx * dx + dy * dy + dz * dz;
-  if (r2 > R(0)) {
-    R rinv = rsq(r2);
-    if (KIND == FMM_POINT_SOURCE) {
-      R qr = s0 * rinv;
-      if (PS) a[0] += qr;
-      R q3 = qr * rinv * rinv;
-      a[1] += dx * q3;
-      a[2] += dy * q3;
-      a[3] += dz * q3;
-    } else {
-      R rinv2 = rinv * rinv;
-      R den = rinv * rinv2;
-      constexpr int h = GS ? 3 : 0;
-      if (GS) {
-        a[0] += (dz * s1 - dy * s2) * den;
-        a[1] += (dx * s2 - dz * s0) * den;
-        a[2] += (dy * s0 - dx * s1) * den;
-      }
-      if (HS) {
-        R d5 = den * rinv2;
-        R cx = s1 * dz - s2 * dy, cy = s2 * dx - s0 * dz, cz = s0 * dy - s1 * dx;
-        a[(h + 0) % NA] += R(-3) * dx * cx * d5;
-        a[(h + 1) % NA] += (R(-3) * dx * cy + s2 * r2) * d5;
-        a[(h + 2) % NA] += (R(-3) * dx * cz - s1 * r2) * d5;
-        a[(h + 3) % NA] += (R(-3) * dy * cx - s2 * r2) * d5;
-        a[(h + 4) % NA] += R(-3) * dy * cy * d5;
-        a[(h + 5) % NA] += (R(-3) * dy * cz + s0 * r2) * d5;
-        a[(h + 6) % NA] += (R(-3) * dz * cx + s1 * r2) * d5;
-        a[(h + 7) % NA] += (R(-3) * dz * cy - s0 * r2) * d5;
-        a[(h + 8) % NA] += R(-3) * dz * cz * d5;
-      }
-    }
-  }
+// r^-3 of an FP64 pair without a call, a branch or a special case.  y, about r^-1, is the SFU's
+// approximation (rsqrt.approx.ftz.f64) with its low word cleared, so that u = y^2 is exact; with
+// e = 1 - r^2 u (|e| below 2^-18) the binomial series of (1 - e)^(-3/2) and (1 - e)^-1
+//   r^-3 = y^3 (1 + 3/2 e + 15/8 e^2 + 35/16 e^3 ...),  r^-2 = u (1 + e + e^2 + e^3 ...)
+// are cut after e^2, below the rounding of a double.  r^2 = 0 gives y = 0 and all products
+// zero, which skips the pair as the reference does.  Outside the range where y^3 and the
+// products are normal numbers the sums come out non-finite or the caller must not get here
+// (kFarHi): such batches take the general arithmetic (self_batch_f64_*).
+struct InvR {
+  double u, e, r3;  // y^2, 1 - r^2 y^2, q r^-3 (q the factor given)
+};
+__device__ __forceinline__ InvR inv_r3(double r2, double q) {
+  double y;
+  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(r2));
+  const int nz = __double2hiint(r2) | __double2loint(r2);
+  y = __hiloint2double(nz ? __double2hiint(y) : 0, 0);
+  InvR v;
+  v.u = y * y;
+  v.e = fma(-r2, v.u, 1.0);
+  const double h = v.e * fma(v.e, 1.875, 1.5);
+  const double w = (q * y) * v.u;
+  v.r3 = fma(w, h, w);
+  return v;
+}
+
+// bodies with a coordinate of at least 2^160 (high word of the double) take the general
+// arithmetic: r^-5 and the products with it stay normal numbers below
+constexpr int kFarHi = (1023 + 160) << 20;
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// one source body on one target, Laplace, 17 FP64 operations: phi = (q / r^3) r^2
+template <bool PS>
+__device__ __forceinline__ void source_pair_f64(double tx, double ty, double tz, double sx, double sy, double sz,
+                                                double q, double (&a)[4]) {
+  const double dx = tx - sx, dy = ty - sy, dz = tz - sz;
+  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  const double q3 = inv_r3(r2, q).r3;
+  if (PS) a[0] = fma(q3, r2, a[0]);
+  a[1] = fma(dx, q3, a[1]);
+  a[2] = fma(dy, q3, a[2]);
+  a[3] = fma(dz, q3, a[3]);
 }
 
 // One lane's slice of a packed batch on its two targets.  GUARD skips pairs with
@@ -317,6 +320,39 @@ __device__ __forceinline__ void vortex_grad_from_qe(const R (&Q)[9], const R (&E
   g[6] = R(-3) * Q[6] + E[1];
   g[7] = R(-3) * Q[7] - E[0];
   g[8] = R(-3) * Q[8];
+}
+
+// the same sums without the special cases (inv_r3), 38 FP64 operations with both outputs: the
+// gradient is trace-free (d . (G x d) = 0 for every pair), so Q_zz is formed at the end as
+// -(Q_xx + Q_yy)
+template <bool GS, bool HS>
+__device__ __forceinline__ void vortex_pair_f64(double tx, double ty, double tz, double sx, double sy, double sz,
+                                                double s0, double s1, double s2, double (&u)[3], double (&Q)[9],
+                                                double (&E)[3]) {
+  const double dx = tx - sx, dy = ty - sy, dz = tz - sz;
+  const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+  const InvR v = inv_r3(r2, 1.0);
+  const double cx = fma(s1, dz, -(s2 * dy)), cy = fma(s2, dx, -(s0 * dz)), cz = fma(s0, dy, -(s1 * dx));
+  if (GS) {
+    u[0] = fma(cx, v.r3, u[0]);
+    u[1] = fma(cy, v.r3, u[1]);
+    u[2] = fma(cz, v.r3, u[2]);
+  }
+  if (HS) {
+    const double d5 = v.r3 * fma(v.u, fma(v.e, v.e, v.e), v.u);
+    const double px = dx * d5, py = dy * d5, pz = dz * d5;
+    Q[0] = fma(px, cx, Q[0]);
+    Q[1] = fma(px, cy, Q[1]);
+    Q[2] = fma(px, cz, Q[2]);
+    Q[3] = fma(py, cx, Q[3]);
+    Q[4] = fma(py, cy, Q[4]);
+    Q[5] = fma(py, cz, Q[5]);
+    Q[6] = fma(pz, cx, Q[6]);
+    Q[7] = fma(pz, cy, Q[7]);
+    E[0] = fma(s0, v.r3, E[0]);
+    E[1] = fma(s1, v.r3, E[1]);
+    E[2] = fma(s2, v.r3, E[2]);
+  }
 }
 
 // f32x2 with both halves negated
@@ -482,11 +518,12 @@ __device__ __noinline__ void self_batch_f64_vortex(const double2* __restrict__ B
 // W warps per CTA: kWarps, or kWideWarps for launches of few rows (one long row per CTA).
 // resident CTAs of the mixed instances: the registers the packed loop needs (the FP64
 // branch of the batch holding the target's own leaf is a call, and must not raise them);
-// the FP64 vortex CTA path keeps 128 registers (4 CTAs per SM)
+// the FP64 vortex CTA path takes 168 registers (3 CTAs per SM; 300k ring, order 12, whole solve:
+// 28.6 ms, 28.8 with 2 CTAs, and 49.3 with 4, whose 128 registers spill inside the loop)
 template <class R, int KIND, bool HS, bool RW, int W>
 __host__ __device__ constexpr int p2p_min_blocks() {
   constexpr int regs = (KIND == FMM_POINT_VORTEX && HS) ? (RW ? 168 : 128) : (RW ? 72 : 64);
-  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW && W == kWarps) ? 4 : 1;
+  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW && W == kWarps) ? 3 : 1;
   return 65536 / (regs * W * 32) > 0 ? 65536 / (regs * W * 32) : 1;
 }
 
@@ -502,18 +539,17 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
                                                      int exact_self) {
   // chunks (CTA path only; may be null): CTA b takes the source leaves [y, z) of row x and stores
   // its sums (unscaled, not atomically) at chunk_sums + w + NA * (target index in the row) + channel
-  constexpr int NB = batch_bodies<R, KIND>(), NV = Batch<KIND>::nv, NA = n_chan<KIND, GS, HS>();
+  constexpr int NB = batch_bodies<R, KIND>(), NA = n_chan<KIND, GS, HS>();
   constexpr int NS = slots_per_body<R, KIND>();
   constexpr bool MIXED = sizeof(R) == 4;
   constexpr bool PACK = packed<R, KIND>();
   constexpr bool PACKV = packed_vortex<R, KIND>();
-  // unpacked vortex particles with the gradient (the FP64 path) sum it as two parts per target
-  constexpr bool QE = !PACKV && KIND == FMM_POINT_VORTEX && HS;
-  static_assert(!QE || !MIXED, "the mixed vortex path is the packed one");
+  // vortex particles with the gradient on the FP64 path sum it as two parts per target
+  constexpr bool QE = !MIXED && KIND == FMM_POINT_VORTEX && HS;
   static_assert((!PACK && !PACKV) || kTPT == 2, "packed paths pair two targets per lane");
   extern __shared__ __align__(16) unsigned char p2p_smem[];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  R* B = reinterpret_cast<R*>(p2p_smem) + w * NS * NB;  // this warp's batch, plane v at B[v * NB]
+  R* B = reinterpret_cast<R*>(p2p_smem) + w * NS * NB;  // this warp's batch, NS values per body
   double* red = reinterpret_cast<double*>(p2p_smem + W * NS * NB * sizeof(R));  // [W][32 kTPT][NA]
   constexpr bool CH = !RW && W > kWarps;  // only the wide instances take chunks
   const bool chunked = CH && chunks != nullptr;
@@ -568,12 +604,14 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
     while (TS * kTPT < nt) TS <<= 1;
     const int ti = lane & (TS - 1), slice = lane / TS, SS = 32 / TS;
     R tx[kTPT], ty[kTPT], tz[kTPT];
+    int tfar = 0;  // FP64: largest high word of the lane's target coordinates
 #pragma unroll
     for (int k = 0; k < kTPT; ++k) {
       tx[k] = ty[k] = tz[k] = R(0);
       int i = ti + k * TS;
       if (i < nt) {
         double4 p = tpos[ts + tile + i];
+        tfar = max(tfar, max(hi_abs(p.x), max(hi_abs(p.y), hi_abs(p.z))));
         tx[k] = (R)(p.x - ox);
         ty[k] = (R)(p.y - oy);
         tz[k] = (R)(p.z - oz);
@@ -581,209 +619,234 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
     }
     R part[kTPT][NA];
     double tot[kTPT][NA];
+    R us[kTPT][3], Qs[kTPT][9], Es[kTPT][3];  // FP64 vortex particles: velocity, gradient as two sums
+    // FP64: a second pass in the general arithmetic when the first meets a pair out of its range
+    for (bool general = false;; general = true) {
 #pragma unroll
-    for (int k = 0; k < kTPT; ++k)
+      for (int k = 0; k < kTPT; ++k) {
 #pragma unroll
-      for (int a = 0; a < NA; ++a) part[k][a] = R(0), tot[k][a] = 0.0;
-    R Qs[kTPT][9], Es[kTPT][3];  // FP64 vortex gradient as two sums (QE)
+        for (int a = 0; a < NA; ++a) part[k][a] = R(0), tot[k][a] = 0.0;
 #pragma unroll
-    for (int k = 0; k < kTPT; ++k) {
+        for (int a = 0; a < 9; ++a) Qs[k][a] = R(0);
 #pragma unroll
-      for (int a = 0; a < 9; ++a) Qs[k][a] = R(0);
-      Es[k][0] = Es[k][1] = Es[k][2] = R(0);
-    }
-    // next source leaf of this warp, bodies of it already taken, bodies of the range still to take
-    int lb = lb0, poff = poff0, rem = rem0;
-    while (lb < l1 && rem > 0) {
-      // candidate leaves lb + LS * lane; take the longest prefix that fits the batch and the range
-      const int l = lb + LS * lane;
-      int cnt = 0, sb = 0, sl = -1;
-      if (l < l1) {
-        sl = src_of[l];
-        sb = s_start[sl];
-        cnt = s_count[sl];
+        for (int a = 0; a < 3; ++a) us[k][a] = Es[k][a] = R(0);
       }
-      if (lane == 0) {
-        sb += poff;
-        cnt -= poff;
-      }
-      int incl = cnt;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int v = __shfl_up_sync(kAll, incl, o);
-        if (lane >= o) incl += v;
-      }
-      const int excl = incl - cnt;
-      const int lim = min(NB, rem);
-      int nl = __popc(__ballot_sync(kAll, l < l1 && incl <= lim));
-      int nb;
-      if (nl == 0) {  // the first leaf alone overflows the batch or ends the range: lim bodies of it
-        nl = 1;
-        nb = lim;
-        poff += lim;
-      } else {
-        nb = __shfl_sync(kAll, incl, nl - 1);
-        lb += LS * nl;
-        poff = 0;
-      }
-      rem -= nb;
-      // the batch holds the target branch's own bodies (coincident pairs certain)
-      const bool self_batch = __any_sync(kAll, lane < nl && sl == t);
-      // mixed path: that batch in FP64 (the solve's own near field; the influence estimate, which
-      // only needs the magnitude of the field, keeps it in FP32 with the r^2 > 0 guard)
-      // (vortex ring 2e6, p = 12: velocity error 8e-8 against 9e-7 with that batch in FP32, at the
-      // same speed)
-      const bool self_f64 = self_batch && exact_self != 0;
-      // gather: body idx of the batch lies in candidate leaf k (largest k < nl with excl_k <= idx)
-      for (int i0 = 0; i0 < nb; i0 += 32) {
-        const int idx = i0 + lane;
-        int k = 0;
-#pragma unroll
-        for (int step = 16; step > 0; step >>= 1) {
-          int c = k + step;
-          int e = __shfl_sync(kAll, excl, c & 31);
-          if (c < nl && e <= idx) k = c;
+      // next source leaf of this warp, bodies of it already taken, bodies of the range still to take
+      int lb = lb0, poff = poff0, rem = rem0;
+      while (lb < l1 && rem > 0) {
+        // candidate leaves lb + LS * lane; take the longest prefix that fits the batch and the range
+        const int l = lb + LS * lane;
+        int cnt = 0, sb = 0, sl = -1;
+        if (l < l1) {
+          sl = src_of[l];
+          sb = s_start[sl];
+          cnt = s_count[sl];
         }
-        const int ek = __shfl_sync(kAll, excl, k);
-        const int sk = __shfl_sync(kAll, sb, k);
-        if ((PACK || PACKV) && self_f64 && idx < nb) {
-          // FP64 (x, y, z, q) / (x, y, z, G0), (G1, G2, -, -) relative to the target leaf centre
-          const int body = sk + idx - ek;
-          const double4 p = spos[body];
-          const double4 g = sstr[body];
-          if (PACK) {
-            reinterpret_cast<double4*>(B)[idx] = make_double4(p.x - ox, p.y - oy, p.z - oz, g.x);
-          } else {  // 48 bytes per body, the size of the packed FP32 record
-            double2* Bd = reinterpret_cast<double2*>(B) + 3 * idx;
-            Bd[0] = make_double2(p.x - ox, p.y - oy);
-            Bd[1] = make_double2(p.z - oz, g.x);
-            Bd[2] = make_double2(g.y, g.z);
-          }
-        } else if (PACK && idx < nb) {
-          const int body = sk + idx - ek;
-          const double4 p = spos[body];
-          const float x = -(float)(p.x - ox), y = -(float)(p.y - oy), z = -(float)(p.z - oz), q = (float)sstr[body].x;
-          float4* B4 = reinterpret_cast<float4*>(B);
-          B4[2 * idx] = make_float4(x, x, y, y);
-          B4[2 * idx + 1] = make_float4(z, z, q, q);
-        } else if (PACKV && idx < nb) {
-          const int body = sk + idx - ek;
-          const double4 p = spos[body];
-          const double4 g = sstr[body];
-          const float x = -(float)(p.x - ox), y = -(float)(p.y - oy), z = -(float)(p.z - oz);
-          const float g0 = (float)g.x, g1 = (float)g.y, g2 = (float)g.z;
-          float4* B4 = reinterpret_cast<float4*>(B);
-          B4[3 * idx] = make_float4(x, x, y, y);
-          B4[3 * idx + 1] = make_float4(z, z, g0, g0);
-          B4[3 * idx + 2] = make_float4(g1, g1, g2, g2);
-        } else if (idx < nb) {
-          const int body = sk + idx - ek;
-          double4 p = spos[body];
-          double4 q = sstr[body];
-          B[idx] = (R)(p.x - ox);
-          B[NB + idx] = (R)(p.y - oy);
-          B[2 * NB + idx] = (R)(p.z - oz);
-          B[3 * NB + idx] = (R)q.x;
-          if (NV == 6) {
-            B[(4 % NV) * NB + idx] = (R)q.y;
-            B[(5 % NV) * NB + idx] = (R)q.z;
-          }
+        if (lane == 0) {
+          sb += poff;
+          cnt -= poff;
         }
-      }
-      __syncwarp();
-      if constexpr (PACK) {
-        // targets 0 and 1 of the lane in the two halves of every f32x2 operation
-        const float4* B4 = reinterpret_cast<const float4*>(B);
-        const float2 tx2 = make_float2((float)tx[0], (float)tx[1]);
-        const float2 ty2 = make_float2((float)ty[0], (float)ty[1]);
-        const float2 tz2 = make_float2((float)tz[0], (float)tz[1]);
-        float2 ph = make_float2(0.f, 0.f), gx = ph, gy = ph, gz = ph;
-        // the batch holding the target's own leaf runs in FP64 and skips coincident bodies;
-        // the others run unguarded and, in the rare case that their sums come out non-finite
-        // (bodies that coincide in FP32), repeat the batch with the r^2 > 0 guard
-        if (self_f64) {
-          double txd[2], tyd[2], tzd[2];
-          self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
-          self_batch_f64_source<PS, NA>(reinterpret_cast<const double4*>(B), slice, nb, SS, txd, tyd, tzd, tot);
-        } else if (self_batch) {
-          packed_batch<true, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+        int incl = cnt;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          int v = __shfl_up_sync(kAll, incl, o);
+          if (lane >= o) incl += v;
+        }
+        const int excl = incl - cnt;
+        const int lim = min(NB, rem);
+        int nl = __popc(__ballot_sync(kAll, l < l1 && incl <= lim));
+        int nb;
+        if (nl == 0) {  // the first leaf alone overflows the batch or ends the range: lim bodies of it
+          nl = 1;
+          nb = lim;
+          poff += lim;
         } else {
-          packed_batch<false, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
-          if (!isfinite(ph.x + ph.y + gx.x + gx.y + gy.x + gy.y + gz.x + gz.y)) {
-            ph = gx = gy = gz = make_float2(0.f, 0.f);
+          nb = __shfl_sync(kAll, incl, nl - 1);
+          lb += LS * nl;
+          poff = 0;
+        }
+        rem -= nb;
+        // the batch holds the target branch's own bodies (coincident pairs certain)
+        const bool self_batch = __any_sync(kAll, lane < nl && sl == t);
+        // mixed path: that batch in FP64 (the solve's own near field; the influence estimate, which
+        // only needs the magnitude of the field, keeps it in FP32 with the r^2 > 0 guard)
+        // (vortex ring 2e6, p = 12: velocity error 8e-8 against 9e-7 with that batch in FP32, at the
+        // same speed)
+        const bool self_f64 = self_batch && exact_self != 0;
+        int far = 0;  // FP64: largest high word of the coordinates
+        // gather: body idx of the batch lies in candidate leaf k (largest k < nl with excl_k <= idx)
+        for (int i0 = 0; i0 < nb; i0 += 32) {
+          const int idx = i0 + lane;
+          int k = 0;
+#pragma unroll
+          for (int step = 16; step > 0; step >>= 1) {
+            int c = k + step;
+            int e = __shfl_sync(kAll, excl, c & 31);
+            if (c < nl && e <= idx) k = c;
+          }
+          const int ek = __shfl_sync(kAll, excl, k);
+          const int sk = __shfl_sync(kAll, sb, k);
+          if ((PACK || PACKV) && self_f64 && idx < nb) {
+            // FP64 (x, y, z, q) / (x, y, z, G0), (G1, G2, -, -) relative to the target leaf centre
+            const int body = sk + idx - ek;
+            const double4 p = spos[body];
+            const double4 g = sstr[body];
+            if (PACK) {
+              reinterpret_cast<double4*>(B)[idx] = make_double4(p.x - ox, p.y - oy, p.z - oz, g.x);
+            } else {  // 48 bytes per body, the size of the packed FP32 record
+              double2* Bd = reinterpret_cast<double2*>(B) + 3 * idx;
+              Bd[0] = make_double2(p.x - ox, p.y - oy);
+              Bd[1] = make_double2(p.z - oz, g.x);
+              Bd[2] = make_double2(g.y, g.z);
+            }
+          } else if (PACK && idx < nb) {
+            const int body = sk + idx - ek;
+            const double4 p = spos[body];
+            const float x = -(float)(p.x - ox), y = -(float)(p.y - oy), z = -(float)(p.z - oz), q = (float)sstr[body].x;
+            float4* B4 = reinterpret_cast<float4*>(B);
+            B4[2 * idx] = make_float4(x, x, y, y);
+            B4[2 * idx + 1] = make_float4(z, z, q, q);
+          } else if (PACKV && idx < nb) {
+            const int body = sk + idx - ek;
+            const double4 p = spos[body];
+            const double4 g = sstr[body];
+            const float x = -(float)(p.x - ox), y = -(float)(p.y - oy), z = -(float)(p.z - oz);
+            const float g0 = (float)g.x, g1 = (float)g.y, g2 = (float)g.z;
+            float4* B4 = reinterpret_cast<float4*>(B);
+            B4[3 * idx] = make_float4(x, x, y, y);
+            B4[3 * idx + 1] = make_float4(z, z, g0, g0);
+            B4[3 * idx + 2] = make_float4(g1, g1, g2, g2);
+          } else if (idx < nb) {
+            const int body = sk + idx - ek;
+            const double4 p = spos[body];
+            const double4 q = sstr[body];
+            far = max(far, max(hi_abs(p.x), max(hi_abs(p.y), hi_abs(p.z))));
+            if constexpr (KIND == FMM_POINT_SOURCE) {
+              reinterpret_cast<double4*>(B)[idx] = make_double4(p.x, p.y, p.z, q.x);
+            } else {
+              double2* Bd = reinterpret_cast<double2*>(B) + 3 * idx;
+              Bd[0] = make_double2(p.x, p.y);
+              Bd[1] = make_double2(p.z, q.x);
+              Bd[2] = make_double2(q.y, q.z);
+            }
+          }
+        }
+        __syncwarp();
+        if constexpr (PACK) {
+          // targets 0 and 1 of the lane in the two halves of every f32x2 operation
+          const float4* B4 = reinterpret_cast<const float4*>(B);
+          const float2 tx2 = make_float2((float)tx[0], (float)tx[1]);
+          const float2 ty2 = make_float2((float)ty[0], (float)ty[1]);
+          const float2 tz2 = make_float2((float)tz[0], (float)tz[1]);
+          float2 ph = make_float2(0.f, 0.f), gx = ph, gy = ph, gz = ph;
+          // the batch holding the target's own leaf runs in FP64 and skips coincident bodies;
+          // the others run unguarded and, in the rare case that their sums come out non-finite
+          // (bodies that coincide in FP32), repeat the batch with the r^2 > 0 guard
+          if (self_f64) {
+            double txd[2], tyd[2], tzd[2];
+            self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
+            self_batch_f64_source<PS, NA>(reinterpret_cast<const double4*>(B), slice, nb, SS, txd, tyd, tzd, tot);
+          } else if (self_batch) {
             packed_batch<true, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+          } else {
+            packed_batch<false, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+            if (!isfinite(ph.x + ph.y + gx.x + gx.y + gy.x + gy.y + gz.x + gz.y)) {
+              ph = gx = gy = gz = make_float2(0.f, 0.f);
+              packed_batch<true, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+            }
+          }
+          part[0][0] += (R)ph.x;
+          part[1][0] += (R)ph.y;
+          part[0][1 % NA] += (R)gx.x;
+          part[1][1 % NA] += (R)gx.y;
+          part[0][2 % NA] += (R)gy.x;
+          part[1][2 % NA] += (R)gy.y;
+          part[0][3 % NA] += (R)gz.x;
+          part[1][3 % NA] += (R)gz.y;
+        } else if constexpr (PACKV) {
+          const float2 tx2 = make_float2((float)tx[0], (float)tx[1]);
+          const float2 ty2 = make_float2((float)ty[0], (float)ty[1]);
+          const float2 tz2 = make_float2((float)tz[0], (float)tz[1]);
+          const float4* B4 = reinterpret_cast<const float4*>(B);
+          float2 acc[NA];
+          // as on the point-source path: the batch holding the target's own leaf runs in FP64
+          if (self_f64) {
+#pragma unroll
+            for (int a = 0; a < NA; ++a) acc[a] = make_float2(0.f, 0.f);
+            double txd[2], tyd[2], tzd[2];
+            self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
+            self_batch_f64_vortex<GS, HS, NA>(reinterpret_cast<const double2*>(B), slice, nb, SS, txd, tyd, tzd, tot);
+          } else if (self_batch) {
+            packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+          } else {
+            packed_vortex_batch<false, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+            float sum = 0.f;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) sum += acc[a].x + acc[a].y;
+            if (!isfinite(sum)) packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+          }
+#pragma unroll
+          for (int a = 0; a < NA; ++a) {
+            part[0][a] += (R)acc[a].x;
+            part[1][a] += (R)acc[a].y;
+          }
+        } else if constexpr (KIND == FMM_POINT_SOURCE) {
+          const double4* Bd = reinterpret_cast<const double4*>(B);
+          if (general || __any_sync(kAll, max(far, tfar) >= kFarHi)) {
+            const double gx[2] = {tx[0], tx[1]}, gy[2] = {ty[0], ty[1]}, gz[2] = {tz[0], tz[1]};
+            self_batch_f64_source<PS, NA>(Bd, slice, nb, SS, gx, gy, gz, tot);
+          } else {
+#pragma unroll 2
+            for (int j = slice; j < nb; j += SS) {
+              const double4 b = Bd[j];
+#pragma unroll
+              for (int k = 0; k < kTPT; ++k) source_pair_f64<PS>(tx[k], ty[k], tz[k], b.x, b.y, b.z, b.w, part[k]);
+            }
+          }
+        } else {
+          const double2* Bd = reinterpret_cast<const double2*>(B);
+          if (general || __any_sync(kAll, max(far, tfar) >= kFarHi)) {
+            const double gx[2] = {tx[0], tx[1]}, gy[2] = {ty[0], ty[1]}, gz[2] = {tz[0], tz[1]};
+            self_batch_f64_vortex<GS, HS, NA>(Bd, slice, nb, SS, gx, gy, gz, tot);
+          } else {
+            for (int j = slice; j < nb; j += SS) {
+              const double2 a = Bd[3 * j], b = Bd[3 * j + 1], c = Bd[3 * j + 2];
+#pragma unroll
+              for (int k = 0; k < kTPT; ++k)
+                vortex_pair_f64<GS, HS>(tx[k], ty[k], tz[k], a.x, a.y, b.x, b.y, c.x, c.y, us[k], Qs[k], Es[k]);
+            }
           }
         }
-        part[0][0] += (R)ph.x;
-        part[1][0] += (R)ph.y;
-        part[0][1 % NA] += (R)gx.x;
-        part[1][1 % NA] += (R)gx.y;
-        part[0][2 % NA] += (R)gy.x;
-        part[1][2 % NA] += (R)gy.y;
-        part[0][3 % NA] += (R)gz.x;
-        part[1][3 % NA] += (R)gz.y;
-      } else if constexpr (PACKV) {
-        const float2 tx2 = make_float2((float)tx[0], (float)tx[1]);
-        const float2 ty2 = make_float2((float)ty[0], (float)ty[1]);
-        const float2 tz2 = make_float2((float)tz[0], (float)tz[1]);
-        const float4* B4 = reinterpret_cast<const float4*>(B);
-        float2 acc[NA];
-        // as on the point-source path: the batch holding the target's own leaf runs in FP64
-        if (self_f64) {
-#pragma unroll
-          for (int a = 0; a < NA; ++a) acc[a] = make_float2(0.f, 0.f);
-          double txd[2], tyd[2], tzd[2];
-          self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
-          self_batch_f64_vortex<GS, HS, NA>(reinterpret_cast<const double2*>(B), slice, nb, SS, txd, tyd, tzd, tot);
-        } else if (self_batch) {
-          packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
-        } else {
-          packed_vortex_batch<false, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
-          float sum = 0.f;
-#pragma unroll
-          for (int a = 0; a < NA; ++a) sum += acc[a].x + acc[a].y;
-          if (!isfinite(sum)) packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
-        }
-#pragma unroll
-        for (int a = 0; a < NA; ++a) {
-          part[0][a] += (R)acc[a].x;
-          part[1][a] += (R)acc[a].y;
-        }
-      } else if constexpr (QE) {
-        for (int j = slice; j < nb; j += SS) {
-          const R sx = B[j], sy = B[NB + j], sz = B[2 * NB + j], s0 = B[3 * NB + j];
-          const R s1 = B[(4 % NV) * NB + j], s2 = B[(5 % NV) * NB + j];
+        __syncwarp();
+        if (MIXED) {
 #pragma unroll
           for (int k = 0; k < kTPT; ++k)
-            vortex_pair_qe<R, GS>(tx[k], ty[k], tz[k], sx, sy, sz, s0, s1, s2, part[k], Qs[k], Es[k]);
+#pragma unroll
+            for (int a = 0; a < NA; ++a) tot[k][a] += (double)part[k][a], part[k][a] = R(0);
         }
+      }
+      if constexpr (MIXED) {
+        break;
       } else {
-        for (int j = slice; j < nb; j += SS) {
-          const R sx = B[j], sy = B[NB + j], sz = B[2 * NB + j], s0 = B[3 * NB + j];
-          const R s1 = NV == 6 ? B[(4 % NV) * NB + j] : R(0);
-          const R s2 = NV == 6 ? B[(5 % NV) * NB + j] : R(0);
+        bool finite = true;
 #pragma unroll
-          for (int k = 0; k < kTPT; ++k)
-            pair1<R, KIND, PS, GS, HS, NA>(tx[k], ty[k], tz[k], sx, sy, sz, s0, s1, s2, part[k]);
+        for (int k = 0; k < kTPT; ++k) {
+          if constexpr (KIND == FMM_POINT_VORTEX && GS) {
+#pragma unroll
+            for (int a = 0; a < 3; ++a) part[k][a % NA] = us[k][a];
+          }
+          if constexpr (QE) {
+            Qs[k][8] = -(Qs[k][0] + Qs[k][4]);
+            vortex_grad_from_qe<double>(Qs[k], Es[k], &part[k][(GS ? 3 : 0) % NA]);
+          }
+#pragma unroll
+          for (int a = 0; a < NA; ++a) {
+            tot[k][a] += part[k][a];
+            finite = finite && isfinite(tot[k][a]);
+          }
         }
+        if (general || !__any_sync(kAll, !finite)) break;
       }
-      __syncwarp();
-      if (MIXED) {
-#pragma unroll
-        for (int k = 0; k < kTPT; ++k)
-#pragma unroll
-          for (int a = 0; a < NA; ++a) tot[k][a] += (double)part[k][a], part[k][a] = R(0);
-      }
-    }
-    if constexpr (QE) {
-#pragma unroll
-      for (int k = 0; k < kTPT; ++k) vortex_grad_from_qe<R>(Qs[k], Es[k], &part[k][(GS ? 3 : 0) % NA]);
-    }
-    if (!MIXED) {
-#pragma unroll
-      for (int k = 0; k < kTPT; ++k)
-#pragma unroll
-        for (int a = 0; a < NA; ++a) tot[k][a] = (double)part[k][a];
     }
     // slices -> lanes ti (< TS), then warps -> shared memory
     for (int o = TS; o < 32; o <<= 1)
@@ -927,86 +990,89 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   note_launch();
   // target leaves of a few bodies (on average <= 8), packed FP32 kernel: one warp per row
   // (measured slower for the FP64 kernel, whose rows keep a CTA each)
-  if (packed<R, KIND>() && tt.n_bodies <= 8 * tt.n_leaves) {
-    if (smem > 48 * 1024)
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_p2p<R, KIND, PS, GS, HS, true><<<(rows + kWarps - 1) / kWarps, kWarps * 32, smem, st>>>(
-        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr,
-        nullptr, exact_self);
-  } else {
-    int dev = 0, n_sm = 0;
-    FMM_CUDA_TRY(cudaGetDevice(&dev));
-    FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-    // estimated body pairs of the launch: chunking costs a host round trip and a second kernel,
-    // which only pays for launches of much work (and the round trip holds back a serving
-    // worker's next launches)
-    const double est_pairs = (double)L.n_direct * ((double)stt.n_bodies / std::max<int64_t>(1, stt.n_leaves)) *
-                             ((double)tt.n_bodies / std::max<int64_t>(1, tt.n_leaves));
-    const bool chunk = est_pairs > kChunkPairs;
-    if (rows < kWideRowsPerSM * n_sm && !chunk) {
-      constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
-      k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<rows, kWideWarps * 32, smw, st>>>(
-          L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-          stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr, nullptr,
-          exact_self);
-    } else if (rows < kWideRowsPerSM * n_sm) {
-      // few rows: cut them into chunks of about the same number of source leaves (some
-      // kChunksPerSM per SM over the launch), one wide CTA each; the chunks' partial sums are
-      // added in chunk order by k_p2p_chunk_sum
-      constexpr int NA = n_chan<KIND, GS, HS>();
-      std::vector<int> h_off(rows + 1), h_tgt(rows), h_cnt(tt.n_branches);
-      FMM_CUDA_TRY(cudaMemcpyAsync(h_off.data(), L.dir_off.ptr, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-      FMM_CUDA_TRY(cudaMemcpyAsync(h_tgt.data(), L.dir_tgt.ptr, rows * sizeof(int), cudaMemcpyDeviceToHost, st));
-      FMM_CUDA_TRY(cudaMemcpyAsync(h_cnt.data(), tt.body_count.ptr, tt.n_branches * sizeof(int),
-                                   cudaMemcpyDeviceToHost, st));
-      FMM_CUDA_TRY(cudaStreamSynchronize(st));
-      const int64_t total = (int64_t)h_off[rows] - h_off[0], goal = (int64_t)kChunksPerSM * n_sm;
-      const int64_t per = std::max<int64_t>(2 * kWideWarps, (total + goal - 1) / goal);
-      std::vector<int4> ch, rt(rows);
-      int64_t out = 0;
-      for (int r = 0; r < rows; ++r) {
-        const int a = h_off[r], nl = h_off[r + 1] - a;
-        const int k = (int)std::max<int64_t>(1, (nl + per - 1) / per);
-        rt[r] = make_int4((int)ch.size(), (int)ch.size() + k, 0, 0);
-        const int64_t nt = h_cnt[h_tgt[r]];
-        for (int j = 0; j < k; ++j) {
-          ch.push_back(make_int4(r, a + (int)((int64_t)nl * j / k), a + (int)((int64_t)nl * (j + 1) / k), (int)out));
-          out += nt * NA;
-          FMM_CHECK(out < INT_MAX, FMM_ERR_MEMORY, "near-field chunk sums exceed the index range");
-        }
-      }
-      // floors of a few MB: regrowing frees device memory, which waits for the whole device (and
-      // for every other context's work on it)
-      L.p2p_chunks.grow(std::max<size_t>(ch.size(), 1 << 16));
-      L.p2p_rowtab.grow(std::max<size_t>(rows, 1 << 12));
-      L.p2p_part.grow(std::max<size_t>((size_t)out + 1, 1 << 19));
-      FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_chunks.ptr, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-      FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_rowtab.ptr, rt.data(), rt.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-      constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
-      k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<(int)ch.size(), kWideWarps * 32, smw, st>>>(
-          L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-          stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, L.p2p_chunks.ptr,
-          L.p2p_part.ptr, exact_self);
-      FMM_CUDA_TRY(cudaGetLastError());
-      note_launch();
-      k_p2p_chunk_sum<KIND, PS, GS, NA><<<rows, 256, 0, st>>>(L.p2p_rowtab.ptr, L.p2p_chunks.ptr, L.p2p_part.ptr,
-                                                               L.dir_tgt.ptr, tt.body_start.ptr, tt.body_count.ptr,
-                                                               acc13);
-    } else {
+  if constexpr (packed<R, KIND>()) {
+    if (tt.n_bodies <= 8 * tt.n_leaves) {
       if (smem > 48 * 1024)
-        FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false>,
+        FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, true>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_p2p<R, KIND, PS, GS, HS, false><<<rows, kWarps * 32, smem, st>>>(
+      k_p2p<R, KIND, PS, GS, HS, true><<<(rows + kWarps - 1) / kWarps, kWarps * 32, smem, st>>>(
           L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
           stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr,
-        nullptr, exact_self);
+          nullptr, exact_self);
+      FMM_CUDA_TRY(cudaGetLastError());
+      return;
     }
+  }
+  int dev = 0, n_sm = 0;
+  FMM_CUDA_TRY(cudaGetDevice(&dev));
+  FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  // estimated body pairs of the launch: chunking costs a host round trip and a second kernel,
+  // which only pays for launches of much work (and the round trip holds back a serving
+  // worker's next launches)
+  const double est_pairs = (double)L.n_direct * ((double)stt.n_bodies / std::max<int64_t>(1, stt.n_leaves)) *
+                           ((double)tt.n_bodies / std::max<int64_t>(1, tt.n_leaves));
+  const bool chunk = est_pairs > kChunkPairs;
+  if (rows < kWideRowsPerSM * n_sm && !chunk) {
+    constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
+    k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<rows, kWideWarps * 32, smw, st>>>(
+        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
+        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr, nullptr,
+        exact_self);
+  } else if (rows < kWideRowsPerSM * n_sm) {
+    // few rows: cut them into chunks of about the same number of source leaves (some
+    // kChunksPerSM per SM over the launch), one wide CTA each; the chunks' partial sums are
+    // added in chunk order by k_p2p_chunk_sum
+    constexpr int NA = n_chan<KIND, GS, HS>();
+    std::vector<int> h_off(rows + 1), h_tgt(rows), h_cnt(tt.n_branches);
+    FMM_CUDA_TRY(cudaMemcpyAsync(h_off.data(), L.dir_off.ptr, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaMemcpyAsync(h_tgt.data(), L.dir_tgt.ptr, rows * sizeof(int), cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaMemcpyAsync(h_cnt.data(), tt.body_count.ptr, tt.n_branches * sizeof(int),
+                                 cudaMemcpyDeviceToHost, st));
+    FMM_CUDA_TRY(cudaStreamSynchronize(st));
+    const int64_t total = (int64_t)h_off[rows] - h_off[0], goal = (int64_t)kChunksPerSM * n_sm;
+    const int64_t per = std::max<int64_t>(2 * kWideWarps, (total + goal - 1) / goal);
+    std::vector<int4> ch, rt(rows);
+    int64_t out = 0;
+    for (int r = 0; r < rows; ++r) {
+      const int a = h_off[r], nl = h_off[r + 1] - a;
+      const int k = (int)std::max<int64_t>(1, (nl + per - 1) / per);
+      rt[r] = make_int4((int)ch.size(), (int)ch.size() + k, 0, 0);
+      const int64_t nt = h_cnt[h_tgt[r]];
+      for (int j = 0; j < k; ++j) {
+        ch.push_back(make_int4(r, a + (int)((int64_t)nl * j / k), a + (int)((int64_t)nl * (j + 1) / k), (int)out));
+        out += nt * NA;
+        FMM_CHECK(out < INT_MAX, FMM_ERR_MEMORY, "near-field chunk sums exceed the index range");
+      }
+    }
+    // floors of a few MB: regrowing frees device memory, which waits for the whole device (and
+    // for every other context's work on it)
+    L.p2p_chunks.grow(std::max<size_t>(ch.size(), 1 << 16));
+    L.p2p_rowtab.grow(std::max<size_t>(rows, 1 << 12));
+    L.p2p_part.grow(std::max<size_t>((size_t)out + 1, 1 << 19));
+    FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_chunks.ptr, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_rowtab.ptr, rt.data(), rt.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
+    constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
+                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
+    k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<(int)ch.size(), kWideWarps * 32, smw, st>>>(
+        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
+        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, L.p2p_chunks.ptr,
+        L.p2p_part.ptr, exact_self);
+    FMM_CUDA_TRY(cudaGetLastError());
+    note_launch();
+    k_p2p_chunk_sum<KIND, PS, GS, NA><<<rows, 256, 0, st>>>(L.p2p_rowtab.ptr, L.p2p_chunks.ptr, L.p2p_part.ptr,
+                                                             L.dir_tgt.ptr, tt.body_start.ptr, tt.body_count.ptr,
+                                                             acc13);
+  } else {
+    if (smem > 48 * 1024)
+      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    k_p2p<R, KIND, PS, GS, HS, false><<<rows, kWarps * 32, smem, st>>>(
+        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
+        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr,
+      nullptr, exact_self);
   }
   FMM_CUDA_TRY(cudaGetLastError());
 }
