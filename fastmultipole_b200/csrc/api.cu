@@ -495,7 +495,7 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   markf(0);
   if (o.upward_pass && split) {
     p2m_all(fs);
-    launch_m2m(S, p, lh, c->tables, fs);
+    launch_m2m(S, p, lh, fs);
   }
   markf(1);
   // ---- interaction lists (src/interaction_list.jl:3-19, 183-213)
@@ -540,7 +540,7 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   mark(3);
   if (o.upward_pass && !split) {
     p2m_all(st);
-    launch_m2m(S, p, lh, c->tables, st);
+    launch_m2m(S, p, lh, st);
   }
   if (!split) mark(4);
   // ---- relative error methods: influence estimate on its own stream, joined before the M2L
@@ -582,7 +582,7 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   markf(3);
   if (!split) mark(6);
   if (o.downward_pass) {
-    launch_l2l(T, p, lh, c->tables, fs);
+    launch_l2l(T, p, lh, fs);
     launch_l2p(T, p, lh, ps, gs, hs, far13, fs);
   }
   markf(4);

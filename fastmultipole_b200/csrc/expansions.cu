@@ -78,54 +78,6 @@ __device__ __forceinline__ unsigned long long m2l_pair_flops(int P, bool lh) {
   return lh ? 2 * f : f;
 }
 
-template <int SLOTS, bool LH>
-__global__ void __launch_bounds__(32 * kWarps) k_m2l(const int* __restrict__ tgt_list, const int* __restrict__ off,
-                                                     const int* __restrict__ src_of, int n_targets,
-                                                     double* __restrict__ local, const double* __restrict__ multipole,
-                                                     const double* __restrict__ tcen, const double* __restrict__ tbox,
-                                                     const double* __restrict__ trad,
-                                                     const double* __restrict__ maxinf,
-                                                     const double* __restrict__ scen, int p, int em, double eps,
-                                                     int be, int* __restrict__ p_used, Tab tb, M2LStats stats) {
-  extern __shared__ double smem[];
-  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x * kWarps + wid;
-  if (b >= n_targets) return;
-  WS w = ws_of(smem + wid * ws_doubles(p), p);
-  eng::SlotNM<SLOTS> L;
-  L.init(w.NH);
-  const int t = tgt_list[b];
-  const int64_t NH4 = 4 * nh(p);
-  eng::M2LGeom g;
-  for (int d = 0; d < 3; ++d) {
-    g.tc[d] = tcen[3 * t + d];
-    g.tbox[d] = tbox[3 * t + d];
-  }
-  g.trad = trad[t];
-  g.maxinf = maxinf[t];
-  double acc[SLOTS][LH ? 4 : 2];
-  eng::acc_zero<SLOTS, LH>(acc);
-  int pmax = 0;
-  bool all_ok = true;
-  unsigned long long fl = 0;
-  for (int l = off[b]; l < off[b + 1]; ++l) {
-    int s = src_of[l];
-    double sc[3] = {scen[3 * s], scen[3 * s + 1], scen[3 * s + 2]};
-    bool ok;
-    int P = eng::chain_m2l<SLOTS, LH>(w, acc, multipole + NH4 * s, sc, g, p, em, eps, be, ok, tb, L);
-    if (p_used && lane == 0) p_used[l] = P;
-    pmax = max(pmax, P);
-    all_ok = all_ok && ok;
-    fl += m2l_pair_flops(P, LH);
-  }
-  eng::acc_store_add<SLOTS, LH>(local + NH4 * t, acc, w.NH);
-  if (lane == 0) {
-    atomicMax(stats.pmax, pmax);
-    if (!all_ok) atomicExch(stats.fail, 1);
-    atomicAdd(stats.flops, fl);
-  }
-}
-
 // M2L at orders <= 3 without error control: warp per target, lane per pair
 // (thread-per-pair chain of pair_m2l.cuh), lane partials summed by shuffles
 template <int P, bool LH>
@@ -165,53 +117,6 @@ __global__ void __launch_bounds__(32 * kWarps) k_m2l_pair(const int* __restrict_
     atomicMax(stats.pmax, P);
     atomicAdd(stats.flops, (unsigned long long)(l1 - l0) * m2l_pair_flops(P, LH));
   }
-}
-
-// M2M for one level: warp per parent, loop over its children
-template <int SLOTS, bool LH>
-__global__ void __launch_bounds__(32 * kWarps) k_m2m(int l0, int l1, const int* __restrict__ child_start,
-                                                     const int* __restrict__ n_children,
-                                                     const double* __restrict__ scen, double* __restrict__ M, int p,
-                                                     Tab tb) {
-  extern __shared__ double smem[];
-  const int wid = threadIdx.x >> 5;
-  const int k = l0 + blockIdx.x * kWarps + wid;
-  if (k >= l1) return;
-  int nc = n_children[k];
-  if (nc == 0) return;
-  WS w = ws_of(smem + wid * ws_doubles(p), p);
-  eng::SlotNM<SLOTS> L;
-  L.init(w.NH);
-  const int64_t NH4 = 4 * nh(p);
-  double acc[SLOTS][LH ? 4 : 2];
-  eng::acc_zero<SLOTS, LH>(acc);
-  int c0 = child_start[k];
-  for (int c = c0; c < c0 + nc; ++c) {
-    double dx = scen[3 * k] - scen[3 * c], dy = scen[3 * k + 1] - scen[3 * c + 1], dz = scen[3 * k + 2] - scen[3 * c + 2];
-    eng::chain_mm_ll<SLOTS, LH>(w, acc, M + NH4 * c, dx, dy, dz, p, false, tb, L);
-  }
-  eng::acc_store_add<SLOTS, LH>(M + NH4 * k, acc, w.NH);
-}
-
-// L2L for one level: warp per child of a level-l parent
-template <int SLOTS, bool LH>
-__global__ void __launch_bounds__(32 * kWarps) k_l2l(int c0, int c1, const int* __restrict__ parent,
-                                                     const double* __restrict__ tcen, double* __restrict__ Lx, int p,
-                                                     Tab tb) {
-  extern __shared__ double smem[];
-  const int wid = threadIdx.x >> 5;
-  const int c = c0 + blockIdx.x * kWarps + wid;
-  if (c >= c1) return;
-  WS w = ws_of(smem + wid * ws_doubles(p), p);
-  eng::SlotNM<SLOTS> L;
-  L.init(w.NH);
-  const int64_t NH4 = 4 * nh(p);
-  int k = parent[c];
-  double acc[SLOTS][LH ? 4 : 2];
-  eng::acc_zero<SLOTS, LH>(acc);
-  double dx = tcen[3 * c] - tcen[3 * k], dy = tcen[3 * c + 1] - tcen[3 * k + 1], dz = tcen[3 * c + 2] - tcen[3 * k + 2];
-  eng::chain_mm_ll<SLOTS, LH>(w, acc, Lx + NH4 * k, dx, dy, dz, p, true, tb, L);
-  eng::acc_store_add<SLOTS, LH>(Lx + NH4 * c, acc, w.NH);
 }
 
 // unit operator: explicit pairs (target k <- source k)
@@ -977,68 +882,6 @@ void launch_p2m(DevTree& s, int p, int kind, const DevTables&, cudaStream_t st) 
 }
 
 namespace {
-struct M2MLaunch {
-  DevTree& s;
-  int p;
-  Tab tb;
-  cudaStream_t st;
-  template <int S, bool LH>
-  void go() {
-    size_t sm = pair_smem(p);
-    allow_smem(k_m2m<S, LH>, sm);
-    for (int l = s.n_levels - 2; l >= 0; --l) {
-      int l0 = (int)s.levels_start[l], l1 = (int)s.levels_end[l];
-      int g = (l1 - l0 + kWarps - 1) / kWarps;
-      note_launch();
-      k_m2m<S, LH><<<g, 32 * kWarps, sm, st>>>(l0, l1, s.child_start.ptr, s.n_children.ptr, s.scenter.ptr,
-                                               s.multipole.ptr, p, tb);
-    }
-    FMM_CUDA_TRY(cudaGetLastError());
-  }
-};
-
-struct M2LLaunch {
-  DevTree& t;
-  const DevTree& s;
-  const DevLists& L;
-  int p, em, be;
-  double eps;
-  int* p_used;
-  M2LStats S;
-  Tab tb;
-  cudaStream_t st;
-  template <int SL, bool LH>
-  void go() {
-    size_t sm = pair_smem(p);
-    allow_smem(k_m2l<SL, LH>, sm);
-    int g = (int)((L.n_m2l_targets + kWarps - 1) / kWarps);
-    note_launch();
-    k_m2l<SL, LH><<<g, 32 * kWarps, sm, st>>>(L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, (int)L.n_m2l_targets,
-                                              t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr, t.tradius.ptr,
-                                              t.max_influence.ptr, s.scenter.ptr, p, em, eps, be, p_used, tb, S);
-    FMM_CUDA_TRY(cudaGetLastError());
-  }
-};
-
-struct L2LLaunch {
-  DevTree& t;
-  int p;
-  Tab tb;
-  cudaStream_t st;
-  template <int S, bool LH>
-  void go() {
-    size_t sm = pair_smem(p);
-    allow_smem(k_l2l<S, LH>, sm);
-    for (int l = 1; l < t.n_levels; ++l) {
-      int c0 = (int)t.levels_start[l], c1 = (int)t.levels_end[l];
-      int g = (c1 - c0 + kWarps - 1) / kWarps;
-      note_launch();
-      k_l2l<S, LH><<<g, 32 * kWarps, sm, st>>>(c0, c1, t.parent.ptr, t.tcenter.ptr, t.local.ptr, p, tb);
-    }
-    FMM_CUDA_TRY(cudaGetLastError());
-  }
-};
-
 struct OpPairsLaunch {
   int64_t n;
   double* target;
@@ -1079,12 +922,6 @@ struct OpM2LLaunch {
 };
 }  // namespace
 
-void launch_m2m(DevTree& s, int p, bool lh, const DevTables& tb, cudaStream_t st) {
-  if (launch_m2m_lane(s, p, lh, st)) return;
-  M2MLaunch f{s, p, tab_of(tb), st};
-  dispatch_slots(p, lh, f);
-}
-
 void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
                 int* p_used, int* stats, const DevTables& tb, int precision, cudaStream_t st) {
   if (L.n_m2l_targets == 0) return;
@@ -1111,14 +948,8 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
     return;
   }
   if (launch_m2l_lane(t, s, L, p, lh, em, eps, be, p_used, stats, precision, st)) return;
-  M2LLaunch f{t, s, L, p, em, be, eps, p_used, S, tab_of(tb), st};
-  dispatch_slots(p, lh, f);
-}
-
-void launch_l2l(DevTree& t, int p, bool lh, const DevTables& tb, cudaStream_t st) {
-  if (launch_l2l_lane(t, p, lh, st)) return;
-  L2LLaunch f{t, p, tab_of(tb), st};
-  dispatch_slots(p, lh, f);
+  // higher orders, and vortex particles with error control
+  launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, st);
 }
 
 void launch_l2p(DevTree& t, int p, bool lh, bool ps, bool gs, bool hs, double* acc13, cudaStream_t st) {
