@@ -230,6 +230,7 @@ struct fmm_ctx {
   DevBuf<double> stage_s, stage_t, out16, est_out16;
   DevBuf<double> adj_src, adj_out16, stage_d, vjp_out;  // fmm_vjp
   DevBuf<double> multi16;                                // fmm_solve_multi
+  DevBuf<double> direct_part;                            // fmm_direct: sums of the source splits
   // influence estimate on its own stream (run_fmm)
   cudaStream_t est_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -743,7 +744,7 @@ void ctx_release_buffers(fmm_ctx* c) {
   release_scratch(c->sc);
   release_scratch(c->est_sc);
   for (DevBuf<double>* b : {&c->stage_s, &c->stage_t, &c->out16, &c->est_out16, &c->adj_src, &c->adj_out16,
-                            &c->stage_d, &c->vjp_out, &c->multi16})
+                            &c->stage_d, &c->vjp_out, &c->multi16, &c->direct_part})
     b->release();
   c->have_solve = false;
 }
@@ -827,6 +828,7 @@ int fmm_ctx_destroy(fmm_ctx* c) {
   c->stage_d.release();
   c->vjp_out.release();
   c->multi16.release();
+  c->direct_part.release();
   c->stats.release();
   delete c;
   return FMM_OK;
@@ -862,7 +864,7 @@ size_t fmm_ctx_device_bytes(const fmm_ctx* c) {
        (s.vals_a.cap + s.vals_b.cap + s.tmp_i.cap + s.tmp_j.cap + s.tmp_k.cap + s.cnt_a.cap + s.cnt_b.cap) * 4 +
        (s.front_a.cap + s.front_b.cap + s.dir_raw.cap + s.m2l_raw.cap) * 8 + s.tmp_d.cap * 8;
   b += (c->stage_s.cap + c->stage_t.cap + c->out16.cap + c->est_out16.cap) * 8;
-  b += (c->adj_src.cap + c->adj_out16.cap + c->stage_d.cap + c->vjp_out.cap + c->multi16.cap) * 8;
+  b += (c->adj_src.cap + c->adj_out16.cap + c->stage_d.cap + c->vjp_out.cap + c->multi16.cap + c->direct_part.cap) * 8;
   return b;
 }
 
@@ -1148,7 +1150,7 @@ int fmm_direct(fmm_ctx* c, const fmm_target_system* target, const fmm_source_sys
     c->main.acc13.grow(13 * (size_t)nt + 1);
     FMM_CUDA_TRY(cudaMemsetAsync(c->main.acc13.ptr, 0, 13 * nt * sizeof(double), c->stream));
     launch_direct(T.pos.ptr, nt, S.pos.ptr, S.str.ptr, source->n_bodies, c->main.acc13.ptr, source->kind, gs != 0,
-                  hs != 0, precision, c->stream);
+                  hs != 0, precision, c->stream, &c->direct_part);
     (void)ps;
     c->out16.grow(16 * (size_t)nt + 1);
     note_launch();

@@ -113,9 +113,12 @@ void launch_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc1
 // sum over the direct list of n_target * n_source (atomically added to *out)
 void count_p2p_pairs(const DevTree& tt, const DevTree& stt, const DevLists& L, unsigned long long* out,
                      cudaStream_t st);
-// All pairs (direct!): targets in pos order, sources; writes acc13.
+// All pairs (direct!): targets in pos order, sources; accumulates into acc13.
+// part (may be null): buffer for the sums of source splits; without it nothing is allocated and
+// every target block goes through all the sources
 void launch_direct(const double4* tpos, int64_t nt, const double4* spos, const double4* sstr, int64_t ns,
-                   double* acc13, int kind, bool gs, bool hs, int precision, cudaStream_t st);
+                   double* acc13, int kind, bool gs, bool hs, int precision, cudaStream_t st,
+                   DevBuf<double>* part = nullptr);
 
 // ---- expansions.cu ----
 void upload_tables(DevTables& dt, int p, cudaStream_t st);
