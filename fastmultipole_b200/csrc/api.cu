@@ -712,8 +712,8 @@ void release_lists(DevLists& l) {
 
 void release_scratch(Scratch& s) {
   rel(s.cub); rel(s.keys_a); rel(s.keys_b); rel(s.vals_a); rel(s.vals_b); rel(s.tmp_i); rel(s.tmp_j); rel(s.tmp_k);
-  rel(s.front_a); rel(s.front_b); rel(s.dir_raw); rel(s.m2l_raw); rel(s.cnt_a); rel(s.cnt_b); rel(s.counts);
-  rel(s.tmp_d); rel(s.staging); rel(s.out16); rel(s.flag);
+  rel(s.front_a); rel(s.front_b); rel(s.dir_raw); rel(s.m2l_raw); rel(s.cnt_a); rel(s.counts);
+  rel(s.tmp_d); rel(s.alt_pos); rel(s.alt_str); rel(s.staging); rel(s.out16); rel(s.flag);
 }
 
 }  // namespace
@@ -861,8 +861,9 @@ size_t fmm_ctx_device_bytes(const fmm_ctx* c) {
   }
   const Scratch& s = c->sc;
   b += s.cub.cap + (s.keys_a.cap + s.keys_b.cap) * 8 +
-       (s.vals_a.cap + s.vals_b.cap + s.tmp_i.cap + s.tmp_j.cap + s.tmp_k.cap + s.cnt_a.cap + s.cnt_b.cap) * 4 +
-       (s.front_a.cap + s.front_b.cap + s.dir_raw.cap + s.m2l_raw.cap) * 8 + s.tmp_d.cap * 8;
+       (s.vals_a.cap + s.vals_b.cap + s.tmp_i.cap + s.tmp_j.cap + s.tmp_k.cap + s.cnt_a.cap) * 4 +
+       (s.front_a.cap + s.front_b.cap + s.dir_raw.cap + s.m2l_raw.cap) * 8 + s.tmp_d.cap * 8 +
+       (s.alt_pos.cap + s.alt_str.cap) * sizeof(double4);
   b += (c->stage_s.cap + c->stage_t.cap + c->out16.cap + c->est_out16.cap) * 8;
   b += (c->adj_src.cap + c->adj_out16.cap + c->stage_d.cap + c->vjp_out.cap + c->multi16.cap + c->direct_part.cap) * 8;
   return b;

@@ -60,9 +60,10 @@ struct Scratch {
   DevBuf<int> vals_a, vals_b, tmp_i, tmp_j, tmp_k;
   DevBuf<int2> front_a, front_b;        // traversal frontiers
   DevBuf<int2> dir_raw, m2l_raw;        // list pairs of the traversal in arrival order
-  DevBuf<int> cnt_a, cnt_b;             // pairs per target (direct, M2L)
+  DevBuf<int> cnt_a;                    // list counters and pairs per target (direct, M2L)
   DevBuf<int> counts;                   // small host-visible counters
   DevBuf<double> tmp_d;
+  DevBuf<double4> alt_pos, alt_str;     // the bodies in input order, after a tree build
   DevBuf<double> staging;               // raw caller buffers copied to HBM
   DevBuf<double> out16;                 // target buffer in original order
   DevBuf<int> flag;

@@ -17,8 +17,8 @@
 // rows of an error-controlled solve, by decreasing (r_s + r_t) / separation and then
 // source index, so that the pairs of one lane-per-pair pass stop at similar orders.
 // The result does not depend on the order in which the atomics were served.
-// The host synchronises twice per build: after the traversal (totals, capacity
-// check) and after the row compaction (row counts).
+// Both lists go through each stage in one launch, and the host synchronises once per build:
+// after the row compaction (totals, capacity check, row counts).
 #include <climits>
 
 #include <cub/cub.cuh>
@@ -101,12 +101,23 @@ __device__ int decide(const TreeRef& T, int t, const TreeRef& S, int s, const Ru
   return A_SPLIT_S;
 }
 
-__global__ void k_pack_nodes(int n, const double* __restrict__ center, const double* __restrict__ radius,
-                             const int* __restrict__ n_children, const int* __restrict__ child_start,
-                             const int* __restrict__ body_count, double4* __restrict__ geo, int4* __restrict__ info) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    geo[i] = make_double4(center[3 * i], center[3 * i + 1], center[3 * i + 2], radius[i]);
-    info[i] = make_int4(n_children[i], child_start[i], body_count[i], 0);
+// branch records of one tree in one role, and (front given) the root pair of a traversal
+struct NodeIn {
+  int n;
+  const double *center, *radius;
+  const int *n_children, *child_start, *body_count;
+  double4* geo;
+  int4* info;
+};
+__global__ void k_pack_nodes(NodeIn T, NodeIn S, int2* front, int* ctr) {
+  const NodeIn& a = blockIdx.y ? S : T;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.n; i += gridDim.x * blockDim.x) {
+    a.geo[i] = make_double4(a.center[3 * i], a.center[3 * i + 1], a.center[3 * i + 2], a.radius[i]);
+    a.info[i] = make_int4(a.n_children[i], a.child_start[i], a.body_count[i], 0);
+  }
+  if (front && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
+    front[0] = make_int2(0, 0);
+    ctr[0] = 1;
   }
 }
 
@@ -115,11 +126,6 @@ constexpr int kMaxSteps = 64;  // frontier counters; a traversal takes levels_t 
 enum : int { C_DIR = kMaxSteps, C_M2L, C_FLAG, C_ROWS_DIR, C_ROWS_M2L = C_ROWS_DIR + 8, C_N = 128 };
 constexpr int kStepThreads = 128;
 constexpr int kStepMaxBlocks = 148 * 16;
-
-__global__ void k_root_pair(int2* front, int* ctr) {
-  front[0] = make_int2(0, 0);
-  ctr[0] = 1;
-}
 
 // Add one to cnt[t] for the lanes that pass, one atomic per distinct target of the warp.
 __device__ __forceinline__ void count_targets(bool on, int t, int lane, int* __restrict__ cnt) {
@@ -226,7 +232,8 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
 }
 
 // per target: (count << 32) | (count > 0), so that one exclusive scan gives both the
-// row offset (high word) and the row ordinal among the non-empty targets (low word)
+// row offset (high word) and the row ordinal among the non-empty targets (low word); the
+// direct and the M2L counts one after the other, n + 1 entries each (the last one 0)
 __global__ void k_pack_counts(const int* __restrict__ cnt, int n, unsigned long long* __restrict__ pk) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
     const int c = cnt[t];
@@ -237,58 +244,74 @@ __global__ void k_pack_counts(const int* __restrict__ cnt, int n, unsigned long 
 constexpr int kSmallRow = 256;  // rows up to this length: one warp each (merge sort in registers)
 constexpr int kMidRow = 4096;   // up to this length: one block each; longer: segmented radix sort
 constexpr int kMidClasses = 4;  // block sorts of 512, 1024, 2048 and 4096 keys
-constexpr int kRowCtr = 2 + kMidClasses;  // per list: rows, rows per block class, big rows
 
 __host__ __device__ constexpr int mid_class(int c) { return c <= 512 ? 0 : c <= 1024 ? 1 : c <= 2048 ? 2 : 3; }
 
+// one list (direct or M2L) on its way into target rows
+struct Rows {
+  const int* cnt;        // pairs per target
+  const int2* raw;       // pairs in arrival order
+  int n;                 // pairs
+  int *off, *tgt, *roff; // offsets of all targets, the CSR of the non-empty ones
+  int* ctr;              // rows, rows per block class, big rows
+  int *mid, *big_b, *big_e, *big_r;  // rows per block class (n_targets + 1 each), longer rows
+  int *cursor, *tmp;     // slots taken per target, rows before their sort
+  int *out_t, *out_s;
+  const double4 *tgeo, *sgeo;  // non-null: rows up to kMidRow ordered by separation (RowKey)
+};
+struct RowsPair {
+  Rows l[2];
+};
+
 // offsets of all targets (off, n + 1), the CSR of the non-empty ones (tgt, roff),
 // and the rows too long for a warp sort: row ordinals per block class (mid, n + 1
-// per class) and the bounds of the longer rows (big)
-__global__ void k_rows(const int* __restrict__ cnt, const unsigned long long* __restrict__ ex, int n,
-                       int* __restrict__ off, int* __restrict__ tgt, int* __restrict__ roff, int* __restrict__ ctr,
-                       int* __restrict__ mid, int* __restrict__ big_b, int* __restrict__ big_e,
-                       int* __restrict__ big_r) {
+// per class) and the bounds of the longer rows (big).  blockIdx.y: the list.
+__global__ void k_rows(RowsPair P, const unsigned long long* __restrict__ scan, int n) {
+  const Rows& L = P.l[blockIdx.y];
+  const unsigned long long* ex = scan + (size_t)blockIdx.y * (n + 1);
+  const unsigned long long base = ex[0];
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= n; t += gridDim.x * blockDim.x) {
-    const unsigned long long e = ex[t];
+    const unsigned long long e = ex[t] - base;
     const int o = (int)(e >> 32), r = (int)(e & 0xffffffffu);
-    off[t] = o;
+    L.off[t] = o;
     if (t < n) {
-      const int c = cnt[t];
+      L.cursor[t] = 0;
+      const int c = L.cnt[t];
       if (c > 0) {
-        tgt[r] = t;
-        roff[r] = o;
+        L.tgt[r] = t;
+        L.roff[r] = o;
       }
       if (c > kMidRow) {
-        const int q = atomicAdd(ctr + 1 + kMidClasses, 1);
-        big_b[q] = o;
-        big_e[q] = o + c;
-        big_r[q] = r;
+        const int q = atomicAdd(L.ctr + 1 + kMidClasses, 1);
+        L.big_b[q] = o;
+        L.big_e[q] = o + c;
+        L.big_r[q] = r;
       } else if (c > kSmallRow) {
         const int k = mid_class(c);
-        mid[(size_t)k * (n + 1) + atomicAdd(ctr + 1 + k, 1)] = r;
+        L.mid[(size_t)k * (n + 1) + atomicAdd(L.ctr + 1 + k, 1)] = r;
       }
     } else {
-      roff[r] = o;
-      ctr[0] = r;
+      L.roff[r] = o;
+      L.ctr[0] = r;
     }
   }
 }
 
 // raw pairs into their target's row, sources only (order inside a row fixed by the
 // sort that follows); one cursor atomic per distinct target of a warp
-__global__ void k_scatter(const int2* __restrict__ raw, int n, const int* __restrict__ off, int* __restrict__ cursor,
-                          int* __restrict__ out_s) {
+__global__ void k_scatter(RowsPair P) {
+  const Rows& L = P.l[blockIdx.y];
   const int lane = threadIdx.x & 31;
-  for (int w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); w0 < n; w0 += gridDim.x * blockDim.x) {
+  for (int w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31); w0 < L.n; w0 += gridDim.x * blockDim.x) {
     const int i = w0 + lane;
-    const bool on = i < n;
-    const int2 p = on ? raw[i] : make_int2(-1 - lane, 0);
+    const bool on = i < L.n;
+    const int2 p = on ? L.raw[i] : make_int2(-1 - lane, 0);
     const unsigned grp = __match_any_sync(kFull, p.x);
     const int leader = __ffs(grp) - 1;
     int b = 0;
-    if (on && lane == leader) b = atomicAdd(cursor + p.x, __popc(grp));
+    if (on && lane == leader) b = atomicAdd(L.cursor + p.x, __popc(grp));
     b = __shfl_sync(kFull, b, leader);
-    if (on) out_s[off[p.x] + b + __popc(grp & ((1u << lane) - 1u))] = p.y;
+    if (on) L.tmp[L.off[p.x] + b + __popc(grp & ((1u << lane) - 1u))] = p.y;
   }
 }
 
@@ -325,65 +348,74 @@ __device__ __forceinline__ RowKey row_key(const double4* tgeo, const double4* sg
 
 constexpr int kSortWarps = 8;
 
-// rows of 32 (ITEMS / 2) + 1 .. 32 ITEMS entries (1 .. 32 for ITEMS = 1): one warp per row
-template <int ITEMS>
-__global__ void __launch_bounds__(kSortWarps * 32) k_sort_warp(const int* __restrict__ tgt,
-                                                                const int* __restrict__ roff, int n_rows,
-                                                                const int* __restrict__ in, int* __restrict__ out_t,
-                                                                int* __restrict__ out_s, const double4* tgeo,
-                                                                const double4* sgeo) {
+// one row of up to 32 ITEMS entries, sorted by a warp
+template <int ITEMS, class Temp>
+__device__ __forceinline__ void sort_row_warp(Temp& tmp, const Rows& L, int b, int len, int t, int lane) {
   using WMS = cub::WarpMergeSort<unsigned, ITEMS, 32>;
-  __shared__ typename WMS::TempStorage tmp[kSortWarps];
-  constexpr int lo = ITEMS == 1 ? 1 : 16 * ITEMS + 1, hi = 32 * ITEMS;
+  WMS ws(reinterpret_cast<typename WMS::TempStorage&>(tmp));
+  const RowKey rk = row_key(L.tgeo, L.sgeo, t);
+  unsigned keys[ITEMS];
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int i = lane * ITEMS + j;
+    keys[j] = i < len ? rk.enc(L.tmp[b + i]) : UINT_MAX;
+  }
+  ws.Sort(keys, KeyLess(), len, UINT_MAX);
+#pragma unroll
+  for (int j = 0; j < ITEMS; ++j) {
+    const int i = lane * ITEMS + j;
+    if (i < len) L.out_t[b + i] = t, L.out_s[b + i] = rk.dec(keys[j]);
+  }
+  __syncwarp();
+}
+
+// rows of up to kSmallRow entries: one warp each.  blockIdx.y: the list
+__global__ void __launch_bounds__(kSortWarps * 32) k_sort_warp(RowsPair P) {
+  using Temp = typename cub::WarpMergeSort<unsigned, 8, 32>::TempStorage;
+  __shared__ Temp tmp[kSortWarps];
+  const Rows& L = P.l[blockIdx.y];
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  WMS ws(tmp[w]);
+  const int n_rows = L.ctr[0];
   for (int r = blockIdx.x * kSortWarps + w; r < n_rows; r += gridDim.x * kSortWarps) {
-    const int b = roff[r], len = roff[r + 1] - b;
-    if (len < lo || len > hi) continue;
-    const int t = tgt[r];
+    const int b = L.roff[r], len = L.roff[r + 1] - b;
+    if (len > kSmallRow) continue;
+    const int t = L.tgt[r];
     if (len == 1) {
-      if (lane == 0) out_t[b] = t, out_s[b] = in[b];
-      continue;
+      if (lane == 0) L.out_t[b] = t, L.out_s[b] = L.tmp[b];
+    } else if (len <= 32) {
+      sort_row_warp<1>(tmp[w], L, b, len, t, lane);
+    } else if (len <= 64) {
+      sort_row_warp<2>(tmp[w], L, b, len, t, lane);
+    } else if (len <= 128) {
+      sort_row_warp<4>(tmp[w], L, b, len, t, lane);
+    } else {
+      sort_row_warp<8>(tmp[w], L, b, len, t, lane);
     }
-    const RowKey rk = row_key(tgeo, sgeo, t);
-    unsigned keys[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const int i = lane * ITEMS + j;
-      keys[j] = i < len ? rk.enc(in[b + i]) : UINT_MAX;
-    }
-    ws.Sort(keys, KeyLess(), len, UINT_MAX);
-#pragma unroll
-    for (int j = 0; j < ITEMS; ++j) {
-      const int i = lane * ITEMS + j;
-      if (i < len) out_t[b + i] = t, out_s[b + i] = rk.dec(keys[j]);
-    }
-    __syncwarp();
   }
 }
 
-// rows of one block class: one block of THREADS x ITEMS keys per row
+// rows of one block class: one block of THREADS x ITEMS keys per row (n0 rows of the first
+// list, the others of the second)
 template <int THREADS, int ITEMS>
-__global__ void __launch_bounds__(THREADS) k_sort_block(const int* __restrict__ mid, const int* __restrict__ tgt,
-                                                      const int* __restrict__ roff, const int* __restrict__ in,
-                                                      int* __restrict__ out_t, int* __restrict__ out_s,
-                                                      const double4* tgeo, const double4* sgeo) {
+__global__ void __launch_bounds__(THREADS) k_sort_block(RowsPair P, size_t mid0, int n0) {
   using BMS = cub::BlockMergeSort<unsigned, THREADS, ITEMS>;
   __shared__ typename BMS::TempStorage tmp;
-  const int r = mid[blockIdx.x];
-  const int b = roff[r], len = roff[r + 1] - b, t = tgt[r];
-  const RowKey rk = row_key(tgeo, sgeo, t);
+  const int q = (int)blockIdx.x < n0 ? 0 : 1;
+  const Rows& L = P.l[q];
+  const int r = L.mid[mid0 + blockIdx.x - (q ? n0 : 0)];
+  const int b = L.roff[r], len = L.roff[r + 1] - b, t = L.tgt[r];
+  const RowKey rk = row_key(L.tgeo, L.sgeo, t);
   unsigned keys[ITEMS];
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = threadIdx.x * ITEMS + j;
-    keys[j] = i < len ? rk.enc(in[b + i]) : UINT_MAX;
+    keys[j] = i < len ? rk.enc(L.tmp[b + i]) : UINT_MAX;
   }
   BMS(tmp).Sort(keys, KeyLess(), len, UINT_MAX);
 #pragma unroll
   for (int j = 0; j < ITEMS; ++j) {
     const int i = threadIdx.x * ITEMS + j;
-    if (i < len) out_t[b + i] = t, out_s[b + i] = rk.dec(keys[j]);
+    if (i < len) L.out_t[b + i] = t, L.out_s[b + i] = rk.dec(keys[j]);
   }
 }
 
@@ -399,99 +431,51 @@ int blocks_for(int64_t n, int threads) {
   return (int)std::max<int64_t>(1, std::min<int64_t>((n + threads - 1) / threads, kStepMaxBlocks));
 }
 
-// one list (direct or M2L) being turned into target rows
-struct RowBuild {
-  const int* cnt;
-  const int2* raw;
-  int n;
-  DevBuf<int>*out_t, *out_s, *tgt, *roff;
-  DevBuf<int>* off;
-  DevBuf<int>* tmp;
-  int* ctr;  // rows, rows per block class, big rows (kRowCtr ints)
-  const double4* tgeo = nullptr;  // non-null: rows up to kMidRow ordered by separation (RowKey)
-  const double4* sgeo = nullptr;
-};
-
-// offsets and row CSR (before the host reads the row counts)
-void rows_of(RowBuild& B, int nt, Scratch& sc, cudaStream_t st) {
-  B.out_t->grow((size_t)B.n + 1);
-  B.out_s->grow((size_t)B.n + 1);
-  B.tgt->grow((size_t)nt + 1);
-  B.roff->grow((size_t)nt + 2);
-  B.off->grow((size_t)nt + 1);
-  sc.keys_a.grow((size_t)nt + 1);
-  sc.keys_b.grow((size_t)nt + 1);
+// rows sorted, both lists in one launch per kind of row (h0, h1: the lists' counters)
+template <int THREADS, int ITEMS>
+void sort_block_class(const RowsPair& P, int k, size_t stride, const int* h0, const int* h1, cudaStream_t st) {
+  const int n0 = h0[1 + k], n1 = h1[1 + k];
+  if (n0 + n1 == 0) return;
   note_launch();
-  k_pack_counts<<<blocks_for(nt + 1, 256), 256, 0, st>>>(B.cnt, nt + 1, sc.keys_a.ptr);
-  size_t tb = 0;
-  cub::DeviceScan::ExclusiveSum(nullptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, nt + 1, st);
-  sc.cub.grow(tb);
-  FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sc.cub.ptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, nt + 1, st));
-  note_launch();
-  k_rows<<<blocks_for(nt + 1, 256), 256, 0, st>>>(B.cnt, sc.keys_b.ptr, nt, B.off->ptr, B.tgt->ptr, B.roff->ptr,
-                                                  B.ctr, sc.row_mid.ptr, sc.row_big_b.ptr, sc.row_big_e.ptr,
-                                                  sc.row_big_r.ptr);
+  k_sort_block<THREADS, ITEMS><<<n0 + n1, THREADS, 0, st>>>(P, (size_t)k * stride, n0);
   FMM_CUDA_TRY(cudaGetLastError());
 }
 
-// scatter into rows and sort every row by source index (after the host read the counts:
-// h = rows, rows per block class, big rows)
-void sort_rows(RowBuild& B, int nt, const int* h, int nbits, Scratch& sc, cudaStream_t st) {
-  if (B.n == 0) return;
-  const int rows = h[0], n_big = h[1 + kMidClasses];
-  B.tmp->grow((size_t)B.n + 1);
-  sc.row_cur.grow((size_t)nt + 1);
-  FMM_CUDA_TRY(cudaMemsetAsync(sc.row_cur.ptr, 0, (size_t)nt * sizeof(int), st));
+void sort_rows(const RowsPair& P, int nt, const int* h0, const int* h1, int nbits, Scratch& sc, cudaStream_t st) {
+  const int n = std::max(P.l[0].n, P.l[1].n), rows = std::max(h0[0], h1[0]);
+  if (n == 0) return;
   note_launch();
-  k_scatter<<<blocks_for(B.n, 256), 256, 0, st>>>(B.raw, B.n, B.off->ptr, sc.row_cur.ptr, B.tmp->ptr);
-  const int gw = blocks_for((int64_t)rows * 32, kSortWarps * 32);
+  k_scatter<<<dim3(blocks_for(n, 256), 2), 256, 0, st>>>(P);
   note_launch();
-  k_sort_warp<1><<<gw, kSortWarps * 32, 0, st>>>(B.tgt->ptr, B.roff->ptr, rows, B.tmp->ptr, B.out_t->ptr, B.out_s->ptr,
-                                                  B.tgeo, B.sgeo);
-  note_launch();
-  k_sort_warp<2><<<gw, kSortWarps * 32, 0, st>>>(B.tgt->ptr, B.roff->ptr, rows, B.tmp->ptr, B.out_t->ptr, B.out_s->ptr,
-                                                  B.tgeo, B.sgeo);
-  note_launch();
-  k_sort_warp<4><<<gw, kSortWarps * 32, 0, st>>>(B.tgt->ptr, B.roff->ptr, rows, B.tmp->ptr, B.out_t->ptr, B.out_s->ptr,
-                                                  B.tgeo, B.sgeo);
-  note_launch();
-  k_sort_warp<8><<<gw, kSortWarps * 32, 0, st>>>(B.tgt->ptr, B.roff->ptr, rows, B.tmp->ptr, B.out_t->ptr, B.out_s->ptr,
-                                                  B.tgeo, B.sgeo);
+  k_sort_warp<<<dim3(blocks_for((int64_t)rows * 32, kSortWarps * 32), 2), kSortWarps * 32, 0, st>>>(P);
   FMM_CUDA_TRY(cudaGetLastError());
-  const int* mid = sc.row_mid.ptr;
   const size_t stride = (size_t)nt + 1;
-  if (h[1] > 0) {
-    note_launch();
-    k_sort_block<128, 4><<<h[1], 128, 0, st>>>(mid, B.tgt->ptr, B.roff->ptr, B.tmp->ptr, B.out_t->ptr, B.out_s->ptr,
-                                               B.tgeo, B.sgeo);
-  }
-  if (h[2] > 0) {
-    note_launch();
-    k_sort_block<256, 4><<<h[2], 256, 0, st>>>(mid + stride, B.tgt->ptr, B.roff->ptr, B.tmp->ptr, B.out_t->ptr,
-                                               B.out_s->ptr, B.tgeo, B.sgeo);
-  }
-  if (h[3] > 0) {
-    note_launch();
-    k_sort_block<256, 8><<<h[3], 256, 0, st>>>(mid + 2 * stride, B.tgt->ptr, B.roff->ptr, B.tmp->ptr, B.out_t->ptr,
-                                               B.out_s->ptr, B.tgeo, B.sgeo);
-  }
-  if (h[4] > 0) {
-    note_launch();
-    k_sort_block<256, 16><<<h[4], 256, 0, st>>>(mid + 3 * stride, B.tgt->ptr, B.roff->ptr, B.tmp->ptr, B.out_t->ptr,
-                                                B.out_s->ptr, B.tgeo, B.sgeo);
-  }
-  FMM_CUDA_TRY(cudaGetLastError());
-  if (n_big > 0) {
+  sort_block_class<128, 4>(P, 0, stride, h0, h1, st);
+  sort_block_class<256, 4>(P, 1, stride, h0, h1, st);
+  sort_block_class<256, 8>(P, 2, stride, h0, h1, st);
+  sort_block_class<256, 16>(P, 3, stride, h0, h1, st);
+  for (int q = 0; q < 2; ++q) {
+    const Rows& L = P.l[q];
+    const int n_big = (q ? h1 : h0)[1 + kMidClasses];
+    if (n_big == 0) continue;
     size_t tb = 0;
-    cub::DeviceSegmentedRadixSort::SortKeys(nullptr, tb, B.tmp->ptr, B.out_s->ptr, B.n, n_big, sc.row_big_b.ptr,
-                                            sc.row_big_e.ptr, 0, nbits, st);
+    cub::DeviceSegmentedRadixSort::SortKeys(nullptr, tb, L.tmp, L.out_s, L.n, n_big, L.big_b, L.big_e, 0, nbits, st);
     sc.cub.grow(tb);
-    FMM_CUDA_TRY(cub::DeviceSegmentedRadixSort::SortKeys(sc.cub.ptr, tb, B.tmp->ptr, B.out_s->ptr, B.n, n_big,
-                                                         sc.row_big_b.ptr, sc.row_big_e.ptr, 0, nbits, st));
+    FMM_CUDA_TRY(cub::DeviceSegmentedRadixSort::SortKeys(sc.cub.ptr, tb, L.tmp, L.out_s, L.n, n_big, L.big_b, L.big_e,
+                                                         0, nbits, st));
     note_launch();
-    k_fill_rows<<<n_big, 256, 0, st>>>(sc.row_big_r.ptr, B.tgt->ptr, B.roff->ptr, B.out_t->ptr);
+    k_fill_rows<<<n_big, 256, 0, st>>>(L.big_r, L.tgt, L.roff, L.out_t);
     FMM_CUDA_TRY(cudaGetLastError());
   }
+}
+
+NodeIn target_nodes(const DevTree& t, Scratch& sc) {
+  return NodeIn{(int)t.n_branches,  t.tcenter.ptr,    t.tradius.ptr,     t.n_children.ptr,
+                t.child_start.ptr, t.body_count.ptr, sc.node_geo_t.ptr, sc.node_info_t.ptr};
+}
+NodeIn source_nodes(const DevTree& t, Scratch& sc) {
+  return NodeIn{(int)t.n_branches,  t.scenter.ptr,    t.sradius.ptr,     t.n_children.ptr,
+                t.child_start.ptr, t.body_count.ptr, sc.node_geo_s.ptr, sc.node_info_s.ptr};
 }
 
 }  // namespace
@@ -504,28 +488,34 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
   sc.node_info_t.grow((size_t)nt);
   sc.node_geo_s.grow((size_t)ns);
   sc.node_info_s.grow((size_t)ns);
-  note_launch();
-  k_pack_nodes<<<blocks_for(nt, 256), 256, 0, st>>>(nt, tt.tcenter.ptr, tt.tradius.ptr, tt.n_children.ptr,
-                                                     tt.child_start.ptr, tt.body_count.ptr, sc.node_geo_t.ptr,
-                                                     sc.node_info_t.ptr);
-  note_launch();
-  k_pack_nodes<<<blocks_for(ns, 256), 256, 0, st>>>(ns, stt.scenter.ptr, stt.sradius.ptr, stt.n_children.ptr,
-                                                     stt.child_start.ptr, stt.body_count.ptr, sc.node_geo_s.ptr,
-                                                     sc.node_info_s.ptr);
-  FMM_CUDA_TRY(cudaGetLastError());
   TreeRef T{sc.node_geo_t.ptr, sc.node_info_t.ptr};
   TreeRef S{sc.node_geo_s.ptr, sc.node_info_s.ptr};
   Rule R{mac, leaf_size_source, method, ff, nf, si};
   const int n_steps = tt.n_levels + stt.n_levels - 1;
   FMM_CHECK(n_steps + 1 < kMaxSteps, FMM_ERR_TREE_DEPTH, "interaction-list traversal deeper than supported");
-  sc.counts.grow(C_N);
-  int* ctr = sc.counts.ptr;
-  sc.cnt_a.grow((size_t)nt + 1);
-  sc.cnt_b.grow((size_t)nt + 1);
+  // counters, then the pairs per target of the two lists (nt + 1 each): one buffer, cleared at once
+  const size_t n1 = (size_t)nt + 1;
+  sc.cnt_a.grow(C_N + 2 * n1);
+  int* ctr = sc.cnt_a.ptr;
+  int *cnt_d = ctr + C_N, *cnt_m = cnt_d + n1;
+  sc.row_mid.grow(2 * (size_t)kMidClasses * n1);
+  sc.row_big_b.grow(2 * n1);
+  sc.row_big_e.grow(2 * n1);
+  sc.row_big_r.grow(2 * n1);
+  sc.row_cur.grow(2 * n1);
+  sc.row_off_a.grow(n1);
+  sc.row_off_b.grow(n1);
+  L.dir_tgt.grow(n1);
+  L.dir_off.grow(n1 + 1);
+  L.m2l_tgt.grow(n1);
+  L.m2l_off.grow(n1 + 1);
+  sc.keys_a.grow(2 * n1);
+  sc.keys_b.grow(2 * n1);
   // capacities: kept from earlier builds, grown when a traversal reports more
   size_t cap_f = std::max<size_t>(4096, (size_t)nt * 32), cap_d = std::max<size_t>(4096, (size_t)tt.n_leaves * 64);
   size_t cap_m = std::max<size_t>(4096, (size_t)nt * 96);
   std::vector<int> h(C_N, 0);
+  RowsPair P;
   for (int attempt = 0;; ++attempt) {
     FMM_CHECK(attempt < 8, FMM_ERR_MEMORY, "interaction-list capacities did not converge");
     sc.front_a.grow(cap_f);
@@ -534,11 +524,12 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
     sc.m2l_raw.grow(cap_m);
     const int cf = (int)std::min<size_t>(sc.front_a.cap, sc.front_b.cap);
     const int cd = (int)sc.dir_raw.cap, cm = (int)sc.m2l_raw.cap;
-    FMM_CUDA_TRY(cudaMemsetAsync(ctr, 0, C_N * sizeof(int), st));
-    FMM_CUDA_TRY(cudaMemsetAsync(sc.cnt_a.ptr, 0, ((size_t)nt + 1) * sizeof(int), st));
-    FMM_CUDA_TRY(cudaMemsetAsync(sc.cnt_b.ptr, 0, ((size_t)nt + 1) * sizeof(int), st));
+    FMM_CUDA_TRY(cudaMemsetAsync(ctr, 0, (C_N + 2 * n1) * sizeof(int), st));
     note_launch();
-    k_root_pair<<<1, 1, 0, st>>>(sc.front_a.ptr, ctr);
+    k_pack_nodes<<<dim3(blocks_for(std::max(nt, ns), 256), 2), 256, 0, st>>>(target_nodes(tt, sc),
+                                                                              source_nodes(stt, sc),
+                                                                              sc.front_a.ptr, ctr);
+    FMM_CUDA_TRY(cudaGetLastError());
     for (int k = 0; k < n_steps; ++k) {
       const int2* fin = (k & 1) ? sc.front_b.ptr : sc.front_a.ptr;
       int2* fout = (k & 1) ? sc.front_a.ptr : sc.front_b.ptr;
@@ -546,9 +537,38 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
       const int64_t hint = k < (int)sc.step_hint.size() ? sc.step_hint[k] : (int64_t)kStepChunk * kStepMaxBlocks;
       note_launch();
       k_step<<<blocks_for(hint + hint / 4 + 32, kStepChunk), kStepThreads, 0, st>>>(
-          fin, fout, k, T, S, R, sc.dir_raw.ptr, sc.m2l_raw.ptr, sc.cnt_a.ptr, sc.cnt_b.ptr, ctr, cf, cd, cm);
+          fin, fout, k, T, S, R, sc.dir_raw.ptr, sc.m2l_raw.ptr, cnt_d, cnt_m, ctr, cf, cd, cm);
       FMM_CUDA_TRY(cudaGetLastError());
     }
+    // row offsets of both lists (of partial counts after an overflow, which are then not used)
+    note_launch();
+    k_pack_counts<<<blocks_for(2 * (int64_t)n1, 256), 256, 0, st>>>(cnt_d, (int)(2 * n1), sc.keys_a.ptr);
+    size_t tb = 0;
+    cub::DeviceScan::ExclusiveSum(nullptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, (int)(2 * n1), st);
+    sc.cub.grow(tb);
+    FMM_CUDA_TRY(cub::DeviceScan::ExclusiveSum(sc.cub.ptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, (int)(2 * n1), st));
+    auto rows = [&](int q, int* cnt, const int2* raw, int* off, int* tgt, int* roff, int slot) {
+      Rows& r = P.l[q];
+      r.cnt = cnt;
+      r.raw = raw;
+      r.n = 0;
+      r.off = off;
+      r.tgt = tgt;
+      r.roff = roff;
+      r.ctr = ctr + slot;
+      r.mid = sc.row_mid.ptr + q * kMidClasses * n1;
+      r.big_b = sc.row_big_b.ptr + q * n1;
+      r.big_e = sc.row_big_e.ptr + q * n1;
+      r.big_r = sc.row_big_r.ptr + q * n1;
+      r.cursor = sc.row_cur.ptr + q * n1;
+      r.tmp = r.out_t = r.out_s = nullptr;
+      r.tgeo = r.sgeo = nullptr;
+    };
+    rows(0, cnt_d, sc.dir_raw.ptr, sc.row_off_a.ptr, L.dir_tgt.ptr, L.dir_off.ptr, C_ROWS_DIR);
+    rows(1, cnt_m, sc.m2l_raw.ptr, sc.row_off_b.ptr, L.m2l_tgt.ptr, L.m2l_off.ptr, C_ROWS_M2L);
+    note_launch();
+    k_rows<<<dim3(blocks_for((int64_t)n1, 256), 2), 256, 0, st>>>(P, sc.keys_b.ptr, nt);
+    FMM_CUDA_TRY(cudaGetLastError());
     FMM_CUDA_TRY(cudaMemcpyAsync(h.data(), ctr, C_N * sizeof(int), cudaMemcpyDeviceToHost, st));
     FMM_CUDA_TRY(cudaStreamSynchronize(st));
     size_t max_f = 0;
@@ -568,30 +588,27 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
   const int n_dir = h[C_DIR], n_m2l = h[C_M2L];
   int nbits = 1;
   while ((1ll << nbits) <= stt.n_branches) ++nbits;
-  // the row classes of one list are built (k_rows) and consumed (sort_rows) before the
-  // next list's k_rows reuses the class arrays, so the lists take turns
-  sc.row_mid.grow((size_t)kMidClasses * (nt + 1));
-  sc.row_big_b.grow((size_t)nt + 1);
-  sc.row_big_e.grow((size_t)nt + 1);
-  sc.row_big_r.grow((size_t)nt + 1);
-  RowBuild lists[2] = {
-      {sc.cnt_a.ptr, sc.dir_raw.ptr, n_dir, &L.dir_t, &L.dir_s, &L.dir_tgt, &L.dir_off, &sc.row_off_a, &sc.row_tmp_a,
-       ctr + C_ROWS_DIR},
-      {sc.cnt_b.ptr, sc.m2l_raw.ptr, n_m2l, &L.m2l_t, &L.m2l_s, &L.m2l_tgt, &L.m2l_off, &sc.row_off_b, &sc.row_tmp_b,
-       ctr + C_ROWS_M2L}};
+  L.dir_t.grow((size_t)n_dir + 1);
+  L.dir_s.grow((size_t)n_dir + 1);
+  L.m2l_t.grow((size_t)n_m2l + 1);
+  L.m2l_s.grow((size_t)n_m2l + 1);
+  sc.row_tmp_a.grow((size_t)n_dir + 1);
+  sc.row_tmp_b.grow((size_t)n_m2l + 1);
+  P.l[0].n = n_dir;
+  P.l[0].tmp = sc.row_tmp_a.ptr;
+  P.l[0].out_t = L.dir_t.ptr;
+  P.l[0].out_s = L.dir_s.ptr;
+  P.l[1].n = n_m2l;
+  P.l[1].tmp = sc.row_tmp_b.ptr;
+  P.l[1].out_t = L.m2l_t.ptr;
+  P.l[1].out_s = L.m2l_s.ptr;
   if (m2l_by_separation && ns < (1 << kSepShift)) {
-    lists[1].tgeo = sc.node_geo_t.ptr;
-    lists[1].sgeo = sc.node_geo_s.ptr;
+    P.l[1].tgeo = sc.node_geo_t.ptr;
+    P.l[1].sgeo = sc.node_geo_s.ptr;
   }
-  int rows[2] = {0, 0};
-  for (int q = 0; q < 2; ++q) {
-    rows_of(lists[q], nt, sc, st);
-    int hq[kRowCtr];
-    FMM_CUDA_TRY(cudaMemcpyAsync(hq, lists[q].ctr, kRowCtr * sizeof(int), cudaMemcpyDeviceToHost, st));
-    FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    rows[q] = hq[0];
-    sort_rows(lists[q], nt, hq, nbits, sc, st);
-  }
+  const int *h_d = h.data() + C_ROWS_DIR, *h_m = h.data() + C_ROWS_M2L;
+  sort_rows(P, nt, h_d, h_m, nbits, sc, st);
+  const int rows[2] = {h_d[0], h_m[0]};
   L.n_direct = n_dir;
   L.n_m2l = n_m2l;
   L.n_dir_targets = rows[0];
@@ -681,13 +698,8 @@ void export_lists_reference_order(const DevLists& L, const DevTree& tt, const De
   sc.node_geo_s.grow((size_t)ns);
   sc.node_info_s.grow((size_t)ns);
   note_launch();
-  k_pack_nodes<<<blocks_for(nt, 256), 256, 0, st>>>(nt, tt.tcenter.ptr, tt.tradius.ptr, tt.n_children.ptr,
-                                                     tt.child_start.ptr, tt.body_count.ptr, sc.node_geo_t.ptr,
-                                                     sc.node_info_t.ptr);
-  note_launch();
-  k_pack_nodes<<<blocks_for(ns, 256), 256, 0, st>>>(ns, stt.scenter.ptr, stt.sradius.ptr, stt.n_children.ptr,
-                                                     stt.child_start.ptr, stt.body_count.ptr, sc.node_geo_s.ptr,
-                                                     sc.node_info_s.ptr);
+  k_pack_nodes<<<dim3(blocks_for(std::max(nt, ns), 256), 2), 256, 0, st>>>(target_nodes(tt, sc), source_nodes(stt, sc),
+                                                                            nullptr, nullptr);
   FMM_CUDA_TRY(cudaGetLastError());
   const TreeRef T{sc.node_geo_t.ptr, sc.node_info_t.ptr};
   const TreeRef S{sc.node_geo_s.ptr, sc.node_info_s.ptr};

@@ -1135,12 +1135,18 @@ void run_direct(const double4* tpos, int64_t nt, const double4* spos, const doub
     splits = std::min<int64_t>(splits, (int64_t)(kDirectPartMax / (NA * sizeof(double))) / nt);
     splits = std::max<int64_t>(1, std::min<int64_t>(splits, 65535));
   }
-  const int64_t per = std::max<int64_t>(1, (chunks + splits - 1) / splits);
+  int64_t per = std::max<int64_t>(1, (chunks + splits - 1) / splits);
   splits = std::max<int64_t>(1, (chunks + per - 1) / per);
   double* sums = nullptr;
   if (splits > 1) {
-    part->grow((size_t)splits * nt * NA);
-    sums = part->ptr;
+    try {
+      part->grow((size_t)splits * nt * NA);
+      sums = part->ptr;
+    } catch (const Error&) {  // no room for the sums: one pass over all the sources needs none
+      cudaGetLastError();
+      splits = 1;
+      per = chunks;
+    }
   }
   FMM_CHECK(per * kP2PThreads < INT_MAX && tiles < INT_MAX, FMM_ERR_MEMORY, "all-pairs sum exceeds the index range");
   note_launch();
