@@ -42,9 +42,10 @@ struct DevLists {
   int64_t n_m2l_targets = 0, n_dir_targets = 0;
   DevBuf<int> m2l_tgt, m2l_off;   // unique targets, offsets (n+1)
   DevBuf<int> dir_tgt, dir_off;
-  // near field of launches of few rows: rows cut into chunks of source leaves (row, leaf range,
-  // offset of the chunk's partial sums), their partial sums, and each row's chunk range
-  DevBuf<int4> p2p_chunks, p2p_rowtab;
+  // near field of launches of few rows: their items (p2p.cu), number of items and sources per
+  // row, and the items' sums
+  DevBuf<int4> p2p_items;
+  DevBuf<int> p2p_meta;
   DevBuf<double> p2p_part;
   // the traversal's rule (for the reference-order export)
   double rule_mac = 0.5;

@@ -13,7 +13,6 @@
 // centre in FP64, then evaluates the kernel in FP32 (rsqrt on the SFU),
 // summing blocks of sources in FP32 and the block partials in FP64.
 #include <climits>
-#include <vector>
 #include <algorithm>
 
 #include "context.cuh"
@@ -31,10 +30,9 @@ __host__ __device__ constexpr int tpt() { return KIND == FMM_POINT_SOURCE ? 4 : 
 __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
 
 // ---------------------------------------------------------------------------
-// Direct-list P2P.  One CTA of kWarps warps (kWideWarps when the launch has few rows, so
-// that a few long rows still fill the GPU) owns one direct-list row (a target leaf).
-// Each warp takes every W-th source leaf of the leaf's direct-list row and
-// gathers up to batch_bodies() bodies of consecutive leaves of its share (many
+// Direct-list P2P.  One CTA of kWarps warps owns one direct-list row (a target leaf), or an
+// item: a tile of its targets and a share of its source leaves.  Each warp takes its part of
+// the source leaves and gathers up to batch_bodies() bodies of consecutive leaves of its share (many
 // small leaves, or a piece of a large one) into its own shared-memory batch,
 // converted once per body (to FP32 relative to the target leaf centre on the
 // mixed path).  Targets sit in registers, kTPT per lane.  A target tile holds
@@ -46,12 +44,15 @@ __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
 // of small target leaves (at most 8 bodies on average) take one warp each instead of
 // a CTA, so that the per-row setup and the cross-warp sum do not dominate their work.
 constexpr int kWarps = 4;
-// launches of fewer rows than kWideRowsPerSM per SM take kWideWarps warps per row: a few
-// long rows (targets of a dual tree near many sources) would otherwise leave the SMs idle
-constexpr int kWideWarps = 16;
-constexpr int kWideRowsPerSM = 4;
-constexpr int kChunksPerSM = 8;  // chunks of the rows of such a launch, per SM
-constexpr double kChunkPairs = 1e8;  // estimated body pairs above which their rows are cut
+// Launches of up to kItemRowsPerSM rows per SM are cut into items of about equal work, some
+// kItemWaves for every CTA that the SMs hold at a time: one tile of a row's targets x a share of the
+// row's source leaves (at least kItemSources bodies), whose sums are added in order by k_p2p_sum.
+// With a CTA of 4 or 16 warps per row the few rows of large leaves (up to three tiles) and the long
+// rows of probe leaves were still running when the others had finished.  10,000 bodies FP64: near
+// field 273 -> 113 us and 50 us to cut and to add; 300k vortex ring FP64: 28.2 -> 25.5 ms (whole
+// solves).  More rows than that fill the GPU by themselves (1e6 bodies: 62.0 ms either way).
+constexpr int kItemRowsPerSM = 64, kItemWaves = 4, kItemSources = 256;
+constexpr double kItemPairs = 4e6;  // below this many pairs the extra launches cost more than they save
 constexpr int kTPT = 2;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -411,31 +412,32 @@ __device__ __noinline__ void self_batch_f64_vortex(const double2* __restrict__ B
 }
 
 // RW: one warp per row (rows of small leaves, kWarps rows per CTA), the warp adding its
-// sums to the targets itself; otherwise one CTA per row, the warps splitting its sources.
-// W warps per CTA: kWarps, or kWideWarps for launches of few rows (one long row per CTA).
+// sums to the targets itself; otherwise one CTA per row or item, the warps splitting its sources.
 // resident CTAs of the mixed instances: the registers the packed loop needs (the FP64
 // branch of the batch holding the target's own leaf is a call, and must not raise them);
 // the FP64 vortex CTA path takes 168 registers (3 CTAs per SM; 300k ring, order 12, whole solve:
 // 28.6 ms, 28.8 with 2 CTAs, and 49.3 with 4, whose 128 registers spill inside the loop)
-template <class R, int KIND, bool HS, bool RW, int W>
+template <class R, int KIND, bool HS, bool RW>
 __host__ __device__ constexpr int p2p_min_blocks() {
   constexpr int regs = (KIND == FMM_POINT_VORTEX && HS) ? (RW ? 168 : 128) : (RW ? 72 : 64);
-  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW && W == kWarps) ? 3 : 1;
-  return 65536 / (regs * W * 32) > 0 ? 65536 / (regs * W * 32) : 1;
+  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW) ? 3 : 1;
+  return 65536 / (regs * kWarps * 32);
 }
 
-template <class R, int KIND, bool PS, bool GS, bool HS, bool RW, int W = kWarps>
-__global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) k_p2p(const int* __restrict__ tgt_list, const int* __restrict__ off,
+template <class R, int KIND, bool PS, bool GS, bool HS, bool RW, bool ITEMS>
+__global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()) k_p2p(const int* __restrict__ tgt_list, const int* __restrict__ off,
                                                      int n_rows, const int* __restrict__ src_of,
                                                      const int* __restrict__ t_start, const int* __restrict__ t_count,
                                                      const double* __restrict__ t_center,
                                                      const int* __restrict__ s_start, const int* __restrict__ s_count,
                                                      const double4* __restrict__ tpos, const double4* __restrict__ spos,
                                                      const double4* __restrict__ sstr, double* __restrict__ acc13,
-                                                     const int4* __restrict__ chunks, double* __restrict__ chunk_sums,
-                                                     int exact_self) {
-  // chunks (CTA path only; may be null): CTA b takes the source leaves [y, z) of row x and stores
-  // its sums (unscaled, not atomically) at chunk_sums + w + NA * (target index in the row) + channel
+                                                     const int4* __restrict__ items, const int* __restrict__ n_items,
+                                                     double* __restrict__ item_sums, int exact_self) {
+  // items (ITEMS, CTA path only), two int4 each: row, tile and source leaves [z, w); and the place of
+  // the item's sums (unscaled) in item_sums, or -1 to add them to the targets
+  constexpr int W = kWarps;
+  static_assert(!(RW && ITEMS), "a warp per row takes whole rows");
   constexpr int NB = batch_bodies<R, KIND>(), NA = n_chan<KIND, GS, HS>();
   constexpr int NS = slots_per_body<R, KIND>();
   constexpr bool MIXED = sizeof(R) == 4;
@@ -448,20 +450,19 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   R* B = reinterpret_cast<R*>(p2p_smem) + w * NS * NB;  // this warp's batch, NS values per body
   double* red = reinterpret_cast<double*>(p2p_smem + W * NS * NB * sizeof(R));  // [W][32 kTPT][NA]
-  constexpr bool CH = !RW && W > kWarps;  // only the wide instances take chunks
-  const bool chunked = CH && chunks != nullptr;
-  const int4 ck = chunked ? chunks[blockIdx.x] : make_int4(0, 0, 0, 0);
-  const int row = RW ? blockIdx.x * W + w : (chunked ? ck.x : (int)blockIdx.x);
+  if (ITEMS && (int)blockIdx.x >= *n_items) return;
+  const int4 it = ITEMS ? items[2 * blockIdx.x] : make_int4(0, 0, 0, 0);
+  const int row = RW ? blockIdx.x * W + w : (ITEMS ? it.x : (int)blockIdx.x);
   if (RW && row >= n_rows) return;  // whole warps: no block barrier on the RW path
   const int t = tgt_list[row];
-  const int l0 = chunked ? ck.y : off[row], l1 = chunked ? ck.z : off[row + 1];
+  const int l0 = ITEMS ? it.z : off[row], l1 = ITEMS ? it.w : off[row + 1];
   const int ts = t_start[t], tc = t_count[t];
-  // this warp's share of the row.  Vortex particles (CTA path): an equal contiguous range of
-  // the row's source bodies (leaves in row order, split inside a leaf where a range ends), so
-  // the warps reach the block's reduction together whatever the leaf sizes.  Point sources
-  // (CTA path): every W-th leaf (an even split measured no faster there, and its registers
-  // spill at the packed loop's 64).  One warp per row takes them all.
-  constexpr bool BAL = !RW && KIND == FMM_POINT_VORTEX;
+  // this warp's share of the leaves.  CTA path: an equal contiguous range of the source bodies
+  // (leaves in row order, split inside a leaf where a range ends), so the warps reach the
+  // block's reduction together whatever the leaf sizes; point sources every W-th leaf (an even
+  // split measured no faster there, and its registers spill at the packed loop's 64), except FP64
+  // items, whose few leaves do not divide evenly.  One warp per row takes them all.
+  constexpr bool BAL = !RW && (KIND == FMM_POINT_VORTEX || (!MIXED && ITEMS));
   constexpr int LS = (RW || BAL) ? 1 : W;  // stride of this warp's source leaves along the row
   int lb0 = l0 + ((RW || BAL) ? 0 : w), poff0 = 0, rem0 = INT_MAX;
   if (BAL) {
@@ -495,7 +496,7 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
   const double ox = MIXED ? t_center[3 * t] : 0.0;
   const double oy = MIXED ? t_center[3 * t + 1] : 0.0;
   const double oz = MIXED ? t_center[3 * t + 2] : 0.0;
-  for (int tile = 0; tile < tc; tile += 32 * kTPT) {
+  for (int tile = ITEMS ? it.y * 32 * kTPT : 0; tile < tc; tile += 32 * kTPT) {
     const int nt = min(tc - tile, 32 * kTPT);
     int TS = 1;
     while (TS * kTPT < nt) TS <<= 1;
@@ -777,25 +778,28 @@ __global__ void __launch_bounds__(W * 32, p2p_min_blocks<R, KIND, HS, RW, W>()) 
       }
     }
     __syncthreads();
+    const int out = ITEMS ? items[2 * blockIdx.x + 1].x : -1;
     for (int e = threadIdx.x; e < nt * NA; e += W * 32) {
       const int i = e / NA, a = e - i * NA;
       double v = 0;
 #pragma unroll
       for (int q = 0; q < W; ++q) v += red[(q * 32 * kTPT + i) * NA + a];
-      if (chunked) {
-        chunk_sums[ck.w + (int64_t)NA * (tile + i) + a] = v;
+      if (ITEMS && out >= 0) {
+        item_sums[out + e] = v;
         continue;
       }
       if (KIND == FMM_POINT_SOURCE && a == 0 && !PS) continue;
       // atomic: under SelfTuning a non-leaf target branch and its own leaves can both own direct-list rows
       atomicAdd(acc13 + 13 * (int64_t)(ts + tile + i) + chan_row<KIND, GS>(a), v * kOneOver4Pi);
     }
+    if (ITEMS) break;
     __syncthreads();
   }
 }
 
-template <class R, int KIND, bool GS, bool HS, int W = kWarps>
+template <class R, int KIND, bool GS, bool HS>
 constexpr size_t p2p_smem_bytes() {
+  constexpr int W = kWarps;
   return (size_t)W * slots_per_body<R, KIND>() * batch_bodies<R, KIND>() * sizeof(R) +
          (size_t)W * 32 * kTPT * n_chan<KIND, GS, HS>() * sizeof(double);
 }
@@ -999,24 +1003,119 @@ __global__ void k_direct_sum(const double* __restrict__ part, int n_split, int64
   }
 }
 
-// Sums of the chunks of each row (rowtab[r] = first chunk, end) in chunk order, added to the
-// row's targets: the near field of launches whose rows were cut into chunks.
+// source bodies of every row, one warp each
+__global__ void k_p2p_row_sources(const int* __restrict__ off, int rows, const int* __restrict__ src_of,
+                                  const int* __restrict__ s_count, int* __restrict__ n_src) {
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  int v = 0;
+  for (int i = off[row] + lane; i < off[row + 1]; i += 32) v += s_count[src_of[i]];
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kAll, v, o);
+  if (lane == 0) n_src[row] = v;
+}
+
+// target slots that a tile of nt targets occupies (TS lanes, kTPT each)
+__device__ __forceinline__ int tile_slots(int nt) {
+  int ts = 1;
+  while (ts * kTPT < nt) ts <<= 1;
+  return ts * kTPT;
+}
+
+// The items of a launch, one block: every tile of a row is cut into shares of about the launch's
+// work / goal slot pairs.  Items and their sums' places come from scans over the rows, so that the
+// cut, and with it the order of every sum, depends on the tree and the lists alone.
+constexpr int kPlanThreads = 1024;
+__global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict__ tgt_list,
+                                                           const int* __restrict__ off, int rows,
+                                                           const int* __restrict__ t_count,
+                                                           const int* __restrict__ n_src, int goal, int na,
+                                                           int max_sums, int4* __restrict__ items,
+                                                           int* __restrict__ n_items) {
+  __shared__ unsigned long long tot[kPlanThreads / 32];
+  __shared__ int2 sh[kPlanThreads / 32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  unsigned long long work = 0;
+  for (int r = threadIdx.x; r < rows; r += kPlanThreads) {
+    const int tc = t_count[tgt_list[r]];
+    int slots = 0;
+    for (int t = 0; t < tc; t += 32 * kTPT) slots += tile_slots(min(tc - t, 32 * kTPT));
+    work += (unsigned long long)slots * (unsigned)n_src[r];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) work += __shfl_xor_sync(kAll, work, o);
+  if (lane == 0) tot[w] = work;
+  __syncthreads();
+  work = 0;
+  for (int q = 0; q < kPlanThreads / 32; ++q) work += tot[q];
+  const unsigned long long share = work / goal + 1;
+  int2 run = make_int2(0, 0);  // items, sums of the rows before
+  for (int r0 = 0; r0 < rows; r0 += kPlanThreads) {
+    const int r = r0 + threadIdx.x;
+    int tc = 0, ns = 0, a = 0, nl = 0;
+    if (r < rows) {
+      tc = t_count[tgt_list[r]];
+      ns = n_src[r];
+      a = off[r];
+      nl = off[r + 1] - a;
+    }
+    auto cut = [&](int nt) {
+      const unsigned long long c = ((unsigned long long)tile_slots(nt) * (unsigned)ns + share - 1) / share;
+      return (int)max(1ull, min(c, (unsigned long long)min(nl, ns / kItemSources)));
+    };
+    int2 v = make_int2(0, 0);
+    for (int t = 0; t < tc; t += 32 * kTPT) {
+      const int nt = min(tc - t, 32 * kTPT), c = cut(nt);
+      v.x += c;
+      if (c > 1) v.y += c * nt * na;
+    }
+    int2 in = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(kAll, in.x, o), y = __shfl_up_sync(kAll, in.y, o);
+      if (lane >= o) in.x += x, in.y += y;
+    }
+    if (lane == 31) sh[w] = in;
+    __syncthreads();
+    int2 ex = make_int2(run.x + in.x - v.x, run.y + in.y - v.y);
+    for (int q = 0; q < kPlanThreads / 32; ++q) {
+      if (q < w) ex.x += sh[q].x, ex.y += sh[q].y;
+      run.x += sh[q].x;
+      run.y += sh[q].y;
+    }
+    __syncthreads();
+    for (int t = 0; t < tc; t += 32 * kTPT) {
+      const int nt = min(tc - t, 32 * kTPT), c = cut(nt);
+      // (the bound on the items leaves room for every row's sums)
+      const bool split = c > 1 && ex.y + c * nt * na <= max_sums;
+      for (int j = 0; j < c; ++j) {
+        const int lo = split ? a + (int)((long long)nl * j / c) : a;
+        const int hi = split ? a + (int)((long long)nl * (j + 1) / c) : (j == 0 ? a + nl : a);
+        items[2 * (ex.x + j)] = make_int4(r, t / (32 * kTPT), lo, hi);
+        items[2 * (ex.x + j) + 1] = make_int4(split ? ex.y + j * nt * na : -1, split && j == 0 ? c : 0, nt, 0);
+      }
+      ex.x += c;
+      if (c > 1) ex.y += c * nt * na;
+    }
+  }
+  if (threadIdx.x == 0) *n_items = run.x;
+}
+
+// the shares of every tile that was cut, added in order
 template <int KIND, bool PS, bool GS, int NA>
-__global__ void k_p2p_chunk_sum(const int4* __restrict__ rowtab, const int4* __restrict__ chunks,
-                                const double* __restrict__ part, const int* __restrict__ tgt_list,
-                                const int* __restrict__ t_start, const int* __restrict__ t_count,
-                                double* __restrict__ acc13) {
-  const int r = blockIdx.x;
-  const int4 rt = rowtab[r];
-  const int t = tgt_list[r];
-  const int ts = t_start[t], tc = t_count[t];
-  for (int e = threadIdx.x; e < tc * NA; e += blockDim.x) {
-    const int i = e / NA, a = e - i * NA;
-    if (KIND == FMM_POINT_SOURCE && a == 0 && !PS) continue;
+__global__ void k_p2p_sum(const int4* __restrict__ items, const int* __restrict__ n_items,
+                          const double* __restrict__ sums, const int* __restrict__ tgt_list,
+                          const int* __restrict__ t_start, double* __restrict__ acc13) {
+  if ((int)blockIdx.x >= *n_items) return;
+  const int4 a = items[2 * blockIdx.x], b = items[2 * blockIdx.x + 1];
+  if (b.y == 0) return;
+  const int first = t_start[tgt_list[a.x]] + a.y * 32 * kTPT;
+  for (int e = threadIdx.x; e < b.z * NA; e += blockDim.x) {
+    const int i = e / NA, ch = e - i * NA;
+    if (KIND == FMM_POINT_SOURCE && ch == 0 && !PS) continue;
     double v = 0.0;
-    for (int c = rt.x; c < rt.y; ++c) v += part[chunks[c].w + (int64_t)e];
-    // atomic: under SelfTuning a non-leaf target branch and its own leaves can both own rows
-    atomicAdd(acc13 + 13 * (int64_t)(ts + i) + chan_row<KIND, GS>(a), v * kOneOver4Pi);
+    for (int c = 0; c < b.y; ++c) v += sums[b.x + c * b.z * NA + e];
+    acc13[13 * (int64_t)(first + i) + chan_row<KIND, GS>(ch)] += v * kOneOver4Pi;  // the tile's only writer
   }
 }
 
@@ -1031,12 +1130,12 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   if constexpr (packed<R, KIND>()) {
     if (tt.n_bodies <= 8 * tt.n_leaves) {
       if (smem > 48 * 1024)
-        FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, true>,
+        FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, true, false>,
                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-      k_p2p<R, KIND, PS, GS, HS, true><<<(rows + kWarps - 1) / kWarps, kWarps * 32, smem, st>>>(
+      k_p2p<R, KIND, PS, GS, HS, true, false><<<(rows + kWarps - 1) / kWarps, kWarps * 32, smem, st>>>(
           L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
           stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr,
-          nullptr, exact_self);
+          nullptr, nullptr, exact_self);
       FMM_CUDA_TRY(cudaGetLastError());
       return;
     }
@@ -1044,73 +1143,48 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   int dev = 0, n_sm = 0;
   FMM_CUDA_TRY(cudaGetDevice(&dev));
   FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  // estimated body pairs of the launch: chunking costs a host round trip and a second kernel,
-  // which only pays for launches of much work (and the round trip holds back a serving
-  // worker's next launches)
+  constexpr int NA = n_chan<KIND, GS, HS>();
   const double est_pairs = (double)L.n_direct * ((double)stt.n_bodies / std::max<int64_t>(1, stt.n_leaves)) *
                            ((double)tt.n_bodies / std::max<int64_t>(1, tt.n_leaves));
-  const bool chunk = est_pairs > kChunkPairs;
-  if (rows < kWideRowsPerSM * n_sm && !chunk) {
-    constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
-    FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
-    k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<rows, kWideWarps * 32, smw, st>>>(
-        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr, nullptr,
-        exact_self);
-  } else if (rows < kWideRowsPerSM * n_sm) {
-    // few rows: cut them into chunks of about the same number of source leaves (some
-    // kChunksPerSM per SM over the launch), one wide CTA each; the chunks' partial sums are
-    // added in chunk order by k_p2p_chunk_sum
-    constexpr int NA = n_chan<KIND, GS, HS>();
-    std::vector<int> h_off(rows + 1), h_tgt(rows), h_cnt(tt.n_branches);
-    FMM_CUDA_TRY(cudaMemcpyAsync(h_off.data(), L.dir_off.ptr, (rows + 1) * sizeof(int), cudaMemcpyDeviceToHost, st));
-    FMM_CUDA_TRY(cudaMemcpyAsync(h_tgt.data(), L.dir_tgt.ptr, rows * sizeof(int), cudaMemcpyDeviceToHost, st));
-    FMM_CUDA_TRY(cudaMemcpyAsync(h_cnt.data(), tt.body_count.ptr, tt.n_branches * sizeof(int),
-                                 cudaMemcpyDeviceToHost, st));
-    FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    const int64_t total = (int64_t)h_off[rows] - h_off[0], goal = (int64_t)kChunksPerSM * n_sm;
-    const int64_t per = std::max<int64_t>(2 * kWideWarps, (total + goal - 1) / goal);
-    std::vector<int4> ch, rt(rows);
-    int64_t out = 0;
-    for (int r = 0; r < rows; ++r) {
-      const int a = h_off[r], nl = h_off[r + 1] - a;
-      const int k = (int)std::max<int64_t>(1, (nl + per - 1) / per);
-      rt[r] = make_int4((int)ch.size(), (int)ch.size() + k, 0, 0);
-      const int64_t nt = h_cnt[h_tgt[r]];
-      for (int j = 0; j < k; ++j) {
-        ch.push_back(make_int4(r, a + (int)((int64_t)nl * j / k), a + (int)((int64_t)nl * (j + 1) / k), (int)out));
-        out += nt * NA;
-        FMM_CHECK(out < INT_MAX, FMM_ERR_MEMORY, "near-field chunk sums exceed the index range");
-      }
-    }
-    // floors of a few MB: regrowing frees device memory, which waits for the whole device (and
-    // for every other context's work on it)
-    L.p2p_chunks.grow(std::max<size_t>(ch.size(), 1 << 16));
-    L.p2p_rowtab.grow(std::max<size_t>(rows, 1 << 12));
-    L.p2p_part.grow(std::max<size_t>((size_t)out + 1, 1 << 19));
-    FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_chunks.ptr, ch.data(), ch.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    FMM_CUDA_TRY(cudaMemcpyAsync(L.p2p_rowtab.ptr, rt.data(), rt.size() * sizeof(int4), cudaMemcpyHostToDevice, st));
-    constexpr size_t smw = p2p_smem_bytes<R, KIND, GS, HS, kWideWarps>();
-    FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, kWideWarps>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smw));
-    k_p2p<R, KIND, PS, GS, HS, false, kWideWarps><<<(int)ch.size(), kWideWarps * 32, smw, st>>>(
-        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, L.p2p_chunks.ptr,
-        L.p2p_part.ptr, exact_self);
-    FMM_CUDA_TRY(cudaGetLastError());
+  // rows that are not leaves (SelfTuning) can be nested, their targets' other rows adding at the
+  // same time: they keep whole rows, added with atomics
+  if (est_pairs > kItemPairs && rows <= kItemRowsPerSM * n_sm && L.rule_method != FMM_LIST_SELF_TUNING) {
+    if (smem > 48 * 1024)
+      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, true>,
+                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    int per_sm = 0;
+    FMM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p<R, KIND, PS, GS, HS, false, true>,
+                                                               kWarps * 32, smem));
+    const int goal = kItemWaves * std::max(1, per_sm) * n_sm;
+    // a tile per 64 targets begun, a share more per 1 / goal of the work; at most twice the goal of
+    // them in tiles that are cut
+    const int64_t most = rows + tt.n_bodies / (32 * kTPT) + goal + 1;
+    const int64_t sums = (int64_t)2 * goal * 32 * kTPT * NA;
+    L.p2p_items.grow(2 * (size_t)most);
+    L.p2p_meta.grow((size_t)rows + 1);
+    L.p2p_part.grow((size_t)sums);
     note_launch();
-    k_p2p_chunk_sum<KIND, PS, GS, NA><<<rows, 256, 0, st>>>(L.p2p_rowtab.ptr, L.p2p_chunks.ptr, L.p2p_part.ptr,
-                                                             L.dir_tgt.ptr, tt.body_start.ptr, tt.body_count.ptr,
-                                                             acc13);
+    k_p2p_row_sources<<<(int)((rows * 32ll + 255) / 256), 256, 0, st>>>(L.dir_off.ptr, rows, L.dir_s.ptr,
+                                                                        stt.body_count.ptr, L.p2p_meta.ptr + 1);
+    note_launch();
+    k_p2p_plan<<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
+                                           goal, NA, (int)sums, L.p2p_items.ptr, L.p2p_meta.ptr);
+    note_launch();
+    k_p2p<R, KIND, PS, GS, HS, false, true><<<(int)most, kWarps * 32, smem, st>>>(
+        L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
+        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, L.p2p_items.ptr,
+        L.p2p_meta.ptr, L.p2p_part.ptr, exact_self);
+    note_launch();
+    k_p2p_sum<KIND, PS, GS, NA><<<(int)most, 128, 0, st>>>(L.p2p_items.ptr, L.p2p_meta.ptr, L.p2p_part.ptr,
+                                                          L.dir_tgt.ptr, tt.body_start.ptr, acc13);
   } else {
     if (smem > 48 * 1024)
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false>,
+      FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, false>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    k_p2p<R, KIND, PS, GS, HS, false><<<rows, kWarps * 32, smem, st>>>(
+    k_p2p<R, KIND, PS, GS, HS, false, false><<<rows, kWarps * 32, smem, st>>>(
         L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
-        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr,
-      nullptr, exact_self);
+        stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, nullptr, nullptr, nullptr,
+        exact_self);
   }
   FMM_CUDA_TRY(cudaGetLastError());
 }

@@ -85,3 +85,27 @@ def test_f64_overflowing_gradient_keeps_the_potential(ctx):
     v, m = sums(b[:, :3], b, False)[0]
     assert np.all(abs(out[:, 3] - v) <= 4 * (80 + 16) * EPS * m)
     assert not np.all(np.isfinite(out[:, 4:7]))
+
+
+@pytest.mark.parametrize("kind,hess", [(1, False), (3, False), (3, True)])
+@pytest.mark.parametrize("leaf,ls_t", [(16, 3), (60, 47), (150, 20)])
+def test_items_cover_every_pair(ctx, kind, hess, leaf, ls_t):
+    """Enough pairs for the launch to be cut into items: rows of several target tiles, ragged tiles, and
+    rows of a few targets with thousands of sources."""
+    b = bodies(4111, kind, 1.0, 31)
+    pos = np.concatenate([bodies(1100, kind, 0.2, 32)[:, :3], bodies(37, kind, 3.0, 33)[:, :3], b[:64, :3]])
+    res = {}
+    for prec in ("f64", "mixed"):
+        opt = fm.make_options(expansion_order=3, leaf_size_source=leaf, leaf_size_target=ls_t,
+                              scalar_potential=kind == 1, hessian=hess, farfield=False, multipole_acceptance=1e-9,
+                              precision=prec)
+        res[prec], _ = fm.solve_buffers(b, kind, opt, pos, ctx=ctx)
+    for cols, ref in zip((slice(3, 4), slice(4, 7), slice(7, 16)), sums(pos, b, hess)):
+        if ref is None:
+            continue
+        got = res["f64"][:, cols].reshape(np.shape(ref[0]))
+        assert np.all(abs(got - ref[0]) <= 4 * (len(b) + 16) * EPS * ref[1])
+        # FP32 coordinates relative to a target leaf: 2^-24 of its extent against the distances of a
+        # few thousand bodies in a unit cube (about 1e-2), order 5
+        mixed = res["mixed"][:, cols].reshape(np.shape(ref[0]))
+        assert np.linalg.norm(mixed - got) <= 1e-4 * np.linalg.norm(got)
