@@ -14,6 +14,7 @@
 // summing blocks of sources in FP32 and the block partials in FP64.
 #include <climits>
 #include <algorithm>
+#include <type_traits>
 
 #include "context.cuh"
 
@@ -411,6 +412,27 @@ __device__ __noinline__ void self_batch_f64_vortex(const double2* __restrict__ B
   }
 }
 
+// Targets per lane of a tile of nt targets on the FP64 path: three where 3 x a power of two lanes
+// leave fewer slots empty than 2 x (nt in (2^k, 3/2 2^k]).  Leaves are split by eight, so their sizes
+// spread over a factor of eight and the slots matter: slots per pair 1.24 -> 1.11 (1e6 clustered
+// bodies), 1.36 -> 1.15 (1e4 uniform).
+__host__ __device__ __forceinline__ int targets_per_lane(int nt) {
+  int n2 = 1, n3 = 1;
+  while (n2 * 2 < nt) n2 <<= 1;
+  while (n3 * 3 < nt) n3 <<= 1;
+  return n3 * 3 < n2 * 2 ? 3 : 2;
+}
+template <class R, int KIND, bool HS>
+__host__ __device__ constexpr int max_targets_per_lane() {
+  return sizeof(R) == 4 || (KIND == FMM_POINT_VORTEX && HS) ? kTPT : 3;
+}
+template <int N>
+__device__ __forceinline__ double pick(const double (&v)[N], int q) {
+  return q == 0 ? v[0] : q == 1 ? v[1] : v[N - 1];
+}
+template <int N>
+__device__ __forceinline__ double pick(const float (&v)[N], int) { return v[0]; }
+
 // RW: one warp per row (rows of small leaves, kWarps rows per CTA), the warp adding its
 // sums to the targets itself; otherwise one CTA per row or item, the warps splitting its sources.
 // resident CTAs of the mixed instances: the registers the packed loop needs (the FP64
@@ -420,7 +442,7 @@ __device__ __noinline__ void self_batch_f64_vortex(const double2* __restrict__ B
 template <class R, int KIND, bool HS, bool RW>
 __host__ __device__ constexpr int p2p_min_blocks() {
   constexpr int regs = (KIND == FMM_POINT_VORTEX && HS) ? (RW ? 168 : 128) : (RW ? 72 : 64);
-  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW) ? 3 : 1;
+  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW) ? 3 : 4;
   return 65536 / (regs * kWarps * 32);
 }
 
@@ -441,6 +463,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
   constexpr int NB = batch_bodies<R, KIND>(), NA = n_chan<KIND, GS, HS>();
   constexpr int NS = slots_per_body<R, KIND>();
   constexpr bool MIXED = sizeof(R) == 4;
+  constexpr int KT = max_targets_per_lane<R, KIND, HS>();
   constexpr bool PACK = packed<R, KIND>();
   constexpr bool PACKV = packed_vortex<R, KIND>();
   // vortex particles with the gradient on the FP64 path sum it as two parts per target
@@ -498,13 +521,14 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
   const double oz = MIXED ? t_center[3 * t + 2] : 0.0;
   for (int tile = ITEMS ? it.y * 32 * kTPT : 0; tile < tc; tile += 32 * kTPT) {
     const int nt = min(tc - tile, 32 * kTPT);
+    const int tpt = KT == 3 ? targets_per_lane(nt) : kTPT;
     int TS = 1;
-    while (TS * kTPT < nt) TS <<= 1;
+    while (TS * tpt < nt) TS <<= 1;
     const int ti = lane & (TS - 1), slice = lane / TS, SS = 32 / TS;
-    R tx[kTPT], ty[kTPT], tz[kTPT];
+    R tx[KT], ty[KT], tz[KT];
     int tfar = 0;  // FP64: largest high word of the lane's target coordinates
 #pragma unroll
-    for (int k = 0; k < kTPT; ++k) {
+    for (int k = 0; k < KT; ++k) {
       tx[k] = ty[k] = tz[k] = R(0);
       int i = ti + k * TS;
       if (i < nt) {
@@ -515,13 +539,13 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
         tz[k] = (R)(p.z - oz);
       }
     }
-    R part[kTPT][NA];
-    double tot[kTPT][NA];
-    R us[kTPT][3], Qs[kTPT][9], Es[kTPT][3];  // FP64 vortex particles: velocity, gradient as two sums
+    R part[KT][NA];
+    double tot[KT][NA];
+    R us[KT][3], Qs[KT][9], Es[KT][3];  // FP64 vortex particles: velocity, gradient as two sums
     // FP64: a second pass in the general arithmetic when the first meets a pair out of its range
     for (bool general = false;; general = true) {
 #pragma unroll
-      for (int k = 0; k < kTPT; ++k) {
+      for (int k = 0; k < KT; ++k) {
 #pragma unroll
         for (int a = 0; a < NA; ++a) part[k][a] = R(0), tot[k][a] = 0.0;
 #pragma unroll
@@ -691,34 +715,75 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
         } else if constexpr (KIND == FMM_POINT_SOURCE) {
           const double4* Bd = reinterpret_cast<const double4*>(B);
           if (general || __any_sync(kAll, max(far, tfar) >= kFarHi)) {
-            const double gx[2] = {tx[0], tx[1]}, gy[2] = {ty[0], ty[1]}, gz[2] = {tz[0], tz[1]};
-            self_batch_f64_source<PS, NA>(Bd, slice, nb, SS, gx, gy, gz, tot);
-          } else {
-#pragma unroll 2
-            for (int j = slice; j < nb; j += SS) {
-              const double4 b = Bd[j];
+            // two targets of the lane at a time (the third twice, counted once)
+#pragma unroll 1
+            for (int q = 0; q < tpt; q += 2) {
+              const int q1 = min(q + 1, tpt - 1);
+              const double gx[2] = {pick(tx, q), pick(tx, q1)}, gy[2] = {pick(ty, q), pick(ty, q1)};
+              const double gz[2] = {pick(tz, q), pick(tz, q1)};
+              double g2[2][NA];
 #pragma unroll
-              for (int k = 0; k < kTPT; ++k) source_pair_f64<PS>(tx[k], ty[k], tz[k], b.x, b.y, b.z, b.w, part[k]);
+              for (int a = 0; a < NA; ++a) g2[0][a] = g2[1][a] = 0.0;
+              self_batch_f64_source<PS, NA>(Bd, slice, nb, SS, gx, gy, gz, g2);
+#pragma unroll
+              for (int k = 0; k < KT; ++k)
+                if (k == q || (k == q + 1 && q1 == q + 1))
+#pragma unroll
+                  for (int a = 0; a < NA; ++a) tot[k][a] += g2[k == q ? 0 : 1][a];
             }
+          } else {
+auto pairs = [&](auto n) {
+#pragma unroll 2
+              for (int j = slice; j < nb; j += SS) {
+                const double4 b = Bd[j];
+#pragma unroll
+                for (int k = 0; k < n.value; ++k) source_pair_f64<PS>(tx[k], ty[k], tz[k], b.x, b.y, b.z, b.w, part[k]);
+              }
+            };
+            if (tpt == 3)
+              pairs(std::integral_constant<int, KT>());
+            else
+              pairs(std::integral_constant<int, 2>());
           }
         } else {
           const double2* Bd = reinterpret_cast<const double2*>(B);
           if (general || __any_sync(kAll, max(far, tfar) >= kFarHi)) {
-            const double gx[2] = {tx[0], tx[1]}, gy[2] = {ty[0], ty[1]}, gz[2] = {tz[0], tz[1]};
-            self_batch_f64_vortex<GS, HS, NA>(Bd, slice, nb, SS, gx, gy, gz, tot);
+            if constexpr (KT == 2) {
+              const double gx[2] = {tx[0], tx[1]}, gy[2] = {ty[0], ty[1]}, gz[2] = {tz[0], tz[1]};
+              self_batch_f64_vortex<GS, HS, NA>(Bd, slice, nb, SS, gx, gy, gz, tot);
+            } else {
+              // two targets of the lane at a time (the third twice, counted once)
+#pragma unroll 1
+              for (int q = 0; q < tpt; q += 2) {
+                const int q1 = min(q + 1, tpt - 1);
+                const double gx[2] = {pick(tx, q), pick(tx, q1)}, gy[2] = {pick(ty, q), pick(ty, q1)};
+                const double gz[2] = {pick(tz, q), pick(tz, q1)};
+                double g2[2][NA];
+#pragma unroll
+                for (int a = 0; a < NA; ++a) g2[0][a] = g2[1][a] = 0.0;
+                self_batch_f64_vortex<GS, HS, NA>(Bd, slice, nb, SS, gx, gy, gz, g2);
+#pragma unroll
+                for (int k = 0; k < KT; ++k)
+                  if (k == q || (k == q + 1 && q1 == q + 1))
+#pragma unroll
+                    for (int a = 0; a < NA; ++a) tot[k][a] += g2[k == q ? 0 : 1][a];
+              }
+            }
           } else {
+            // (two targets: a third costs the gradient's kernel its registers, 25.5 -> 29.4 ms on the 300k ring)
             for (int j = slice; j < nb; j += SS) {
               const double2 a = Bd[3 * j], b = Bd[3 * j + 1], c = Bd[3 * j + 2];
 #pragma unroll
-              for (int k = 0; k < kTPT; ++k)
-                vortex_pair_f64<GS, HS>(tx[k], ty[k], tz[k], a.x, a.y, b.x, b.y, c.x, c.y, us[k], Qs[k], Es[k]);
+              for (int k = 0; k < KT; ++k)
+                if (KT == 2 || k < tpt)
+                  vortex_pair_f64<GS, HS>(tx[k], ty[k], tz[k], a.x, a.y, b.x, b.y, c.x, c.y, us[k], Qs[k], Es[k]);
             }
           }
         }
         __syncwarp();
         if (MIXED) {
 #pragma unroll
-          for (int k = 0; k < kTPT; ++k)
+          for (int k = 0; k < KT; ++k)
 #pragma unroll
             for (int a = 0; a < NA; ++a) tot[k][a] += (double)part[k][a], part[k][a] = R(0);
         }
@@ -728,7 +793,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
       } else {
         bool finite = true;
 #pragma unroll
-        for (int k = 0; k < kTPT; ++k) {
+        for (int k = 0; k < KT; ++k) {
           if constexpr (KIND == FMM_POINT_VORTEX && GS) {
 #pragma unroll
             for (int a = 0; a < 3; ++a) part[k][a % NA] = us[k][a];
@@ -749,14 +814,14 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
     // slices -> lanes ti (< TS), then warps -> shared memory
     for (int o = TS; o < 32; o <<= 1)
 #pragma unroll
-      for (int k = 0; k < kTPT; ++k)
+      for (int k = 0; k < KT; ++k)
 #pragma unroll
         for (int a = 0; a < NA; ++a) tot[k][a] += __shfl_xor_sync(kAll, tot[k][a], o);
     if constexpr (RW) {
       // one warp owns the row: its sums go to the targets directly
       if (slice == 0) {
 #pragma unroll
-        for (int k = 0; k < kTPT; ++k) {
+        for (int k = 0; k < KT; ++k) {
           const int i = ti + k * TS;
           if (i < nt)
 #pragma unroll
@@ -770,7 +835,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
     }
     if (slice == 0) {
 #pragma unroll
-      for (int k = 0; k < kTPT; ++k) {
+      for (int k = 0; k < KT; ++k) {
         int i = ti + k * TS;
         if (i < nt)
 #pragma unroll
@@ -1015,11 +1080,12 @@ __global__ void k_p2p_row_sources(const int* __restrict__ off, int rows, const i
   if (lane == 0) n_src[row] = v;
 }
 
-// target slots that a tile of nt targets occupies (TS lanes, kTPT each)
-__device__ __forceinline__ int tile_slots(int nt) {
+// target slots that a tile of nt targets occupies (three: the FP64 kernels' choice of targets per lane)
+__device__ __forceinline__ int tile_slots(int nt, bool three) {
+  const int tpt = three ? targets_per_lane(nt) : kTPT;
   int ts = 1;
-  while (ts * kTPT < nt) ts <<= 1;
-  return ts * kTPT;
+  while (ts * tpt < nt) ts <<= 1;
+  return ts * tpt;
 }
 
 // The items of a launch, one block: every tile of a row is cut into shares of about the launch's
@@ -1030,7 +1096,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
                                                            const int* __restrict__ off, int rows,
                                                            const int* __restrict__ t_count,
                                                            const int* __restrict__ n_src, int goal, int na,
-                                                           int max_sums, int4* __restrict__ items,
+                                                           int max_sums, int three, int4* __restrict__ items,
                                                            int* __restrict__ n_items) {
   __shared__ unsigned long long tot[kPlanThreads / 32];
   __shared__ int2 sh[kPlanThreads / 32];
@@ -1039,7 +1105,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
   for (int r = threadIdx.x; r < rows; r += kPlanThreads) {
     const int tc = t_count[tgt_list[r]];
     int slots = 0;
-    for (int t = 0; t < tc; t += 32 * kTPT) slots += tile_slots(min(tc - t, 32 * kTPT));
+    for (int t = 0; t < tc; t += 32 * kTPT) slots += tile_slots(min(tc - t, 32 * kTPT), three != 0);
     work += (unsigned long long)slots * (unsigned)n_src[r];
   }
 #pragma unroll
@@ -1060,7 +1126,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       nl = off[r + 1] - a;
     }
     auto cut = [&](int nt) {
-      const unsigned long long c = ((unsigned long long)tile_slots(nt) * (unsigned)ns + share - 1) / share;
+      const unsigned long long c = ((unsigned long long)tile_slots(nt, three != 0) * (unsigned)ns + share - 1) / share;
       return (int)max(1ull, min(c, (unsigned long long)min(nl, ns / kItemSources)));
     };
     int2 v = make_int2(0, 0);
@@ -1168,7 +1234,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
                                                                         stt.body_count.ptr, L.p2p_meta.ptr + 1);
     note_launch();
     k_p2p_plan<<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
-                                           goal, NA, (int)sums, L.p2p_items.ptr, L.p2p_meta.ptr);
+                                           goal, NA, (int)sums, max_targets_per_lane<R, KIND, HS>() == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
     note_launch();
     k_p2p<R, KIND, PS, GS, HS, false, true><<<(int)most, kWarps * 32, smem, st>>>(
         L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,

@@ -662,8 +662,12 @@ template <class F>
 void dispatch_pmax(int p, F&& f) {
   if (p <= 4)
     f.template go<4>();
+  else if (p <= 6)
+    f.template go<6>();
   else if (p <= 8)
     f.template go<8>();
+  else if (p <= 10)
+    f.template go<10>();
   else if (p <= 12)
     f.template go<12>();
   else if (p <= 16)
