@@ -420,10 +420,12 @@ DevTree view_tree(const DevTree& S, const SysView& v) {
   return t;
 }
 
+// host_out: copy the target buffer there before the call's one wait at its end
 // is_estimate: the influence estimate's sub-solve, whose out16 receives one value per body
 // (get_influence: the scalar potential when influence_potential, else |gradient|)
 void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, double* out16, fmm_result* res,
-             bool is_estimate, cudaStream_t st, Scratch& sc, DevBuf<int>& stats, bool influence_potential = false) {
+             bool is_estimate, cudaStream_t st, Scratch& sc, DevBuf<int>& stats, bool influence_potential = false,
+             double* host_out = nullptr) {
   const int p = o.expansion_order;
   const bool multi = in.n_sys > 1;
   // lamb_helmholtz = has_vector_potential(source_systems) (src/fmm.jl:927)
@@ -582,7 +584,8 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
                c->tables, o.precision, fs);
   markf(3);
   if (!split) mark(6);
-  if (o.downward_pass) {
+  // no translation into the locals: they are zero, and so is what the downward pass would add
+  if (o.downward_pass && o.horizontal_pass && W.lists.n_m2l > 0) {
     launch_l2l(T, p, lh, fs);
     launch_l2p(T, p, lh, ps, gs, hs, far13, fs);
   }
@@ -601,6 +604,8 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
                                                     split ? far13 : nullptr);
   FMM_CUDA_TRY(cudaGetLastError());
   mark(7);
+  if (host_out)
+    FMM_CUDA_TRY(cudaMemcpyAsync(host_out, out16, 16 * T.n_bodies * sizeof(double), cudaMemcpyDeviceToHost, st));
   if (res) {
     int h[6] = {0, 0, 0, 0, 0, 0};
     FMM_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -915,16 +920,13 @@ int fmm_solve(fmm_ctx* c, const fmm_target_system* target, const fmm_source_syst
       in.tpos = stage(c, c->stage_t, target->positions, (size_t)target->stride * target->n_bodies, target->memory);
       in.t_stride = target->stride;
     }
-    c->out16.grow(16 * (size_t)in.n_t);
-    run_fmm(c, c->main, in, *opt, c->out16.ptr, result, false, c->stream, c->sc, c->stats);
-    // write the target buffer (rows 1..3 = positions, 4..16 = phi, gradient, hessian)
-    int mem = target->memory;
-    double* dst = target->out;
-    if (mem == FMM_MEMORY_DEVICE)
-      FMM_CUDA_TRY(cudaMemcpyAsync(dst, c->out16.ptr, 16 * in.n_t * sizeof(double), cudaMemcpyDeviceToDevice, c->stream));
-    else
-      FMM_CUDA_TRY(cudaMemcpyAsync(dst, c->out16.ptr, 16 * in.n_t * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    FMM_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    // the target buffer (rows 1..3 = positions, 4..16 = phi, gradient, hessian): device memory is
+    // written by the solve's last kernel, which runs after everything that reads the inputs
+    const bool on_device = target->memory == FMM_MEMORY_DEVICE;
+    if (!on_device) c->out16.grow(16 * (size_t)in.n_t);
+    run_fmm(c, c->main, in, *opt, on_device ? target->out : c->out16.ptr, result, false, c->stream, c->sc, c->stats,
+            false, on_device ? nullptr : target->out);
+    if (!result) FMM_CUDA_TRY(cudaStreamSynchronize(c->stream));  // (with a result the solve has waited for it)
     c->have_solve = true;
     c->last_p = opt->expansion_order;
     c->last_kind = source->kind;
@@ -1226,7 +1228,7 @@ int fmm_get_lists(fmm_ctx* c, int32_t* m2l, int64_t* n_m2l, int32_t* direct, int
     if (n_direct) *n_direct = L.n_direct;
     if (m2l || direct) {
       FMM_CUDA_TRY(cudaSetDevice(c->device));
-      export_lists_reference_order(L, c->main.target(), c->main.source(), c->sc, c->stream, m2l, direct);
+      export_lists_reference_order(L, c->main.source(), c->sc, c->stream, m2l, direct);
     }
     return FMM_OK;
   } catch (const Error& e) {

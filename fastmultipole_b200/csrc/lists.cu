@@ -133,8 +133,8 @@ __device__ __forceinline__ void count_targets(bool on, int t, int lane, int* __r
   if (on && lane == __ffs(grp) - 1) atomicAdd(cnt + t, __popc(grp));
 }
 
-constexpr int kStepItems = 4;                              // pairs per thread and chunk
-constexpr int kStepChunk = kStepThreads * kStepItems;      // pairs per block and chunk
+constexpr int kStepItems = 4;                              // pairs per thread and chunk (most)
+constexpr int kStepChunk = kStepThreads * kStepItems;      // pairs per block and chunk (most)
 
 // Step k of the traversal: every pair of the frontier (ctr[k] pairs) is decided;
 // direct and M2L pairs go to the raw lists and count for their target, split
@@ -161,7 +161,9 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
   const int n = min(ctr[k], cap_f);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   bool bad = false;
-  for (int c0 = blockIdx.x * kStepChunk; c0 < n; c0 += gridDim.x * kStepChunk) {
+  // a frontier that the launch's threads cover takes one pair per thread
+  const int items = n > (int)gridDim.x * kStepThreads ? kStepItems : 1, chunk = items * kStepThreads;
+  for (int c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
     int2 p[kStepItems];
     int a[kStepItems], nn[kStepItems], ch[kStepItems];
     int cd = 0, cm = 0, cf = 0;
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
       a[r] = A_NONE;
       nn[r] = 0;
       ch[r] = 0;
-      if (i < n) {
+      if (r < items && i < n) {
         p[r] = fin[i];
         a[r] = decide(T, p[r].x, S, p[r].y, R, nn[r], ch[r]);
       }
@@ -223,8 +225,10 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
         }
         of += nn[r];
       }
-      count_targets(a[r] == A_DIRECT, p[r].x, lane, cdir);
-      count_targets(a[r] == A_M2L, p[r].x, lane, cm2l);
+      if (r < items) {
+        count_targets(a[r] == A_DIRECT, p[r].x, lane, cdir);
+        count_targets(a[r] == A_M2L, p[r].x, lane, cm2l);
+      }
     }
     __syncthreads();  // wsum / bbase are rewritten by the next chunk
   }
@@ -536,7 +540,7 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
       // grid from this scratch's previous build (the kernel strides over any frontier)
       const int64_t hint = k < (int)sc.step_hint.size() ? sc.step_hint[k] : (int64_t)kStepChunk * kStepMaxBlocks;
       note_launch();
-      k_step<<<blocks_for(hint + hint / 4 + 32, kStepChunk), kStepThreads, 0, st>>>(
+      k_step<<<blocks_for(hint + hint / 4 + 32, kStepThreads), kStepThreads, 0, st>>>(
           fin, fout, k, T, S, R, sc.dir_raw.ptr, sc.m2l_raw.ptr, cnt_d, cnt_m, ctr, cf, cd, cm);
       FMM_CUDA_TRY(cudaGetLastError());
     }
@@ -613,144 +617,145 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
   L.n_m2l = n_m2l;
   L.n_dir_targets = rows[0];
   L.n_m2l_targets = rows[1];
-  L.rule_mac = mac;
-  L.rule_ls = leaf_size_source;
   L.rule_method = method;
-  L.rule_ff = ff;
-  L.rule_nf = nf;
-  L.rule_si = si;
 }
 
 namespace {
 
-constexpr int kMaxDepth = 24;      // ancestor chain of a branch (the octant key allows 21 levels)
-constexpr int kStepsPerWord = 21;  // 3 bits per step, 63 bits per key word
+// The reference's recursion reaches the pairs of one target in the depth-first order of their
+// sources: the paths of (t, s1) and (t, s2) from (root, root) are the same, split by split, up to
+// the pair that splits the lowest common ancestor of s1 and s2 on the source side, where the
+// children are taken in order.  The sources of a row are disjoint, so that order is the order of
+// their first bodies: rows are sorted by (first body, source).
+struct ExportRows {
+  const int *tgt, *off, *src, *first_body;
+  int2* out;
+};
+using ExportKey = unsigned long long;
+__device__ __forceinline__ ExportKey export_key(const ExportRows& E, int i) {
+  const int s = E.src[i];
+  return ((ExportKey)(unsigned)E.first_body[s] << 32) | (unsigned)s;
+}
+struct ExportLess {
+  __device__ __forceinline__ bool operator()(ExportKey a, ExportKey b) const { return a < b; }
+};
+constexpr int kExportRow = 4096;  // longest row of the block sort
 
-// Depth-first rank of every pair: the reference's recursion (src/interaction_list.jl:3-166)
-// reaches (t, s) from (root, root) by one split per step, each into the child that is an
-// ancestor of t (target split) or of s (source split); the side is the rule's decision at
-// that pair.  The child ordinals along the way (3 bits each, first step most significant)
-// order the pairs as the recursion emits them (no emitted pair's path is a prefix of
-// another's, so zero padding keeps the order).  An inconsistent path raises the flag.
-__global__ void k_dfs_keys(const int* __restrict__ lt, const int* __restrict__ ls, int n, TreeRef T, TreeRef S,
-                           const int* __restrict__ parent_t, const int* __restrict__ parent_s, Rule R,
-                           unsigned long long* __restrict__ khi, unsigned long long* __restrict__ klo,
-                           int* __restrict__ perm, int* __restrict__ flag) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    int ct[kMaxDepth], cs[kMaxDepth];
-    int nt = 0, ns = 0;
-    for (int a = lt[i]; a >= 0 && nt < kMaxDepth; a = parent_t[a]) ct[nt++] = a;
-    for (int b = ls[i]; b >= 0 && ns < kMaxDepth; b = parent_s[b]) cs[ns++] = b;
-    unsigned long long hi = 0, lo = 0;
-    bool bad = ct[nt - 1] != 0 || cs[ns - 1] != 0;
-    int it = nt - 1, is = ns - 1, step = 0;
-    while (!bad && (it > 0 || is > 0)) {
-      int nn, c0;
-      const int act = decide(T, ct[it], S, cs[is], R, nn, c0);
-      int ord;
-      if (act == A_SPLIT_T && it > 0) {
-        ord = ct[it - 1] - c0;
-        --it;
-      } else if (act == A_SPLIT_S && is > 0) {
-        ord = cs[is - 1] - c0;
-        --is;
-      } else {
-        bad = true;
-        break;
-      }
-      if (ord < 0 || ord >= nn || ord > 7 || step >= 2 * kStepsPerWord) {
-        bad = true;
-        break;
-      }
-      if (step < kStepsPerWord)
-        hi |= (unsigned long long)ord << (3 * (kStepsPerWord - 1 - step));
-      else
-        lo |= (unsigned long long)ord << (3 * (2 * kStepsPerWord - 1 - step));
-      ++step;
+// rows of up to 128 entries: a warp each
+__global__ void __launch_bounds__(kSortWarps * 32) k_export_warp(ExportRows E, int rows) {
+  using WMS = cub::WarpMergeSort<ExportKey, 4, 32>;
+  __shared__ typename WMS::TempStorage tmp[kSortWarps];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r = blockIdx.x * kSortWarps + w; r < rows; r += gridDim.x * kSortWarps) {
+    const int b = E.off[r], len = E.off[r + 1] - b, t = E.tgt[r];
+    if (len > 128) continue;
+    ExportKey k[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) k[j] = lane * 4 + j < len ? export_key(E, b + lane * 4 + j) : ~0ull;
+    WMS(tmp[w]).Sort(k, ExportLess(), len, ~0ull);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (lane * 4 + j < len) E.out[b + lane * 4 + j] = make_int2(t, (int)(unsigned)k[j]);
+    __syncwarp();
+  }
+}
+// rows of more than LO and up to THREADS x ITEMS entries: a block each
+template <int THREADS, int ITEMS, int LO>
+__global__ void __launch_bounds__(THREADS) k_export_block(ExportRows E, int rows) {
+  using BMS = cub::BlockMergeSort<ExportKey, THREADS, ITEMS>;
+  __shared__ typename BMS::TempStorage tmp;
+  for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int b = E.off[r], len = E.off[r + 1] - b, t = E.tgt[r];
+    if (len <= LO || len > THREADS * ITEMS) continue;
+    ExportKey k[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int i = threadIdx.x * ITEMS + j;
+      k[j] = i < len ? export_key(E, b + i) : ~0ull;
     }
-    if (bad) atomicExch(flag, 1);
-    khi[i] = hi;
-    klo[i] = lo;
-    perm[i] = i;
+    BMS(tmp).Sort(k, ExportLess(), len, ~0ull);
+#pragma unroll
+    for (int j = 0; j < ITEMS; ++j) {
+      const int i = threadIdx.x * ITEMS + j;
+      if (i < len) E.out[b + i] = make_int2(t, (int)(unsigned)k[j]);
+    }
+    __syncthreads();
   }
 }
-
-__global__ void k_permute_u64(const unsigned long long* __restrict__ in, const int* __restrict__ perm, int n,
-                              unsigned long long* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = in[perm[i]];
+// longer rows: keys for a segmented sort, and its result as pairs (rows of up to kExportRow are done)
+__global__ void k_export_keys(ExportRows E, int n, ExportKey* __restrict__ keys) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) keys[i] = export_key(E, i);
 }
-
-__global__ void k_gather_pairs(const int* __restrict__ lt, const int* __restrict__ ls, const int* __restrict__ perm,
-                               int n, int2* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int j = perm[i];
-    out[i] = make_int2(lt[j], ls[j]);
-  }
+__global__ void k_export_long(ExportRows E, const ExportKey* __restrict__ keys) {
+  const int r = blockIdx.x, b = E.off[r], e = E.off[r + 1], t = E.tgt[r];
+  if (e - b <= kExportRow) return;
+  for (int i = b + threadIdx.x; i < e; i += blockDim.x) E.out[i] = make_int2(t, (int)(unsigned)keys[i]);
+}
+// the longest row
+__global__ void k_longest_row(const int* __restrict__ off, int rows, int* __restrict__ longest) {
+  int m = 0;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x)
+    m = max(m, off[r + 1] - off[r]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(kFull, m, o));
+  if ((threadIdx.x & 31) == 0) atomicMax(longest, m);
 }
 
 }  // namespace
 
-void export_lists_reference_order(const DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc,
-                                  cudaStream_t st, int32_t* m2l, int32_t* direct) {
-  const int nt = (int)tt.n_branches, ns = (int)stt.n_branches;
-  sc.node_geo_t.grow((size_t)nt);
-  sc.node_info_t.grow((size_t)nt);
-  sc.node_geo_s.grow((size_t)ns);
-  sc.node_info_s.grow((size_t)ns);
-  note_launch();
-  k_pack_nodes<<<dim3(blocks_for(std::max(nt, ns), 256), 2), 256, 0, st>>>(target_nodes(tt, sc), source_nodes(stt, sc),
-                                                                            nullptr, nullptr);
-  FMM_CUDA_TRY(cudaGetLastError());
-  const TreeRef T{sc.node_geo_t.ptr, sc.node_info_t.ptr};
-  const TreeRef S{sc.node_geo_s.ptr, sc.node_info_s.ptr};
-  const Rule R{L.rule_mac, L.rule_ls, L.rule_method, L.rule_ff, L.rule_nf, L.rule_si};
+void export_lists_reference_order(const DevLists& L, const DevTree& stt, Scratch& sc, cudaStream_t st, int32_t* m2l,
+                                  int32_t* direct) {
   struct One {
-    const DevBuf<int>*t, *s, *off;
+    const DevBuf<int>*tgt, *s, *off;
     int64_t n, rows;
     int32_t* dst;
-  } lists[2] = {{&L.m2l_t, &L.m2l_s, &L.m2l_off, L.n_m2l, L.n_m2l_targets, m2l},
-                {&L.dir_t, &L.dir_s, &L.dir_off, L.n_direct, L.n_dir_targets, direct}};
-  sc.flag.grow(1);
-  for (const One& q : lists) {
+  } lists[2] = {{&L.m2l_tgt, &L.m2l_s, &L.m2l_off, L.n_m2l, L.n_m2l_targets, m2l},
+                {&L.dir_tgt, &L.dir_s, &L.dir_off, L.n_direct, L.n_dir_targets, direct}};
+  sc.flag.grow(2);
+  FMM_CUDA_TRY(cudaMemsetAsync(sc.flag.ptr, 0, 2 * sizeof(int), st));
+  for (int q = 0; q < 2; ++q) {
+    if (!lists[q].dst || lists[q].n == 0) continue;
+    note_launch();
+    k_longest_row<<<blocks_for(lists[q].rows, 256), 256, 0, st>>>(lists[q].off->ptr, (int)lists[q].rows,
+                                                                  sc.flag.ptr + q);
+  }
+  int longest[2] = {0, 0};
+  FMM_CUDA_TRY(cudaMemcpyAsync(longest, sc.flag.ptr, sizeof(longest), cudaMemcpyDeviceToHost, st));
+  FMM_CUDA_TRY(cudaStreamSynchronize(st));
+  for (int k = 0; k < 2; ++k) {
+    const One& q = lists[k];
     if (!q.dst || q.n == 0) continue;
     const int n = (int)q.n, rows = (int)q.rows;
-    sc.keys_a.grow(2 * (size_t)n);
-    sc.keys_b.grow(2 * (size_t)n);
-    sc.vals_a.grow((size_t)n);
-    sc.vals_b.grow((size_t)n);
-    unsigned long long *hi = sc.keys_a.ptr, *lo = sc.keys_a.ptr + n, *k1 = sc.keys_b.ptr, *k2 = sc.keys_b.ptr + n;
-    FMM_CUDA_TRY(cudaMemsetAsync(sc.flag.ptr, 0, sizeof(int), st));
-    note_launch();
-    k_dfs_keys<<<blocks_for(n, 256), 256, 0, st>>>(q.t->ptr, q.s->ptr, n, T, S, tt.parent.ptr, stt.parent.ptr, R, hi,
-                                                  lo, sc.vals_a.ptr, sc.flag.ptr);
-    FMM_CUDA_TRY(cudaGetLastError());
-    // lexicographic (hi, lo) inside every row: stable sort by lo, then stable sort by hi
-    const int* beg = q.off->ptr;
-    const int* end = q.off->ptr + 1;
-    size_t tb = 0, tb2 = 0;
-    FMM_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(nullptr, tb, lo, k1, sc.vals_a.ptr, sc.vals_b.ptr, n, rows,
-                                                           beg, end, st));
-    FMM_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(nullptr, tb2, hi, k2, sc.vals_b.ptr, sc.vals_a.ptr, n,
-                                                           rows, beg, end, st));
-    sc.cub.grow(std::max(tb, tb2));
-    note_launch();
-    FMM_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(sc.cub.ptr, tb, lo, k1, sc.vals_a.ptr, sc.vals_b.ptr, n,
-                                                           rows, beg, end, st));
-    // the second pass needs the hi keys in the order of the first: gather them
-    note_launch();
-    k_permute_u64<<<blocks_for(n, 256), 256, 0, st>>>(hi, sc.vals_b.ptr, n, lo);
-    note_launch();
-    FMM_CUDA_TRY(cub::DeviceSegmentedSort::StableSortPairs(sc.cub.ptr, tb2, lo, k2, sc.vals_b.ptr, sc.vals_a.ptr, n,
-                                                           rows, beg, end, st));
     sc.front_a.grow((size_t)n);
+    const ExportRows E{q.tgt->ptr, q.off->ptr, q.s->ptr, stt.body_start.ptr, sc.front_a.ptr};
     note_launch();
-    k_gather_pairs<<<blocks_for(n, 256), 256, 0, st>>>(q.t->ptr, q.s->ptr, sc.vals_a.ptr, n, sc.front_a.ptr);
+    k_export_warp<<<blocks_for((int64_t)rows * 32, kSortWarps * 32), kSortWarps * 32, 0, st>>>(E, rows);
+    if (longest[k] > 128) {
+      note_launch();
+      k_export_block<128, 4, 128><<<std::min(rows, kStepMaxBlocks), 128, 0, st>>>(E, rows);
+    }
+    if (longest[k] > 512) {
+      note_launch();
+      k_export_block<256, 16, 512><<<std::min(rows, kStepMaxBlocks), 256, 0, st>>>(E, rows);
+    }
     FMM_CUDA_TRY(cudaGetLastError());
-    int bad = 0;
-    FMM_CUDA_TRY(cudaMemcpyAsync(&bad, sc.flag.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (longest[k] > kExportRow) {
+      sc.keys_a.grow((size_t)n);
+      sc.keys_b.grow((size_t)n);
+      note_launch();
+      k_export_keys<<<blocks_for(n, 256), 256, 0, st>>>(E, n, sc.keys_a.ptr);
+      size_t tb = 0;
+      FMM_CUDA_TRY(cub::DeviceSegmentedSort::SortKeys(nullptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, n, rows, E.off,
+                                                      E.off + 1, st));
+      sc.cub.grow(tb);
+      FMM_CUDA_TRY(cub::DeviceSegmentedSort::SortKeys(sc.cub.ptr, tb, sc.keys_a.ptr, sc.keys_b.ptr, n, rows, E.off,
+                                                      E.off + 1, st));
+      note_launch();
+      k_export_long<<<rows, 256, 0, st>>>(E, sc.keys_b.ptr);
+      FMM_CUDA_TRY(cudaGetLastError());
+    }
     FMM_CUDA_TRY(cudaMemcpyAsync(q.dst, sc.front_a.ptr, (size_t)n * sizeof(int2), cudaMemcpyDeviceToHost, st));
     FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    FMM_CHECK(!bad, FMM_ERR_STATE, "a list pair is not reachable by the traversal rule (reference-order export)");
   }
 }
 
