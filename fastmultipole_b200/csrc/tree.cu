@@ -501,42 +501,49 @@ struct Geometry {
   double *tc, *sc, *tr, *sr, *tb, *sb;
 };
 
-// shrink_branch! (src/tree.jl:1163-1174); the children were written by other SMs
-__device__ void shrink_branch(const Geometry& G, int k, int c0, int nc) {
-  double tmn[3], tmx[3], smn[3], smx[3];
+// min / max over the first eight lanes of a group, by that group's lanes alone (mask)
+__device__ __forceinline__ double min8(unsigned mask, double v) {
+  for (int o = 4; o > 0; o >>= 1) v = fmin(v, __shfl_xor_sync(mask, v, o));
+  return v;
+}
+__device__ __forceinline__ double max8(unsigned mask, double v) {
+  for (int o = 4; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(mask, v, o));
+  return v;
+}
+
+// shrink_branch! (src/tree.jl:1163-1174), one lane per child (eight lanes; those past the children
+// repeat the first); the children were written by other SMs
+__device__ __forceinline__ void shrink_branch(const Geometry& G, unsigned mask, int lane, int k, int c0, int nc) {
+  const int c = c0 + (lane < nc ? lane : 0);
+  double tc[3], sc[3], tcen[3], scen[3], tb[3], sb[3];
   for (int d = 0; d < 3; ++d) {
-    tmn[d] = tmx[d] = __ldcg(G.tc + 3 * c0 + d);
-    smn[d] = smx[d] = __ldcg(G.sc + 3 * c0 + d);
+    tc[d] = __ldcg(G.tc + 3 * c + d);
+    sc[d] = __ldcg(G.sc + 3 * c + d);
+    tb[d] = __ldcg(G.tb + 3 * c + d);
+    sb[d] = __ldcg(G.sb + 3 * c + d);
   }
-  for (int c = c0; c < c0 + nc; ++c)
-    for (int d = 0; d < 3; ++d) {
-      const double tc = __ldcg(G.tc + 3 * c + d), tb = __ldcg(G.tb + 3 * c + d);
-      const double sc = __ldcg(G.sc + 3 * c + d), sb = __ldcg(G.sb + 3 * c + d);
-      tmn[d] = fmin(tmn[d], tc - tb);
-      tmx[d] = fmax(tmx[d], tc + tb);
-      smn[d] = fmin(smn[d], sc - sb);
-      smx[d] = fmax(smx[d], sc + sb);
-    }
-  double tcen[3], scen[3];
+  const double tr = __ldcg(G.tr + c), sr = __ldcg(G.sr + c);
   for (int d = 0; d < 3; ++d) {
-    tcen[d] = (tmn[d] + tmx[d]) * 0.5;
-    scen[d] = (smn[d] + smx[d]) * 0.5;
+    // the first child's centre takes part too, as in the reference
+    const double tmn = min8(mask, fmin(tc[d], tc[d] - tb[d])), tmx = max8(mask, fmax(tc[d], tc[d] + tb[d]));
+    const double smn = min8(mask, fmin(sc[d], sc[d] - sb[d])), smx = max8(mask, fmax(sc[d], sc[d] + sb[d]));
+    tcen[d] = (tmn + tmx) * 0.5;
+    scen[d] = (smn + smx) * 0.5;
+    tb[d] = tmx - tcen[d];
+    sb[d] = smx - scen[d];
   }
-  double trad = 0.0, srad = 0.0;
-  for (int c = c0; c < c0 + nc; ++c) {
-    double dx = __ldcg(G.tc + 3 * c) - tcen[0], dy = __ldcg(G.tc + 3 * c + 1) - tcen[1],
-           dz = __ldcg(G.tc + 3 * c + 2) - tcen[2];
-    trad = fmax(trad, sqrt(dx * dx + dy * dy + dz * dz) + __ldcg(G.tr + c));
-    dx = __ldcg(G.sc + 3 * c) - scen[0];
-    dy = __ldcg(G.sc + 3 * c + 1) - scen[1];
-    dz = __ldcg(G.sc + 3 * c + 2) - scen[2];
-    srad = fmax(srad, sqrt(dx * dx + dy * dy + dz * dz) + __ldcg(G.sr + c));
-  }
+  double dx = tc[0] - tcen[0], dy = tc[1] - tcen[1], dz = tc[2] - tcen[2];
+  const double trad = max8(mask, fmax(0.0, sqrt(dx * dx + dy * dy + dz * dz) + tr));
+  dx = sc[0] - scen[0];
+  dy = sc[1] - scen[1];
+  dz = sc[2] - scen[2];
+  const double srad = max8(mask, fmax(0.0, sqrt(dx * dx + dy * dy + dz * dz) + sr));
+  if (lane != 0) return;
   for (int d = 0; d < 3; ++d) {
     G.tc[3 * k + d] = tcen[d];
     G.sc[3 * k + d] = scen[d];
-    G.tb[3 * k + d] = tmx[d] - tcen[d];
-    G.sb[3 * k + d] = smx[d] - scen[d];
+    G.tb[3 * k + d] = tb[d];
+    G.sb[3 * k + d] = sb[d];
   }
   G.tr[k] = trad;
   G.sr[k] = srad;
@@ -613,21 +620,29 @@ __global__ void k_leaf_bodies(Branches B, int n_leaves, const int* __restrict__ 
   }
   trad = wmax<G>(trad);
   srad = wmax<G>(srad);
-  if (!valid || lane != 0) return;
-  for (int d = 0; d < 3; ++d) {
-    geo.tc[3 * b + d] = tcen[d];
-    geo.sc[3 * b + d] = scen[d];
-    geo.tb[3 * b + d] = tmx[d] - tcen[d];
-    geo.sb[3 * b + d] = smx[d] - scen[d];
+  if (!valid || lane >= 8) return;
+  if (lane == 0) {
+    for (int d = 0; d < 3; ++d) {
+      geo.tc[3 * b + d] = tcen[d];
+      geo.sc[3 * b + d] = scen[d];
+      geo.tb[3 * b + d] = tmx[d] - tcen[d];
+      geo.sb[3 * b + d] = smx[d] - scen[d];
+    }
+    geo.tr[b] = trad;
+    geo.sr[b] = srad;
   }
-  geo.tr[b] = trad;
-  geo.sr[b] = srad;
+  const unsigned mask = 0xffu << (threadIdx.x & 31 & ~7);  // the group's first eight lanes
   for (int k = B.parent[b]; k >= 0; k = B.parent[k]) {
-    __threadfence();
     const int nc = B.n_children[k];
-    if (atomicAdd(B.done + k, 1) != nc - 1) break;
-    __threadfence();
-    shrink_branch(geo, k, B.child_start[k], nc);
+    int last = 0;
+    if (lane == 0) {
+      __threadfence();
+      last = atomicAdd(B.done + k, 1) == nc - 1;
+      __threadfence();
+    }
+    if (!__shfl_sync(mask, last, 0, 8)) break;
+    shrink_branch(geo, mask, lane, k, B.child_start[k], nc);
+    __syncwarp(mask);
   }
 }
 
