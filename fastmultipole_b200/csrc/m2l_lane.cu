@@ -1353,48 +1353,40 @@ __global__ void __launch_bounds__(32) k_m2l_lane_lh(const int* __restrict__ tgt_
   }
 }
 
-template <int PMAX, class V>
-void run_m2l_lane_lh_v(DevTree& t, const DevTree& s, const DevLists& L, int P, int* p_used, int* stats,
+template <int PMAX>
+void run_m2l_lane_lh(DevTree& t, const DevTree& s, const DevLists& L, int P, int* p_used, int* stats,
                        cudaStream_t st) {
-  constexpr size_t sm = lane_lh_smem_bytes<PMAX, V>();
+  constexpr size_t sm = lane_lh_smem_bytes<PMAX, float>();
   if (sm > 48 * 1024)
-    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane_lh<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane_lh<PMAX, float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   note_launch();
-  k_m2l_lane_lh<PMAX, V><<<(int)L.n_m2l_targets, 32, sm, st>>>(
+  k_m2l_lane_lh<PMAX, float><<<(int)L.n_m2l_targets, 32, sm, st>>>(
       L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, P,
       p_used, stats, reinterpret_cast<unsigned long long*>(stats + 2));
   FMM_CUDA_TRY(cudaGetLastError());
 }
-template <int PMAX>
-void run_m2l_lane_lh(DevTree& t, const DevTree& s, const DevLists& L, int P, int* p_used, int* stats, int precision,
-                     cudaStream_t st) {
-  if (precision == FMM_PRECISION_MIXED)
-    run_m2l_lane_lh_v<PMAX, float>(t, s, L, P, p_used, stats, st);
-  else
-    run_m2l_lane_lh_v<PMAX, double>(t, s, L, P, p_used, stats, st);
-}
-
 }  // namespace
 
 bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
                      int* p_used, int* stats, int precision, cudaStream_t st) {
   if (p < 1 || p > kLaneMaxP) return false;
   if (lh) {
-    // vortex particles: the plain M2L from order 4 (orders <= 3 take the thread-per-pair
-    // kernel, the error-controlled ones the general engine)
-    if (em != FMM_ERROR_NONE || p < 4) return false;
+    // vortex particles: the plain M2L of the mixed path from order 4 (orders <= 3 take the
+    // thread-per-pair kernel; the error-controlled ones and FP64 translate_deg.cu, which ran the
+    // 300k ring's FP64 M2L, order 12, in 1.5 ms where this kernel took 2.1)
+    if (em != FMM_ERROR_NONE || p < 4 || precision != FMM_PRECISION_MIXED) return false;
     if (L.n_m2l_targets == 0) return true;
     ensure_lane_tables(st);
     switch (p) {
-      case 4: run_m2l_lane_lh<4>(t, s, L, p, p_used, stats, precision, st); break;
-      case 5: run_m2l_lane_lh<5>(t, s, L, p, p_used, stats, precision, st); break;
-      case 6: run_m2l_lane_lh<6>(t, s, L, p, p_used, stats, precision, st); break;
-      case 7: run_m2l_lane_lh<7>(t, s, L, p, p_used, stats, precision, st); break;
-      case 8: run_m2l_lane_lh<8>(t, s, L, p, p_used, stats, precision, st); break;
-      case 9: run_m2l_lane_lh<9>(t, s, L, p, p_used, stats, precision, st); break;
-      case 10: run_m2l_lane_lh<10>(t, s, L, p, p_used, stats, precision, st); break;
-      case 11: run_m2l_lane_lh<11>(t, s, L, p, p_used, stats, precision, st); break;
-      default: run_m2l_lane_lh<12>(t, s, L, p, p_used, stats, precision, st); break;
+      case 4: run_m2l_lane_lh<4>(t, s, L, p, p_used, stats, st); break;
+      case 5: run_m2l_lane_lh<5>(t, s, L, p, p_used, stats, st); break;
+      case 6: run_m2l_lane_lh<6>(t, s, L, p, p_used, stats, st); break;
+      case 7: run_m2l_lane_lh<7>(t, s, L, p, p_used, stats, st); break;
+      case 8: run_m2l_lane_lh<8>(t, s, L, p, p_used, stats, st); break;
+      case 9: run_m2l_lane_lh<9>(t, s, L, p, p_used, stats, st); break;
+      case 10: run_m2l_lane_lh<10>(t, s, L, p, p_used, stats, st); break;
+      case 11: run_m2l_lane_lh<11>(t, s, L, p, p_used, stats, st); break;
+      default: run_m2l_lane_lh<12>(t, s, L, p, p_used, stats, st); break;
     }
     return true;
   }
