@@ -412,6 +412,27 @@ __device__ __noinline__ void self_batch_f64_vortex(const double2* __restrict__ B
   }
 }
 
+// Targets of the next tile of a row with rem targets left.  SUB (two targets per lane, expensive
+// pairs): a remainder that would leave a quarter or more of its slots empty gives a full power of two
+// first.  The sources are gathered once more for the rest, which the vortex kernels' 32 or more
+// operations per pair outweigh.
+template <bool SUB>
+__host__ __device__ __forceinline__ int next_tile(int rem) {
+  constexpr int most = 32 * kTPT;
+  if (rem >= most) return most;
+  if (SUB) {
+    if (rem > most / 2 && rem <= most * 3 / 4) return most / 2;
+    if (rem > most / 4 && rem <= most * 3 / 8) return most / 4;
+  }
+  return rem;
+}
+// (300k ring FP64 25.1 -> 23.8 ms, 2e6 ring mixed 210.4 -> 205.8 ms; mixed point sources only in whole
+// rows, 1e6 bodies 34.7 -> 34.5 ms: as items of the gradient of 2e5 sources 2.99 -> 3.22 ms)
+template <class R, int KIND, bool ITEMS>
+__host__ __device__ constexpr bool sub_tiles() {
+  return KIND == FMM_POINT_VORTEX || (sizeof(R) == 4 && !ITEMS);
+}
+
 // Targets per lane of a tile of nt targets on the FP64 path: three where 3 x a power of two lanes
 // leave fewer slots empty than 2 x (nt in (2^k, 3/2 2^k]).  Leaves are split by eight, so their sizes
 // spread over a factor of eight and the slots matter: slots per pair 1.24 -> 1.11 (1e6 clustered
@@ -456,7 +477,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
                                                      const double4* __restrict__ sstr, double* __restrict__ acc13,
                                                      const int4* __restrict__ items, const int* __restrict__ n_items,
                                                      double* __restrict__ item_sums, int exact_self) {
-  // items (ITEMS, CTA path only), two int4 each: row, tile and source leaves [z, w); and the place of
+  // items (ITEMS, CTA path only), two int4 each: row, first target of the tile, source leaves [z, w); and the place of
   // the item's sums (unscaled) in item_sums, or -1 to add them to the targets
   constexpr int W = kWarps;
   static_assert(!(RW && ITEMS), "a warp per row takes whole rows");
@@ -519,8 +540,9 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
   const double ox = MIXED ? t_center[3 * t] : 0.0;
   const double oy = MIXED ? t_center[3 * t + 1] : 0.0;
   const double oz = MIXED ? t_center[3 * t + 2] : 0.0;
-  for (int tile = ITEMS ? it.y * 32 * kTPT : 0; tile < tc; tile += 32 * kTPT) {
-    const int nt = min(tc - tile, 32 * kTPT);
+  constexpr bool SUB = sub_tiles<R, KIND, ITEMS || RW>() && KT == kTPT;
+  for (int tile = ITEMS ? it.y : 0, nt; tile < tc; tile += nt) {
+    nt = next_tile<SUB>(tc - tile);
     const int tpt = KT == 3 ? targets_per_lane(nt) : kTPT;
     int TS = 1;
     while (TS * tpt < nt) TS <<= 1;
@@ -1092,6 +1114,7 @@ __device__ __forceinline__ int tile_slots(int nt, bool three) {
 // work / goal slot pairs.  Items and their sums' places come from scans over the rows, so that the
 // cut, and with it the order of every sum, depends on the tree and the lists alone.
 constexpr int kPlanThreads = 1024;
+template <bool SUB>
 __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict__ tgt_list,
                                                            const int* __restrict__ off, int rows,
                                                            const int* __restrict__ t_count,
@@ -1105,7 +1128,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
   for (int r = threadIdx.x; r < rows; r += kPlanThreads) {
     const int tc = t_count[tgt_list[r]];
     int slots = 0;
-    for (int t = 0; t < tc; t += 32 * kTPT) slots += tile_slots(min(tc - t, 32 * kTPT), three != 0);
+    for (int t = 0, nt; t < tc; t += nt) {
+      nt = next_tile<SUB>(tc - t);
+      slots += tile_slots(nt, three != 0);
+    }
     work += (unsigned long long)slots * (unsigned)n_src[r];
   }
 #pragma unroll
@@ -1130,8 +1156,9 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       return (int)max(1ull, min(c, (unsigned long long)min(nl, ns / kItemSources)));
     };
     int2 v = make_int2(0, 0);
-    for (int t = 0; t < tc; t += 32 * kTPT) {
-      const int nt = min(tc - t, 32 * kTPT), c = cut(nt);
+    for (int t = 0, nt; t < tc; t += nt) {
+      nt = next_tile<SUB>(tc - t);
+      const int c = cut(nt);
       v.x += c;
       if (c > 1) v.y += c * nt * na;
     }
@@ -1150,14 +1177,15 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       run.y += sh[q].y;
     }
     __syncthreads();
-    for (int t = 0; t < tc; t += 32 * kTPT) {
-      const int nt = min(tc - t, 32 * kTPT), c = cut(nt);
+    for (int t = 0, nt; t < tc; t += nt) {
+      nt = next_tile<SUB>(tc - t);
+      const int c = cut(nt);
       // (the bound on the items leaves room for every row's sums)
       const bool split = c > 1 && ex.y + c * nt * na <= max_sums;
       for (int j = 0; j < c; ++j) {
         const int lo = split ? a + (int)((long long)nl * j / c) : a;
         const int hi = split ? a + (int)((long long)nl * (j + 1) / c) : (j == 0 ? a + nl : a);
-        items[2 * (ex.x + j)] = make_int4(r, t / (32 * kTPT), lo, hi);
+        items[2 * (ex.x + j)] = make_int4(r, t, lo, hi);
         items[2 * (ex.x + j) + 1] = make_int4(split ? ex.y + j * nt * na : -1, split && j == 0 ? c : 0, nt, 0);
       }
       ex.x += c;
@@ -1175,7 +1203,7 @@ __global__ void k_p2p_sum(const int4* __restrict__ items, const int* __restrict_
   if ((int)blockIdx.x >= *n_items) return;
   const int4 a = items[2 * blockIdx.x], b = items[2 * blockIdx.x + 1];
   if (b.y == 0) return;
-  const int first = t_start[tgt_list[a.x]] + a.y * 32 * kTPT;
+  const int first = t_start[tgt_list[a.x]] + a.y;
   for (int e = threadIdx.x; e < b.z * NA; e += blockDim.x) {
     const int i = e / NA, ch = e - i * NA;
     if (KIND == FMM_POINT_SOURCE && ch == 0 && !PS) continue;
@@ -1222,9 +1250,9 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     FMM_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_p2p<R, KIND, PS, GS, HS, false, true>,
                                                                kWarps * 32, smem));
     const int goal = kItemWaves * std::max(1, per_sm) * n_sm;
-    // a tile per 64 targets begun, a share more per 1 / goal of the work; at most twice the goal of
-    // them in tiles that are cut
-    const int64_t most = rows + tt.n_bodies / (32 * kTPT) + goal + 1;
+    // a tile per 64 targets begun (up to three with sub-tiles), a share more per 1 / goal of the work;
+    // at most twice the goal of them in tiles that are cut
+    const int64_t most = 3 * (int64_t)rows + tt.n_bodies / (32 * kTPT) + goal + 1;
     const int64_t sums = (int64_t)2 * goal * 32 * kTPT * NA;
     L.p2p_items.grow(2 * (size_t)most);
     L.p2p_meta.grow((size_t)rows + 1);
@@ -1233,7 +1261,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     k_p2p_row_sources<<<(int)((rows * 32ll + 255) / 256), 256, 0, st>>>(L.dir_off.ptr, rows, L.dir_s.ptr,
                                                                         stt.body_count.ptr, L.p2p_meta.ptr + 1);
     note_launch();
-    k_p2p_plan<<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
+    k_p2p_plan<sub_tiles<R, KIND, true>() && max_targets_per_lane<R, KIND, HS>() == kTPT><<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
                                            goal, NA, (int)sums, max_targets_per_lane<R, KIND, HS>() == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
     note_launch();
     k_p2p<R, KIND, PS, GS, HS, false, true><<<(int)most, kWarps * 32, smem, st>>>(
