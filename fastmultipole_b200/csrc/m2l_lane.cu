@@ -826,31 +826,38 @@ __global__ void __launch_bounds__(32 * W) k_m2l_lane(const int* __restrict__ tgt
 constexpr int kWideM2LWarps = 4;
 constexpr int kWideM2LRowsPerSM = 4;
 
+int sm_count() {
+  int dev = 0, n_sm = 0;
+  FMM_CUDA_TRY(cudaGetDevice(&dev));
+  FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
+  return n_sm;
+}
+
 template <int PMAX, class V>
 void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double eps, int be, int* p_used, int* stats,
                 cudaStream_t st) {
   const size_t sm = lane_smem_bytes<PMAX, V>();
   note_launch();
-  int dev = 0, n_sm = 0;
-  FMM_CUDA_TRY(cudaGetDevice(&dev));
-  FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
-  if (L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * n_sm) {
-    // few target rows (small problems, probe trees): kWideM2LWarps warps share each row
-    constexpr int WW = kWideM2LWarps;
-    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V, WW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)(WW * sm)));
-    k_m2l_lane<PMAX, V, WW><<<(int)L.n_m2l_targets, 32 * WW, WW * sm, st>>>(
-        L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-        t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
-        reinterpret_cast<unsigned long long*>(stats + 2));
-  } else {
-    if (sm > 48 * 1024)
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
-    k_m2l_lane<PMAX, V><<<(int)L.n_m2l_targets, 32, sm, st>>>(
-        L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-        t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
-        reinterpret_cast<unsigned long long*>(stats + 2));
+  if constexpr (sizeof(V) == 4) {
+    if (L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) {
+      // few target rows (small problems, probe trees): kWideM2LWarps warps share each row
+      constexpr int WW = kWideM2LWarps;
+      FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V, WW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        (int)(WW * sm)));
+      k_m2l_lane<PMAX, V, WW><<<(int)L.n_m2l_targets, 32 * WW, WW * sm, st>>>(
+          L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
+          t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
+          reinterpret_cast<unsigned long long*>(stats + 2));
+      FMM_CUDA_TRY(cudaGetLastError());
+      return;
+    }
   }
+  if (sm > 48 * 1024)
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+  k_m2l_lane<PMAX, V><<<(int)L.n_m2l_targets, 32, sm, st>>>(
+      L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
+      t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
+      reinterpret_cast<unsigned long long*>(stats + 2));
   FMM_CUDA_TRY(cudaGetLastError());
 }
 
@@ -1401,6 +1408,10 @@ bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, boo
       run_m2l_small<3>(t, s, L, p_used, stats, precision, st);
     return true;
   }
+  // FP64 with few target rows: the degrees of a pair spread over warps shorten the chain (1e4 bodies,
+  // order 6, 59 us here with four warps per row; the 24,000 rows of 1e6 bodies, order 10, take 10.5 ms
+  // here and 11.7 there)
+  if (precision != FMM_PRECISION_MIXED && L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) return false;
   switch (p) {
     case 1: run_lane<1>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
     case 2: run_lane<2>(t, s, L, em, eps, be, p_used, stats, precision, st); break;

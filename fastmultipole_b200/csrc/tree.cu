@@ -164,15 +164,21 @@ __device__ __forceinline__ int key_digit(unsigned long long k, int l) {
   return (int)((k >> (3 * (kMaxDepth - 1 - l))) & 7ull);
 }
 
-// first position in [lo, hi) whose level-l digit is >= o
+// first position in [lo, hi) whose level-l digit is >= o (three probes a round: the rounds' loads,
+// not the comparisons, take the time)
 __device__ int lower_bound_digit(const unsigned long long* keys, int lo, int hi, int l, int o) {
-  while (lo < hi) {
-    int mid = lo + ((hi - lo) >> 1);
-    if (key_digit(keys[mid], l) < o)
-      lo = mid + 1;
-    else
-      hi = mid;
+  while (hi - lo > 3) {
+    const int q = (hi - lo) >> 2, a = lo + q, b = a + q, c = b + q;
+    const bool pa = key_digit(keys[a], l) < o, pb = key_digit(keys[b], l) < o, pc = key_digit(keys[c], l) < o;
+    if (pb) {
+      lo = (pc ? c : b) + 1;
+      if (!pc) hi = c;
+    } else {
+      hi = pa ? b : a;
+      if (pa) lo = a + 1;
+    }
   }
+  while (lo < hi && key_digit(keys[lo], l) < o) ++lo;
   return lo;
 }
 
@@ -709,8 +715,8 @@ void build_tree(DevTree& t, Scratch& sc, cudaStream_t st, int64_t leaf_size, int
   note_launch();
   k_keys<<<blocks_for(n), kThreads, 0, st>>>(t.pos.ptr, n, root, sc.keys_a.ptr, sc.vals_a.ptr);
   FMM_CUDA_TRY(cudaGetLastError());
-  // the digits of kShallow levels first (five radix passes instead of eight); all of them when a
-  // branch below still has to split
+  // the digits of as many levels first as a density 8^6 times the mean would split to (four or five
+  // radix passes instead of eight); all of them when a branch below still has to split
   auto sort_keys = [&](int depth) {
     const int lo = 3 * (kMaxDepth - depth);
     size_t tmp_bytes = 0;
@@ -720,8 +726,9 @@ void build_tree(DevTree& t, Scratch& sc, cudaStream_t st, int64_t leaf_size, int
     FMM_CUDA_TRY(cub::DeviceRadixSort::SortPairs(sc.cub.ptr, tmp_bytes, sc.keys_a.ptr, sc.keys_b.ptr, sc.vals_a.ptr,
                                                  sc.vals_b.ptr, (int)n, lo, 3 * kMaxDepth, st));
   };
-  constexpr int kShallow = 13;
-  int depth = kShallow;
+  int depth = 6;
+  for (int64_t m = n; m > leaf_size && depth < kMaxDepth; m >>= 3) ++depth;
+  depth = std::min(kMaxDepth, (3 * depth + 7) / 8 * 8 / 3);  // to the end of a radix pass
   sort_keys(depth);
   const int* perm = sc.vals_b.ptr;
 
