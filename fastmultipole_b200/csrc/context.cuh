@@ -141,9 +141,10 @@ void launch_op_l2p(int64_t n, const double* dx, const double* local, int p, bool
                    double* out13, cudaStream_t st);
 
 // ---- translate_deg.cu ----
-// M2L of any order up to kMaxP, plain or error-controlled, FP64, degrees spread over a CTA's warps
+// M2L of any order up to kMaxP, plain or error-controlled, degrees spread over a CTA's warps; FP64, or
+// FP32 on the mixed path for a fixed order up to 12
 void launch_m2l_deg(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int error_method, double eps,
-                    int be, int* stats, cudaStream_t st);
+                    int be, int* stats, int precision, cudaStream_t st);
 void launch_m2m(DevTree& s, int p, bool lh, cudaStream_t st);
 void launch_l2l(DevTree& t, int p, bool lh, cudaStream_t st);
 

@@ -949,7 +949,7 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
   }
   if (launch_m2l_lane(t, s, L, p, lh, em, eps, be, p_used, stats, precision, st)) return;
   // higher orders, and vortex particles with error control
-  launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, st);
+  launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, precision, st);
 }
 
 void launch_l2p(DevTree& t, int p, bool lh, bool ps, bool gs, bool hs, double* acc13, cudaStream_t st) {

@@ -11,7 +11,9 @@
 // dependent stages set the time.  Whole solves, before -> after: 150k clustered point sources,
 // order 16, tolerance 1e-7: 98.4 -> 10.2 ms; 48k vortex particles, order 16, tolerance 1e-6: 18.0 ->
 // 4.45 ms; 30k vortex ring, order 8: 2.17 -> 1.49 ms (M2M and L2L alone).  Bound now by the FP64 pipe
-// and, at orders above 12, by the shared memory of the rotated degrees (two CTAs per SM).
+// and, at orders above 12, by the shared memory of the rotated degrees (two CTAs per SM).  In FP32
+// (fixed orders of the mixed path) against a kernel with a lane per pair, seven warps per SM: 300k
+// clustered bodies, order 10, M2L 2.04 -> 1.02 ms; 200k vortex ring, order 12, 1.42 -> 0.67 ms.
 //
 // Rotations about y are factorised as in m2l_lane.cu, with the magnitudes applied outside
 // the two matrix products, so that one constant table of the Wigner matrix at pi/2 serves both
@@ -37,6 +39,15 @@ __constant__ double c_Az[kNh], c_Bz[kNh], c_Ae[kNh], c_Be[kNh];
 __constant__ double c_Mt[kNh], c_Lt[kNh];
 __constant__ double c_fact[2 * kMaxP + 2];
 __constant__ double c_ifact[kMaxP + 1] = {FMM_INV_FACTORIALS};
+// FP32 tables up to order 12 for the mixed path: B H over a, zeta and eta, the magnitude multiplied
+// in before the one rounding; column (n, nu) at float4 kColQ hi(n, nu), zero past its degree, read
+// four entries per constant load.  The same column gives the second product, whose outputs take
+// A / B in FP64: factors rounded to FP32 by themselves would be the same for every pair and add up
+// (ring far field 6.6e-9 -> 1.3e-8; with a second table of A H 6.6e-9 too, at 1.2 times the time)
+constexpr int kMaxF = 12, kColQ = 4, kNhF = hi(kMaxF + 1, 0);
+__constant__ float4 c_BzF[kNhF * kColQ], c_BeF[kNhF * kColQ];
+__constant__ double c_ABz[kNhF], c_ABe[kNhF];
+__constant__ float c_factF[2 * kMaxF + 2];
 
 std::mutex g_mu;
 bool g_done[64];
@@ -73,6 +84,27 @@ void ensure_tables(cudaStream_t st) {
   put(c_fact, fact);
   put(c_Mt, std::vector<double>(h.Mt.begin(), h.Mt.begin() + kNh));
   put(c_Lt, std::vector<double>(h.Lt.begin(), h.Lt.begin() + kNh));
+  auto put_f = [&](const void* sym, const std::vector<float>& v) {
+    FMM_CUDA_TRY(cudaMemcpyToSymbolAsync(sym, v.data(), v.size() * sizeof(float), 0, cudaMemcpyHostToDevice, st));
+  };
+  std::vector<float> bzf((size_t)kNhF * kColQ * 4, 0.f), bef(bzf);
+  std::vector<double> abz(kNhF), abe(kNhF);
+  for (int n = 0; n <= kMaxF; ++n)
+    for (int a = 0; a <= n; ++a) {
+      abz[hi(n, a)] = az[hi(n, a)] / bz[hi(n, a)];
+      abe[hi(n, a)] = ae[hi(n, a)] / be[hi(n, a)];
+      for (int nu = 0; nu <= n; ++nu) {
+        const double h0 = H[lenT(n - 1) + nu * (n + 1) + a];
+        const size_t d = (size_t)hi(n, nu) * kColQ * 4 + a;
+        bzf[d] = (float)(bz[hi(n, a)] * h0);
+        bef[d] = (float)(be[hi(n, a)] * h0);
+      }
+    }
+  put_f(c_BzF, bzf);
+  put_f(c_BeF, bef);
+  put(c_ABz, abz);
+  put(c_ABe, abe);
+  put_f(c_factF, std::vector<float>(fact.begin(), fact.begin() + 2 * kMaxF + 2));
   FMM_CUDA_TRY(cudaStreamSynchronize(st));
   if (dev < 64) g_done[dev] = true;
 }
@@ -99,104 +131,125 @@ __device__ __forceinline__ Geo geo_of(double x, double y, double z) {
 }
 
 // rotate_z of degree n of one set of an interleaved expansion, times sc, into padded registers
-template <int PMAX>
+template <int PMAX, class V>
 __device__ __forceinline__ void rotz_in(int n, const double2* __restrict__ e, int set, const Geo& g, double sc,
-                                        double (&Xr)[PMAX + 1], double (&Xi)[PMAX + 1]) {
+                                        V (&Xr)[PMAX + 1], V (&Xi)[PMAX + 1]) {
   double er = sc, ei = 0.0;
 #pragma unroll
   for (int a = 0; a <= PMAX; ++a) {
-    Xr[a] = Xi[a] = 0.0;
+    Xr[a] = Xi[a] = V(0);
     if (a > n) continue;
     const double2 u = e[2 * (hi(n, 0) + a) + set];
-    Xr[a] = u.x * er - u.y * ei;
-    Xi[a] = u.x * ei + u.y * er;
+    Xr[a] = (V)(u.x * er - u.y * ei);
+    Xi[a] = (V)(u.x * ei + u.y * er);
     const double t = er;
     er = er * g.cph - ei * g.sph;
     ei = t * g.sph + ei * g.cph;
+  }
+}
+
+// one FP32 column in registers
+template <int PMAX>
+__device__ __forceinline__ void column(const float4* __restrict__ q, float (&h)[PMAX + 1]) {
+#pragma unroll
+  for (int i = 0; i <= PMAX / 4; ++i) {
+    const float4 v = q[i];
+    const float w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (4 * i + j <= PMAX) h[(4 * i + j) % (PMAX + 1)] = w[j];
   }
 }
 
 // rotate_y of degree n in place (entries past n: zero on entry, undefined on return).  LOCAL: eta
-// magnitudes and e^{-+i nu beta}.  Column nu of H serves both products: E, O, Z of the input, and
-// P_nu +- Q_nu into every output (the derivation is in m2l_lane.cu).  Sums run to PMAX from one
-// column base, so the table is read at fixed offsets and no term is predicated.
-template <int PMAX, bool LOCAL>
-__device__ __forceinline__ void rot_y(int n, const Geo& g, double (&Xr)[PMAX + 1], double (&Xi)[PMAX + 1]) {
-  double Yr[PMAX + 1], Yi[PMAX + 1];
+// magnitudes and e^{-+i nu beta}.  Column nu gives E, O, Z of the input, and P_nu +- Q_nu into every
+// output (the derivation is in m2l_lane.cu); FP64 applies the magnitudes outside the nu loop, so that
+// one table serves both products and both sets; FP32 see its tables.  Sums run to PMAX from one column base, so the
+// tables are read at fixed offsets and no term is predicated.
+template <int PMAX, bool LOCAL, class V>
+__device__ __forceinline__ void rot_y(int n, V cth, V sth, V (&Xr)[PMAX + 1], V (&Xi)[PMAX + 1]) {
+  constexpr bool F32 = sizeof(V) == 4;
+  V Yr[PMAX + 1], Yi[PMAX + 1];
   const int b0 = hi(n, 0);
 #pragma unroll
   for (int a = 0; a <= PMAX; ++a) {
-    Yr[a] = Yi[a] = 0.0;
-    if (a > n) continue;
-    const double b = LOCAL ? c_Be[b0 + a] : c_Bz[b0 + a];
+    Yr[a] = Yi[a] = V(0);
+    if (F32 || a > n) continue;
+    const V b = (V)(LOCAL ? c_Be[b0 + a] : c_Bz[b0 + a]);
     Xr[a] *= b;
     Xi[a] *= b;
   }
-  double c = 1.0, s = 0.0;  // cos, sin (nu beta) by the reference's recurrence
+  V c = V(1), s = V(0);  // cos, sin (nu beta) by the reference's recurrence
 #pragma unroll 1
   for (int nu = 0; nu <= n; ++nu) {
     if (nu > 0) {
-      const double cn = g.cth * c - g.sth * s;
-      const double sn = g.sth * c + g.cth * s;
+      const V cn = cth * c - sth * s;
+      const V sn = sth * c + cth * s;
       c = cn;
       s = sn;
     }
+    V h[F32 ? PMAX + 1 : 1];
+    if constexpr (F32) column<PMAX>((LOCAL ? c_BeF : c_BzF) + (b0 + nu) * kColQ, h);
     const double* __restrict__ col = c_H + (lenT(n - 1) + nu * (n + 1));
-    double Er = 0, Ei = 0, Or = 0, Oi = 0;
+    auto H = [&](int a) -> V {
+      if constexpr (F32) return h[a];
+      else return col[a];
+    };
+    V Er = 0, Ei = 0, Or = 0, Oi = 0;
 #pragma unroll
     for (int a = 1; a <= PMAX; ++a) {
-      const double h = col[a];
       if (a & 1) {
-        Or += h * Xr[a];
-        Oi += h * Xi[a];
+        Or += H(a) * Xr[a];
+        Oi += H(a) * Xi[a];
       } else {
-        Er += h * Xr[a];
-        Ei += h * Xi[a];
+        Er += H(a) * Xr[a];
+        Ei += H(a) * Xi[a];
       }
     }
-    const double Zr = col[0] * Xr[0], Zi = col[0] * Xi[0];
-    const double w = nu == 0 ? 0.5 : 1.0;  // weight w_nu / 2
-    const double sg = ((n + nu) & 1) ? -w : w;
-    const double S1r = Er - Or, S1i = Ei - Oi;
-    const double S3r = Er + Or, S3i = Ei + Oi;
-    const double S2r = Zr + S3r, S2i = -(Zi + S3i);
-    const double S4r = Zr + S1r, S4i = -(Zi + S1i);
-    const double A1r = w * S1r + sg * S2r, A1i = w * S1i + sg * S2i;
-    const double A3r = w * S3r + sg * S4r, A3i = w * S3i + sg * S4i;
-    const double ss = LOCAL ? -s : s;
-    const double Pr = c * A1r - ss * A1i, Pi = c * A1i + ss * A1r;
-    const double Qr = c * A3r + ss * A3i, Qi = c * A3i - ss * A3r;
-    const double Rpr = Pr + Qr, Rpi = Pi + Qi, Rmr = Pr - Qr, Rmi = Pi - Qi;
+    const V Zr = H(0) * Xr[0], Zi = H(0) * Xi[0];
+    const V w = nu == 0 ? V(0.5) : V(1);  // weight w_nu / 2
+    const V sg = ((n + nu) & 1) ? -w : w;
+    const V S1r = Er - Or, S1i = Ei - Oi;
+    const V S3r = Er + Or, S3i = Ei + Oi;
+    const V S2r = Zr + S3r, S2i = -(Zi + S3i);
+    const V S4r = Zr + S1r, S4i = -(Zi + S1i);
+    const V A1r = w * S1r + sg * S2r, A1i = w * S1i + sg * S2i;
+    const V A3r = w * S3r + sg * S4r, A3i = w * S3i + sg * S4i;
+    const V ss = LOCAL ? -s : s;
+    const V Pr = c * A1r - ss * A1i, Pi = c * A1i + ss * A1r;
+    const V Qr = c * A3r + ss * A3i, Qi = c * A3i - ss * A3r;
+    const V Rpr = Pr + Qr, Rpi = Pi + Qi, Rmr = Pr - Qr, Rmi = Pi - Qi;
 #pragma unroll
     for (int m = 0; m <= PMAX; ++m) {
-      const double h = col[m];
-      Yr[m] += h * ((m & 1) ? Rmr : Rpr);
-      Yi[m] += h * ((m & 1) ? Rmi : Rpi);
+      Yr[m] += H(m) * ((m & 1) ? Rmr : Rpr);
+      Yi[m] += H(m) * ((m & 1) ? Rmi : Rpi);
     }
   }
 #pragma unroll
   for (int m = 0; m <= PMAX; ++m) {
     if (m > n) break;
-    const double a = LOCAL ? c_Ae[b0 + m] : c_Az[b0 + m];
-    Xr[m] = a * Yr[m];
-    Xi[m] = a * Yi[m];
+    double a;
+    if constexpr (F32) a = LOCAL ? c_ABe[b0 + m] : c_ABz[b0 + m];
+    else a = LOCAL ? c_Ae[b0 + m] : c_Az[b0 + m];
+    Xr[m] = (V)(a * Yr[m]);
+    Xi[m] = (V)(a * Yi[m]);
   }
 }
 
 // back_rotate_z of degree n in place
-template <int PMAX>
-__device__ __forceinline__ void rotz_back(int n, const Geo& g, double (&Yr)[PMAX + 1], double (&Yi)[PMAX + 1]) {
-  double er = 1.0, ei = 0.0;
+template <int PMAX, class V>
+__device__ __forceinline__ void rotz_back(int n, V cph, V sph, V (&Yr)[PMAX + 1], V (&Yi)[PMAX + 1]) {
+  V er = V(1), ei = V(0);
 #pragma unroll
   for (int m = 0; m <= PMAX; ++m) {
     if (m > n) break;
-    const double vr = Yr[m] * er + Yi[m] * ei;
-    const double vi = Yi[m] * er - Yr[m] * ei;
+    const V vr = Yr[m] * er + Yi[m] * ei;
+    const V vi = Yi[m] * er - Yr[m] * ei;
     Yr[m] = vr;
     Yi[m] = vi;
-    const double t = er;
-    er = er * g.cph - ei * g.sph;
-    ei = t * g.sph + ei * g.cph;
+    const V t = er;
+    er = er * cph - ei * sph;
+    ei = t * sph + ei * cph;
   }
 }
 
@@ -229,26 +282,29 @@ __device__ __forceinline__ unsigned long long pair_flops(int p) {
 constexpr int kW = 4;
 
 template <int PMAX, bool LH>
-__host__ __device__ constexpr int stage_doubles() {  // one warp's staging of one plane of a degree
-  return LH ? 2 * (PMAX + 1) * 17 : (PMAX + 1) * 33;
+__host__ __device__ constexpr int stage_entries() {  // one warp's staging of one plane of a degree (even)
+  return LH ? 2 * (PMAX + 1) * 17 : ((PMAX + 1) * 33 + 1) & ~1;
 }
-template <int PMAX, bool LH>
-size_t m2l_deg_smem(int p) {
+// V: FP32 on the mixed path (fixed order up to 12, no error control), else FP64
+template <int PMAX, bool LH, class V>
+size_t m2l_deg_smem(int p, bool errc) {
   const size_t NH = nh(p);
-  return ((LH ? 4 : 2) * NH + (p + 1) * 32 + kW * 32 + kW * stage_doubles<PMAX, LH>() + 2 * NH * 32) * sizeof(double) +
-         kW * 32 * sizeof(int);
+  return ((LH ? 4 : 2) * NH + (errc ? (p + 1) * 32 : 0) + kW * 32) * sizeof(double) +
+         (kW * stage_entries<PMAX, LH>() + 2 * NH * 32) * sizeof(V) + (errc ? kW * 32 * sizeof(int) : 0);
 }
 
 // sum_{np <= top} (n + np)! M'(np, m) for m <= mmax, source degrees outer
-template <int PMAX>
-__device__ __forceinline__ void coax(int n, int mmax, int top, const double* Ms, int lane, double (&Xr)[PMAX + 1],
-                                     double (&Xi)[PMAX + 1]) {
+template <int PMAX, class V>
+__device__ __forceinline__ void coax(int n, int mmax, int top, const V* Ms, int lane, V (&Xr)[PMAX + 1],
+                                     V (&Xi)[PMAX + 1]) {
 #pragma unroll
-  for (int m = 0; m <= PMAX; ++m) Xr[m] = Xi[m] = 0.0;
+  for (int m = 0; m <= PMAX; ++m) Xr[m] = Xi[m] = V(0);
 #pragma unroll 1
   for (int np = 0; np <= top; ++np) {
-    const double c = c_fact[n + np];
-    const double* s = Ms + 2 * hi(np, 0) * 32 + lane;
+    V c;
+    if constexpr (sizeof(V) == 4) c = c_factF[n + np];
+    else c = c_fact[n + np];
+    const V* s = Ms + 2 * hi(np, 0) * 32 + lane;
 #pragma unroll
     for (int m = 0; m <= PMAX; ++m) {
       if (m > mmax || m > np) break;
@@ -258,8 +314,8 @@ __device__ __forceinline__ void coax(int n, int mmax, int top, const double* Ms,
   }
 }
 
-template <int PMAX, bool LH>
-__global__ void __launch_bounds__(32 * kW, 2)
+template <int PMAX, bool LH, class V>
+__global__ void __launch_bounds__(32 * kW, sizeof(V) == 4 ? 4 : 2)
     k_m2l_deg(const int* __restrict__ tgt_list, const int* __restrict__ off, const int* __restrict__ src_of,
               double* __restrict__ local, const double* __restrict__ multipole, const double* __restrict__ tcen,
               const double* __restrict__ tbox, const double* __restrict__ trad, const double* __restrict__ maxinf,
@@ -273,14 +329,16 @@ __global__ void __launch_bounds__(32 * kW, 2)
   const int set = LH ? lane >> 4 : 0, slot = LH ? lane & 15 : lane;
   double* acc = smem_d;                                 // [4 i + 2 set + c] (LH) or [2 i + c]
   double* pw = acc + 2 * SETS * NH;                     // degree powers of the lane's set [p+1][32]
-  double* tsc = pw + (p + 1) * 32 + w * 32;             // this warp's t^-(n+1) (phi), t^-(n+2) (chi)
-  double* stage = pw + (p + 1) * 32 + kW * 32 + w * stage_doubles<PMAX, LH>();
-  double* Ms = pw + (p + 1) * 32 + kW * 32 + kW * stage_doubles<PMAX, LH>();  // [2 i + c][32]
+  const bool errc = sizeof(V) == 8 && em != FMM_ERROR_NONE;
+  double* tscs = pw + (errc ? (p + 1) * 32 : 0);
+  double* tsc = tscs + w * 32;                          // this warp's t^-(n+1) (phi), t^-(n+2) (chi)
+  V* stages = reinterpret_cast<V*>(tscs + kW * 32);
+  V* stage = stages + w * stage_entries<PMAX, LH>();
+  V* Ms = stages + kW * stage_entries<PMAX, LH>();      // [2 i + c][32]
   int* passed = reinterpret_cast<int*>(Ms + 2 * NH * 32);                     // [kW][32]
   const int b = blockIdx.x;
   const int t = tgt_list[b];
   const double tc0 = tcen[3 * t], tc1 = tcen[3 * t + 1], tc2 = tcen[3 * t + 2];
-  const bool errc = em != FMM_ERROR_NONE;
   const bool relative = (em == FMM_POWER_RELATIVE_GRADIENT || em == FMM_ROTATED_COEFFICIENTS_RELATIVE_GRADIENT ||
                          em == FMM_POWER_RELATIVE_POTENTIAL);
   const bool potential = em == FMM_POWER_ABSOLUTE_POTENTIAL || em == FMM_POWER_RELATIVE_POTENTIAL;
@@ -325,9 +383,9 @@ __global__ void __launch_bounds__(32 * kW, 2)
       const int n = n0 + w;
       if (n <= p && active) {
         for (; n_sc < n; ++n_sc) sc *= rinv;
-        double Xr[PMAX + 1], Xi[PMAX + 1];
-        rotz_in<PMAX>(n, src, set, g, sc, Xr, Xi);
-        if (power) {  // rotate_z_n_power! (src/rotate.jl:528-576), weight 1 for every order
+        V Xr[PMAX + 1], Xi[PMAX + 1];
+        rotz_in<PMAX, V>(n, src, set, g, sc, Xr, Xi);
+        if (errc && power) {  // rotate_z_n_power! (src/rotate.jl:528-576), weight 1 for every order
           double a = 0.0;
 #pragma unroll
           for (int m = 0; m <= PMAX; ++m) {
@@ -338,8 +396,8 @@ __global__ void __launch_bounds__(32 * kW, 2)
           }
           pw[n * 32 + lane] = sqrt(a);
         }
-        rot_y<PMAX, false>(n, g, Xr, Xi);
-        double* o = Ms + 2 * hi(n, 0) * 32 + lane;
+        rot_y<PMAX, false, V>(n, (V)g.cth, (V)g.sth, Xr, Xi);
+        V* o = Ms + 2 * hi(n, 0) * 32 + lane;
 #pragma unroll
         for (int m = 0; m <= PMAX; ++m) {
           if (m > n) break;
@@ -348,101 +406,103 @@ __global__ void __launch_bounds__(32 * kW, 2)
         }
       }
       if (!errc) continue;
-      __syncthreads();
-      bool pass = false;
-      if (n >= 1 && n <= p) {  // the same for the whole warp: the exchanges below are uniform
-        for (; nt < n; ++nt) {
-          mp_pow *= r_mp_inv;
-          np1_fact *= nt + 1;
-          rl_pow *= r_l;
-          nm1_inv /= nt;
-        }
-        const int in0 = hi(n, 0);
-        double e_mp;
-        if (power) {
-          // phi: power of degree n - 1 (potential variants: n); chi: power of degree n
-          const int np = (potential || (LH && set)) ? n : n - 1;
-          const double Nn = (LH && set) ? c_Mt[in0] : c_Mt[hi(n - 1, 0)];
-          e_mp = 1.7320508075688772 * pw[np * 32 + lane] * mp_pow * np1_fact / Nn;
-          if (LH && set) e_mp *= n;
-          if (potential) e_mp *= r_mp / (n + 1);
-        } else {
-          const double* s = Ms + 2 * in0 * 32 + lane;
-          double un = 1.0;  // the stored degree is scaled by t^-n (chi t^(1-n))
-          for (int k = set; k < n; ++k) un *= g.r;
-          const double a1 = s[2 * 32], b1 = s[3 * 32];
-          e_mp = un * (sqrt(a1 * a1 + b1 * b1) + ((LH && set) ? 0.0 : fabs(s[0]))) * np1_fact * mp_pow;
-          if (LH && set) e_mp *= r_mp;
-        }
-        if (LH) e_mp += __shfl_xor_sync(kAll, e_mp, 16);
-        const bool need = active && e_mp <= thr;
-        if (__any_sync(kAll, need)) {
-          double tn1 = rinv;  // t^-(n+1)
-          for (int k = 0; k < n; ++k) tn1 *= rinv;
-          double e_l;
+      if constexpr (sizeof(V) == 8) {
+        __syncthreads();
+        bool pass = false;
+        if (n >= 1 && n <= p) {  // the same for the whole warp: the exchanges below are uniform
+          for (; nt < n; ++nt) {
+            mp_pow *= r_mp_inv;
+            np1_fact *= nt + 1;
+            rl_pow *= r_l;
+            nm1_inv /= nt;
+          }
+          const int in0 = hi(n, 0);
+          double e_mp;
           if (power) {
-            // degree n of translate_multipole_to_local_z_n! and local_power (src/translate.jl:238-295, 455-502)
-            double vr[PMAX + 1], vi[PMAX + 1];
-            coax<PMAX>(n, n, n, Ms, lane, vr, vi);
-            double a = 0.0;
+            // phi: power of degree n - 1 (potential variants: n); chi: power of degree n
+            const int np = (potential || (LH && set)) ? n : n - 1;
+            const double Nn = (LH && set) ? c_Mt[in0] : c_Mt[hi(n - 1, 0)];
+            e_mp = 1.7320508075688772 * pw[np * 32 + lane] * mp_pow * np1_fact / Nn;
+            if (LH && set) e_mp *= n;
+            if (potential) e_mp *= r_mp / (n + 1);
+          } else {
+            const double* s = Ms + 2 * in0 * 32 + lane;
+            double un = 1.0;  // the stored degree is scaled by t^-n (chi t^(1-n))
+            for (int k = set; k < n; ++k) un *= g.r;
+            const double a1 = s[2 * 32], b1 = s[3 * 32];
+            e_mp = un * (sqrt(a1 * a1 + b1 * b1) + ((LH && set) ? 0.0 : fabs(s[0]))) * np1_fact * mp_pow;
+            if (LH && set) e_mp *= r_mp;
+          }
+          if (LH) e_mp += __shfl_xor_sync(kAll, e_mp, 16);
+          const bool need = active && e_mp <= thr;
+          if (__any_sync(kAll, need)) {
+            double tn1 = rinv;  // t^-(n+1)
+            for (int k = 0; k < n; ++k) tn1 *= rinv;
+            double e_l;
+            if (power) {
+              // degree n of translate_multipole_to_local_z_n! and local_power (src/translate.jl:238-295, 455-502)
+              double vr[PMAX + 1], vi[PMAX + 1];
+              coax<PMAX, double>(n, n, n, Ms, lane, vr, vi);
+              double a = 0.0;
 #pragma unroll
-            for (int m = 0; m <= PMAX; ++m) {
-              if (m > n) break;
-              double pr = vr[m], pi = vi[m];
-              if (LH) {
-                const double qr = __shfl_xor_sync(kAll, vr[m], 16), qi = __shfl_xor_sync(kAll, vi[m], 16);
-                if (set == 0) {
-                  pr -= qi * m / n;
-                  pi += qr * m / n;
-                } else if (m < n) {
-                  pr -= vr[(m + 1) % (PMAX + 1)] * g.r / (n + 1);
-                  pi -= vi[(m + 1) % (PMAX + 1)] * g.r / (n + 1);
+              for (int m = 0; m <= PMAX; ++m) {
+                if (m > n) break;
+                double pr = vr[m], pi = vi[m];
+                if (LH) {
+                  const double qr = __shfl_xor_sync(kAll, vr[m], 16), qi = __shfl_xor_sync(kAll, vi[m], 16);
+                  if (set == 0) {
+                    pr -= qi * m / n;
+                    pi += qr * m / n;
+                  } else if (m < n) {
+                    pr -= vr[(m + 1) % (PMAX + 1)] * g.r / (n + 1);
+                    pi -= vi[(m + 1) % (PMAX + 1)] * g.r / (n + 1);
+                  }
+                }
+                const double Nt = c_Lt[in0 + m];
+                a += (pr * pr + pi * pi) * Nt * Nt;
+              }
+              e_l = 1.7320508075688772 * sqrt(a) * tn1 * rl_pow * nm1_inv / c_Lt[in0];
+              if (LH && set)
+                e_l *= rinv * r_l;
+              else if (potential)
+                e_l *= r_l / n;
+            } else {
+              // translate_multipole_to_local_z_m01_n (src/translate.jl:302-364)
+              double a0 = 0.0, b1r = 0.0, b1i = 0.0;
+              for (int np = 0; np <= n; ++np) {
+                const double c = c_fact[n + np];
+                const double* s = Ms + 2 * hi(np, 0) * 32 + lane;
+                a0 += c * s[0];
+                if (np > 0) {
+                  b1r += c * s[2 * 32];
+                  b1i += c * s[3 * 32];
                 }
               }
-              const double Nt = c_Lt[in0 + m];
-              a += (pr * pr + pi * pi) * Nt * Nt;
-            }
-            e_l = 1.7320508075688772 * sqrt(a) * tn1 * rl_pow * nm1_inv / c_Lt[in0];
-            if (LH && set)
-              e_l *= rinv * r_l;
-            else if (potential)
-              e_l *= r_l / n;
-          } else {
-            // translate_multipole_to_local_z_m01_n (src/translate.jl:302-364)
-            double a0 = 0.0, b1r = 0.0, b1i = 0.0;
-            for (int np = 0; np <= n; ++np) {
-              const double c = c_fact[n + np];
-              const double* s = Ms + 2 * hi(np, 0) * 32 + lane;
-              a0 += c * s[0];
-              if (np > 0) {
-                b1r += c * s[2 * 32];
-                b1i += c * s[3 * 32];
+              if (LH) {
+                const double qr = __shfl_xor_sync(kAll, b1r, 16), qi = __shfl_xor_sync(kAll, b1i, 16);
+                if (set == 0) {
+                  b1r -= qi / n;
+                  b1i += qr / n;
+                }
               }
+              e_l = (LH && set) ? sqrt(b1r * b1r + b1i * b1i) * rinv * r_l : fabs(b1r) + fabs(b1i) + fabs(a0);
+              e_l *= tn1 * rl_pow * nm1_inv;
             }
-            if (LH) {
-              const double qr = __shfl_xor_sync(kAll, b1r, 16), qi = __shfl_xor_sync(kAll, b1i, 16);
-              if (set == 0) {
-                b1r -= qi / n;
-                b1i += qr / n;
-              }
-            }
-            e_l = (LH && set) ? sqrt(b1r * b1r + b1i * b1i) * rinv * r_l : fabs(b1r) + fabs(b1i) + fabs(a0);
-            e_l *= tn1 * rl_pow * nm1_inv;
+            if (LH) e_l += __shfl_xor_sync(kAll, e_l, 16);
+            pass = need && e_mp + e_l * 2.0 <= thr;
           }
-          if (LH) e_l += __shfl_xor_sync(kAll, e_l, 16);
-          pass = need && e_mp + e_l * 2.0 <= thr;
         }
-      }
-      passed[w * 32 + lane] = pass;
-      __syncthreads();
-      if (active) {
+        passed[w * 32 + lane] = pass;
+        __syncthreads();
+        if (active) {
 #pragma unroll
-        for (int q = kW - 1; q >= 0; --q)
-          if (passed[q * 32 + lane]) {
-            P = n0 + q - 1 + (be ? 1 : 0);
-            ok = true;
-            active = false;
-          }
+          for (int q = kW - 1; q >= 0; --q)
+            if (passed[q * 32 + lane]) {
+              P = n0 + q - 1 + (be ? 1 : 0);
+              ok = true;
+              active = false;
+            }
+        }
       }
     }
     __syncthreads();
@@ -456,19 +516,19 @@ __global__ void __launch_bounds__(32 * kW, 2)
     for (int n = w; n <= top; n += kW) {
       for (; n_t < n; ++n_t) tn1 *= rinv;
       const bool on = valid && n <= P;
-      double Xr[PMAX + 1], Xi[PMAX + 1];
-      coax<PMAX>(n, n, on ? P : -1, Ms, lane, Xr, Xi);
+      V Xr[PMAX + 1], Xi[PMAX + 1];
+      coax<PMAX, V>(n, n, on ? P : -1, Ms, lane, Xr, Xi);
       if constexpr (LH) {
         // transform_lamb_helmholtz_local! (src/translate.jl:98-142) on the scaled sets
-        double Nr[PMAX + 1], Ni[PMAX + 1];
-        coax<PMAX>(n + 1, n, (on && set && n < P) ? P : -1, Ms, lane, Nr, Ni);
-        const double inv_n = n > 0 ? 1.0 / n : 0.0, inv_n1 = 1.0 / (n + 1);
+        V Nr[PMAX + 1], Ni[PMAX + 1];
+        coax<PMAX, V>(n + 1, n, (on && set && n < P) ? P : -1, Ms, lane, Nr, Ni);
+        const V inv_n = n > 0 ? V(1) / (V)n : V(0), inv_n1 = V(1) / (V)(n + 1);
 #pragma unroll
         for (int m = 0; m <= PMAX; ++m) {
           if (m > n) break;
-          const double qr = __shfl_xor_sync(kAll, Xr[m], 16), qi = __shfl_xor_sync(kAll, Xi[m], 16);
+          const V qr = __shfl_xor_sync(kAll, Xr[m], 16), qi = __shfl_xor_sync(kAll, Xi[m], 16);
           if (set == 0) {
-            const double a = m * inv_n;
+            const V a = (V)m * inv_n;
             Xr[m] -= a * qi;
             Xi[m] += a * qr;
           } else {
@@ -477,8 +537,8 @@ __global__ void __launch_bounds__(32 * kW, 2)
           }
         }
       }
-      rot_y<PMAX, true>(n, g, Xr, Xi);
-      rotz_back<PMAX>(n, g, Xr, Xi);
+      rot_y<PMAX, true, V>(n, (V)g.cth, (V)g.sth, Xr, Xi);
+      rotz_back<PMAX, V>(n, (V)g.cph, (V)g.sph, Xr, Xi);
       tsc[lane] = set ? tn1 * rinv : tn1;
       // sum over the pairs, value times power of t, one plane (re, im) at a time
 #pragma unroll
@@ -486,16 +546,16 @@ __global__ void __launch_bounds__(32 * kW, 2)
 #pragma unroll
         for (int m = 0; m <= PMAX; ++m) {
           if (m > n) break;
-          const double v = c ? Xi[m] : Xr[m];
-          stage[LH ? (2 * m + set) * 17 + slot : m * 33 + lane] = on ? v : 0.0;
+          const V v = c ? Xi[m] : Xr[m];
+          stage[LH ? (2 * m + set) * 17 + slot : m * 33 + lane] = on ? v : V(0);
         }
         __syncwarp();
         for (int row = lane; row < SETS * (n + 1); row += 32) {
           const double* ts = tsc + ((LH && (row & 1)) ? 16 : 0);
-          const double* sr = stage + row * (LH ? 17 : 33);
+          const V* sr = stage + row * (LH ? 17 : 33);
           double v = 0.0;
 #pragma unroll 8
-          for (int k = 0; k < NP; ++k) v += sr[k] * ts[k];
+          for (int k = 0; k < NP; ++k) v += (double)sr[k] * ts[k];
           acc[2 * (SETS * hi(n, 0) + row) + c] += v;
         }
         __syncwarp();
@@ -556,8 +616,8 @@ __global__ void __launch_bounds__(32 * ((PMAX + mm_degrees(LH)) / mm_degrees(LH)
   double* Ms = smem_d + (size_t)set * 2 * NH * 8;  // the set's rotated degrees [2 i + c][8]
   double Xr[PMAX + 1], Xi[PMAX + 1];
   if (on) {
-    rotz_in<PMAX>(n, src, set, g, 1.0, Xr, Xi);
-    rot_y<PMAX, LOCAL>(n, g, Xr, Xi);
+    rotz_in<PMAX, double>(n, src, set, g, 1.0, Xr, Xi);
+    rot_y<PMAX, LOCAL, double>(n, g.cth, g.sth, Xr, Xi);
 #pragma unroll
     for (int m = 0; m <= PMAX; ++m) {
       if (m > n) break;
@@ -619,8 +679,8 @@ __global__ void __launch_bounds__(32 * ((PMAX + mm_degrees(LH)) / mm_degrees(LH)
     }
   }
   if (on) {
-    rot_y<PMAX, LOCAL>(n, g, Xr, Xi);
-    rotz_back<PMAX>(n, g, Xr, Xi);
+    rot_y<PMAX, LOCAL, double>(n, g.cth, g.sth, Xr, Xi);
+    rotz_back<PMAX, double>(n, g.cph, g.sph, Xr, Xi);
   }
   double2* dst = reinterpret_cast<double2*>(E) + (int64_t)2 * NH * (LOCAL ? c : k);
   if constexpr (LOCAL) {
@@ -682,7 +742,7 @@ void allow_smem(K kernel, size_t bytes) {
     FMM_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
 }
 
-template <bool LH>
+template <bool LH, class V>
 struct M2LDegGo {
   DevTree& t;
   const DevTree& s;
@@ -693,14 +753,16 @@ struct M2LDegGo {
   cudaStream_t st;
   template <int PMAX>
   void go() {
-    const size_t sm = m2l_deg_smem<PMAX, LH>(p);
-    allow_smem(k_m2l_deg<PMAX, LH>, sm);
-    note_launch();
-    k_m2l_deg<PMAX, LH><<<(int)L.n_m2l_targets, 32 * kW, sm, st>>>(
-        L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-        t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, p, em, eps, be, stats, stats + 1,
-        reinterpret_cast<unsigned long long*>(stats + 2));
-    FMM_CUDA_TRY(cudaGetLastError());
+    if constexpr (sizeof(V) == 8 || PMAX <= kMaxF) {
+      const size_t sm = m2l_deg_smem<PMAX, LH, V>(p, em != FMM_ERROR_NONE);
+      allow_smem(k_m2l_deg<PMAX, LH, V>, sm);
+      note_launch();
+      k_m2l_deg<PMAX, LH, V><<<(int)L.n_m2l_targets, 32 * kW, sm, st>>>(
+          L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
+          t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, p, em, eps, be, stats, stats + 1,
+          reinterpret_cast<unsigned long long*>(stats + 2));
+      FMM_CUDA_TRY(cudaGetLastError());
+    }
   }
 };
 
@@ -729,13 +791,19 @@ struct MMLLGo {
 }  // namespace
 
 void launch_m2l_deg(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
-                    int* stats, cudaStream_t st) {
+                    int* stats, int precision, cudaStream_t st) {
   if (L.n_m2l_targets == 0) return;
   ensure_tables(st);
-  if (lh)
-    dispatch_pmax(p, M2LDegGo<true>{t, s, L, p, em, be, eps, stats, st});
+  // FP32 on the mixed path where the pairs' orders are fixed and its tables reach
+  const bool f32 = precision == FMM_PRECISION_MIXED && em == FMM_ERROR_NONE && p <= kMaxF;
+  if (lh && f32)
+    dispatch_pmax(p, M2LDegGo<true, float>{t, s, L, p, em, be, eps, stats, st});
+  else if (f32)
+    dispatch_pmax(p, M2LDegGo<false, float>{t, s, L, p, em, be, eps, stats, st});
+  else if (lh)
+    dispatch_pmax(p, M2LDegGo<true, double>{t, s, L, p, em, be, eps, stats, st});
   else
-    dispatch_pmax(p, M2LDegGo<false>{t, s, L, p, em, be, eps, stats, st});
+    dispatch_pmax(p, M2LDegGo<false, double>{t, s, L, p, em, be, eps, stats, st});
 }
 
 void launch_m2m(DevTree& s, int p, bool lh, cudaStream_t st) {
