@@ -457,10 +457,11 @@ __global__ void __launch_bounds__(32 * kWarps) k_p2m_lane(const int* __restrict_
         __syncwarp();
         const int hn = n * (n + 1) / 2;
         for (int v = lane; v < NC * (n + 1); v += 32) {
-          double t = 0.0;
-#pragma unroll 8
-          for (int k = 0; k < 32; ++k) t += stage[v * 33 + k];
-          Mb[4 * (hn + v / NC) + v % NC] += t;
+          // four partial sums: one chain of 32 additions was most of a degree's time
+          double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+          for (int k = 0; k < 32; ++k) t[k & 3] += stage[v * 33 + k];
+          Mb[4 * (hn + v / NC) + v % NC] += (t[0] + t[1]) + (t[2] + t[3]);
         }
         __syncwarp();
       }
@@ -534,25 +535,21 @@ __global__ void __launch_bounds__(32) k_op_p2m(const double4* __restrict__ pos, 
 constexpr int kL2PThreads = 128;
 constexpr int kCh = 13;  // channels: u, vx, vy, vz, h_xx..h_zz (column-major order)
 
-// threads tid of nthr (the CTA, or a group of lanes of one warp when !cta) fill C
-__device__ void l2p_coefficients(double* C, const double* __restrict__ L, int p, bool lh, bool ps, bool gs, bool hs,
-                                 int tid, int nthr, bool cta) {
+// threads tid of nthr (the CTA, or a group of lanes of one warp when !cta) fill C.  The gradient
+// entries are the velocity formula applied to the velocity coefficients, which are read back from
+// channels 1..3 (kept there whether or not the velocity itself is requested).
+template <bool PS, bool GS, bool HS>
+__device__ __forceinline__ void l2p_coefficients(double* C, const double* __restrict__ L, int p, bool lh, int tid,
+                                                 int nthr, bool cta) {
   // C[(ch * NH + i) * 2 + reim]
   const int NH = (p + 1) * (p + 2) / 2;
+  double2* C2 = reinterpret_cast<double2*>(C);
   for (int i = tid; i < NH; i += nthr) {
     int n, m;
     nm_of(i, n, m);
-    double* c = C;
-    // potential
-    double ur = 0, ui = 0;
-    if (ps && (n == 0 || !lh)) {
-      ur = L[4 * i];
-      ui = L[4 * i + 1];
-    }
-    c[(0 * NH + i) * 2] = ur;
-    c[(0 * NH + i) * 2 + 1] = ui;
-    double vxr = 0, vxi = 0, vyr = 0, vyi = 0, vzr = 0, vzi = 0;
-    if (gs || hs) {
+    if (PS) C2[i] = (n == 0 || !lh) ? make_double2(L[4 * i], L[4 * i + 1]) : make_double2(0.0, 0.0);
+    if (GS || HS) {
+      double vxr = 0, vxi = 0, vyr = 0, vyi = 0, vzr = 0, vzi = 0;
       if (m == 0) {
         if (n == 0 || n < p) {
           int a = i + n + 1, b2 = i + n + 2;
@@ -592,117 +589,46 @@ __device__ void l2p_coefficients(double* C, const double* __restrict__ L, int p,
           vzi -= m * L[4 * i + 2];
         }
       }
-    }
-    double V[6] = {vxr, vxi, vyr, vyi, vzr, vzi};
-    for (int d = 0; d < 3; ++d) {
-      c[((1 + d) * NH + i) * 2] = gs ? V[2 * d] : 0.0;
-      c[((1 + d) * NH + i) * 2 + 1] = gs ? V[2 * d + 1] : 0.0;
+      C2[NH + i] = make_double2(vxr, vxi);
+      C2[2 * NH + i] = make_double2(vyr, vyi);
+      C2[3 * NH + i] = make_double2(vzr, vzi);
     }
   }
   if (cta)
     __syncthreads();
   else
     __syncwarp();
-  // hessian channels from the velocity coefficients ("gradient_n_m"), n <= p-1
-  for (int i = tid; i < NH; i += nthr) {
-    int n, m;
-    nm_of(i, n, m);
-    double h[9][2];
-    for (int a = 0; a < 9; ++a) h[a][0] = h[a][1] = 0.0;
-    if (hs && n <= p - 1) {
-      // G(comp, idx): velocity coefficient comp of entry idx (stored in channels 1..3 when gs;
-      // recomputed here from L when the gradient itself is not requested)
-      auto G = [&](int comp, int idx, int reim) -> double {
-        int nn, mm;
-        nm_of(idx, nn, mm);
-        double vr = 0, vi = 0;
-        // same formulas as above for entry idx, component comp
-        if (mm == 0) {
-          if (nn == 0 || nn < p) {
-            int a = idx + nn + 1, b2 = idx + nn + 2;
-            if (comp == 0) vr -= L[4 * b2 + 1];
-            if (comp == 1) vr -= L[4 * b2];
-            if (comp == 2) {
-              vr -= L[4 * a];
-              vi -= L[4 * a + 1];
-            }
-          }
-          if (lh && nn > 0) {
-            if (comp == 0) vr += nn * L[4 * (idx + 1) + 2];
-            if (comp == 1) vr -= nn * L[4 * (idx + 1) + 3];
-          }
-        } else {
-          if (nn < p) {
-            int am = idx + nn, a0 = idx + nn + 1, ap = idx + nn + 2;
-            if (comp == 0) {
-              vr -= (L[4 * am + 1] + L[4 * ap + 1]) * 0.5;
-              vi += (L[4 * am] + L[4 * ap]) * 0.5;
-            } else if (comp == 1) {
-              vr += (L[4 * am] - L[4 * ap]) * 0.5;
-              vi += (L[4 * am + 1] - L[4 * ap + 1]) * 0.5;
-            } else {
-              vr -= L[4 * a0];
-              vi -= L[4 * a0 + 1];
-            }
-          }
-          if (lh) {
-            double cmr = L[4 * (idx - 1) + 2], cmi = L[4 * (idx - 1) + 3];
-            if (comp == 0) {
-              vr -= (nn + mm) * cmr * 0.5;
-              vi -= (nn + mm) * cmi * 0.5;
-            } else if (comp == 1) {
-              vr -= (nn + mm) * cmi * 0.5;
-              vi += (nn + mm) * cmr * 0.5;
-            }
-            if (mm < nn) {
-              double cpr = L[4 * (idx + 1) + 2], cpi = L[4 * (idx + 1) + 3];
-              if (comp == 0) {
-                vr += (nn - mm) * cpr * 0.5;
-                vi += (nn - mm) * cpi * 0.5;
-              } else if (comp == 1) {
-                vr -= (nn - mm) * cpi * 0.5;
-                vi += (nn - mm) * cpr * 0.5;
-              }
-            }
-            if (comp == 2) {
-              vr += mm * L[4 * idx + 3];
-              vi -= mm * L[4 * idx + 2];
-            }
-          }
-        }
-        return reim ? vi : vr;
-      };
-      for (int col = 0; col < 3; ++col) {
+  if constexpr (HS) {
+    // gradient channels from the velocity coefficients ("gradient_n_m"), n <= p-1: column col
+    // (x, y, z component of the velocity) in rows x, y, z of the derivative, channel 4 + 3 row + col
+    for (int e = tid; e < 3 * NH; e += nthr) {
+      const int col = e / NH, i = e - col * NH;
+      int n, m;
+      nm_of(i, n, m);
+      double2 hx = make_double2(0, 0), hy = hx, hz = hx;
+      if (n <= p - 1) {
+        const double2* G = C2 + (1 + col) * NH;
+        const double2 g0 = G[i + n + 1], gp = G[i + n + 2];
         if (m == 0) {
-          int ap = i + n + 2, a0 = i + n + 1;
-          h[3 * col + 0][0] = -G(col, ap, 1);
-          h[3 * col + 1][0] = -G(col, ap, 0);
-          h[3 * col + 2][0] = -G(col, a0, 0);
-          h[3 * col + 2][1] = -G(col, a0, 1);
+          hx.x = -gp.y;
+          hy.x = -gp.x;
+          hz = make_double2(-g0.x, -g0.y);
         } else {
-          int am = i + n, a0 = i + n + 1, ap = i + n + 2;
-          h[3 * col + 0][0] = -(G(col, am, 1) + G(col, ap, 1)) * 0.5;
-          h[3 * col + 0][1] = (G(col, am, 0) + G(col, ap, 0)) * 0.5;
-          h[3 * col + 1][0] = (G(col, am, 0) - G(col, ap, 0)) * 0.5;
-          h[3 * col + 1][1] = (G(col, am, 1) - G(col, ap, 1)) * 0.5;
-          h[3 * col + 2][0] = -G(col, a0, 0);
-          h[3 * col + 2][1] = -G(col, a0, 1);
+          const double2 gm = G[i + n];
+          hx = make_double2(-(gm.y + gp.y) * 0.5, (gm.x + gp.x) * 0.5);
+          hy = make_double2((gm.x - gp.x) * 0.5, (gm.y - gp.y) * 0.5);
+          hz = make_double2(-g0.x, -g0.y);
         }
       }
+      C2[(4 + col) * NH + i] = hx;
+      C2[(7 + col) * NH + i] = hy;
+      C2[(10 + col) * NH + i] = hz;
     }
-    // channel 4 + (row + 3*col) for the SMatrix(vxx, vxy, vxz, vyx, ...) order:
-    // entry (row r = x|y|z of velocity, col c = derivative direction): vrc at 4 + 3*r + c
-    for (int col = 0; col < 3; ++col)
-      for (int row = 0; row < 3; ++row) {
-        int ch = 4 + 3 * row + col;
-        C[(ch * NH + i) * 2] = h[3 * col + row][0];
-        C[(ch * NH + i) * 2 + 1] = h[3 * col + row][1];
-      }
+    if (cta)
+      __syncthreads();
+    else
+      __syncwarp();
   }
-  if (cta)
-    __syncthreads();
-  else
-    __syncwarp();
 }
 
 // 1/k for the body-wise recursions (k <= 2 kMaxP + 1): a product with 1/k in place of the
@@ -713,9 +639,19 @@ __constant__ double c_rcp[42] = {
     1.0 / 22, 1.0 / 23, 1.0 / 24, 1.0 / 25, 1.0 / 26, 1.0 / 27, 1.0 / 28, 1.0 / 29, 1.0 / 30, 1.0 / 31,
     1.0 / 32, 1.0 / 33, 1.0 / 34, 1.0 / 35, 1.0 / 36, 1.0 / 37, 1.0 / 38, 1.0 / 39, 1.0 / 40, 1.0 / 41};
 
-// contract one body: regular harmonics by the reference's column recursion
-__device__ void l2p_body(const double* C, int p, double x, double y, double z, bool ps, bool gs, bool hs, double* out) {
+// 1 / ((2 m + 2) (2 m + 1)), the step of rho^m / (2 m)! along the diagonal
+__device__ __forceinline__ double rcp_diag(int m) { return c_rcp[2 * m + 2] * c_rcp[2 * m + 1]; }
+
+// contract one body: regular harmonics by the reference's column recursion.  The requested channels
+// are template arguments, so that the sums stay in registers (as run-time flags they were indexed in
+// local memory: 30k vortex ring, order 8, 95 -> 28 us); bound by the FP64 pipe, two FMAs per channel
+// and coefficient.
+template <bool PS, bool GS, bool HS>
+__device__ __forceinline__ void l2p_body(const double* __restrict__ C, int p, double x, double y, double z,
+                                         double* __restrict__ out) {
+  constexpr int C0 = PS ? 0 : GS ? 1 : 4, C1 = HS ? kCh : GS ? 4 : 1;  // channels [C0, C1) (1..3 too for PS and HS)
   const int NH = (p + 1) * (p + 2) / 2;
+  const double2* __restrict__ C2 = reinterpret_cast<const double2*>(C);
   // cos and sin of the polar angle and e^{i (phi + pi/2)} of cartesian_to_spherical
   // (src/rotate.jl:9-21) straight from the offsets, without forming the angles (the same
   // values up to rounding; on the z axis exact 0 where the trigonometric route leaves ~1e-16)
@@ -737,26 +673,24 @@ __device__ void l2p_body(const double* C, int p, double x, double y, double z, b
   double fact = 1.0, pn = 1.0, rhom = 1.0;
   double er = 1.0, ei = 0.0;
   double a[kCh];
+#pragma unroll
   for (int c = 0; c < kCh; ++c) a[c] = 0.0;
-  const int nch = hs ? kCh : 4;
+#pragma unroll 1
   for (int m = 0; m <= p; ++m) {
     double pl = pn;
     double rhon = rhom;
     double p1 = pl, p2 = 0;
-    double wgt = (m == 0) ? 1.0 : 2.0;
+    const double wr = (m == 0 ? 1.0 : 2.0) * er, wi = (m == 0 ? 1.0 : 2.0) * ei;
+#pragma unroll 1
     for (int n = m; n <= p; ++n) {
-      double R;
-      if (n == m) {
-        R = rhom * pl;
-      } else {
-        rhon *= -c_rcp[n + m];
-        R = rhon * pl;
-      }
-      double Rr = R * er, Ri = R * ei;
-      int i = n * (n + 1) / 2 + m;
-      for (int c = 0; c < nch; ++c) {
-        double cr = C[(c * NH + i) * 2], ci = C[(c * NH + i) * 2 + 1];
-        a[c] += wgt * (Rr * cr - Ri * ci);
+      if (n > m) rhon *= -c_rcp[n + m];
+      const double R = rhon * pl;
+      const double Rr = R * wr, Ri = -(R * wi);
+      const double2* q = C2 + (n * (n + 1) / 2 + m);
+#pragma unroll
+      for (int c = C0; c < C1; ++c) {
+        const double2 v = q[c * NH];
+        a[c] = fma(Ri, v.y, fma(Rr, v.x, a[c]));
       }
       // Legendre recursion
       if (n == m) {
@@ -771,73 +705,77 @@ __device__ void l2p_body(const double* C, int p, double x, double y, double z, b
         rhon *= r;
       }
     }
-    rhom /= -(2 * m + 2) * (2 * m + 1);
+    rhom *= -rcp_diag(m);
     pn = -pn * fact * sy;
     fact += 2;
     double tr = er, ti = ei;
     er = tr * iei_r - ti * iei_i;
     ei = tr * iei_i + ti * iei_r;
   }
-  if (ps) out[0] += -a[0] * kOneOver4Pi;
-  if (gs) {
+  if (PS) out[0] += -a[0] * kOneOver4Pi;
+  if (GS) {
     out[1] += a[1] * kOneOver4Pi;
     out[2] += a[2] * kOneOver4Pi;
     out[3] += a[3] * kOneOver4Pi;
   }
-  if (hs)
+  if (HS)
+#pragma unroll
     for (int c = 4; c < kCh; ++c) out[c] += a[c] * kOneOver4Pi;
 }
 
+template <bool PS, bool GS, bool HS>
 __global__ void __launch_bounds__(kL2PThreads) k_l2p(const int* __restrict__ leaf_index,
                                                      const int* __restrict__ body_start,
                                                      const int* __restrict__ body_count,
                                                      const double* __restrict__ tcen, const double4* __restrict__ pos,
-                                                     const double* __restrict__ L, int p, int lh, int ps, int gs, int hs,
+                                                     const double* __restrict__ L, int p, int lh,
                                                      double* __restrict__ acc13) {
-  extern __shared__ double C[];
+  extern __shared__ __align__(16) double C[];
   const int b = leaf_index[blockIdx.x];
-  l2p_coefficients(C, L + 4 * nh(p) * b, p, lh != 0, ps != 0, gs != 0, hs != 0, threadIdx.x, blockDim.x, true);
+  l2p_coefficients<PS, GS, HS>(C, L + 4 * nh(p) * b, p, lh != 0, threadIdx.x, blockDim.x, true);
   const int s0 = body_start[b], cnt = body_count[b];
   const double cx = tcen[3 * b], cy = tcen[3 * b + 1], cz = tcen[3 * b + 2];
   for (int j = threadIdx.x; j < cnt; j += blockDim.x) {
     double4 x = pos[s0 + j];
-    l2p_body(C, p, x.x - cx, x.y - cy, x.z - cz, ps != 0, gs != 0, hs != 0, acc13 + 13 * (int64_t)(s0 + j));
+    l2p_body<PS, GS, HS>(C, p, x.x - cx, x.y - cy, x.z - cz, acc13 + 13 * (int64_t)(s0 + j));
   }
 }
 
 // leaves of a few bodies: a group of 8 lanes per leaf, 16 leaves per CTA of 128 threads,
 // each group with its own coefficients in shared memory
 constexpr int kL2PGroup = 8, kL2PGroupThreads = 128;
+template <bool PS, bool GS, bool HS>
 __global__ void __launch_bounds__(kL2PGroupThreads) k_l2p_group(const int* __restrict__ leaf_index, int n_leaves,
                                                                const int* __restrict__ body_start,
                                                                const int* __restrict__ body_count,
                                                                const double* __restrict__ tcen,
                                                                const double4* __restrict__ pos,
-                                                               const double* __restrict__ L, int p, int lh, int ps,
-                                                               int gs, int hs, double* __restrict__ acc13) {
-  extern __shared__ double Cg[];
+                                                               const double* __restrict__ L, int p, int lh,
+                                                               double* __restrict__ acc13) {
+  extern __shared__ __align__(16) double Cg[];
   const int g = threadIdx.x / kL2PGroup, lane = threadIdx.x % kL2PGroup;
   const int leaf = blockIdx.x * (kL2PGroupThreads / kL2PGroup) + g;
   const bool valid = leaf < n_leaves;  // groups past the end repeat the last leaf and write nothing
   const int b = leaf_index[valid ? leaf : n_leaves - 1];
   double* C = Cg + (size_t)g * kCh * 2 * nh(p);
-  l2p_coefficients(C, L + 4 * nh(p) * b, p, lh != 0, ps != 0, gs != 0, hs != 0, lane, kL2PGroup, false);
+  l2p_coefficients<PS, GS, HS>(C, L + 4 * nh(p) * b, p, lh != 0, lane, kL2PGroup, false);
   if (!valid) return;
   const int s0 = body_start[b], cnt = body_count[b];
   const double cx = tcen[3 * b], cy = tcen[3 * b + 1], cz = tcen[3 * b + 2];
   for (int j = lane; j < cnt; j += kL2PGroup) {
     double4 x = pos[s0 + j];
-    l2p_body(C, p, x.x - cx, x.y - cy, x.z - cz, ps != 0, gs != 0, hs != 0, acc13 + 13 * (int64_t)(s0 + j));
+    l2p_body<PS, GS, HS>(C, p, x.x - cx, x.y - cy, x.z - cz, acc13 + 13 * (int64_t)(s0 + j));
   }
 }
 
+template <bool PS, bool GS, bool HS>
 __global__ void __launch_bounds__(kL2PThreads) k_op_l2p(int64_t n, const double* __restrict__ dx,
-                                                        const double* __restrict__ L, int p, int lh, int ps, int gs,
-                                                        int hs, double* __restrict__ out13) {
-  extern __shared__ double C[];
-  l2p_coefficients(C, L, p, lh != 0, ps != 0, gs != 0, hs != 0, threadIdx.x, blockDim.x, true);
+                                                        const double* __restrict__ L, int p, int lh,
+                                                        double* __restrict__ out13) {
+  extern __shared__ __align__(16) double C[];
+  l2p_coefficients<PS, GS, HS>(C, L, p, lh != 0, threadIdx.x, blockDim.x, true);
   for (int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; j < n; j += (int64_t)gridDim.x * blockDim.x)
-    l2p_body(C, p, dx[3 * j], dx[3 * j + 1], dx[3 * j + 2], ps != 0, gs != 0, hs != 0, out13 + 13 * j);
+    l2p_body<PS, GS, HS>(C, p, dx[3 * j], dx[3 * j + 1], dx[3 * j + 2], out13 + 13 * j);
 }
 
 inline size_t pair_smem(int p) { return (size_t)kWarps * ws_doubles(p) * sizeof(double); }
@@ -952,26 +890,70 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
   launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, precision, st);
 }
 
+namespace {
+// call f.template go<PS, GS, HS>() for the requested outputs (nothing for none)
+template <class F>
+void dispatch_outputs(bool ps, bool gs, bool hs, F&& f) {
+  if (ps && gs && hs) f.template go<true, true, true>();
+  else if (ps && gs) f.template go<true, true, false>();
+  else if (ps && hs) f.template go<true, false, true>();
+  else if (ps) f.template go<true, false, false>();
+  else if (gs && hs) f.template go<false, true, true>();
+  else if (gs) f.template go<false, true, false>();
+  else if (hs) f.template go<false, false, true>();
+}
+
+struct L2PGo {
+  DevTree& t;
+  int p;
+  bool lh;
+  double* acc13;
+  cudaStream_t st;
+  template <bool PS, bool GS, bool HS>
+  void go() {
+    const size_t sm = l2p_smem(p);
+    note_launch();
+    const bool small = t.n_bodies <= 8 * t.n_leaves;
+    const size_t smg = (kL2PGroupThreads / kL2PGroup) * sm;
+    if (small && smg <= 96 * 1024) {
+      // leaves of a few bodies (on average <= 8), low orders: 8 lanes each, 16 per CTA
+      allow_smem(k_l2p_group<PS, GS, HS>, smg);
+      const int per = kL2PGroupThreads / kL2PGroup;
+      k_l2p_group<PS, GS, HS><<<(int)((t.n_leaves + per - 1) / per), kL2PGroupThreads, smg, st>>>(
+          t.leaf_index.ptr, (int)t.n_leaves, t.body_start.ptr, t.body_count.ptr, t.tcenter.ptr, t.pos.ptr, t.local.ptr,
+          p, lh ? 1 : 0, acc13);
+    } else {
+      allow_smem(k_l2p<PS, GS, HS>, sm);
+      k_l2p<PS, GS, HS><<<(int)t.n_leaves, small ? 32 : kL2PThreads, sm, st>>>(
+          t.leaf_index.ptr, t.body_start.ptr, t.body_count.ptr, t.tcenter.ptr, t.pos.ptr, t.local.ptr, p, lh ? 1 : 0,
+          acc13);
+    }
+    FMM_CUDA_TRY(cudaGetLastError());
+  }
+};
+
+struct OpL2PGo {
+  int64_t n;
+  const double *dx, *local;
+  int p;
+  bool lh;
+  double* out13;
+  cudaStream_t st;
+  template <bool PS, bool GS, bool HS>
+  void go() {
+    const size_t sm = l2p_smem(p);
+    allow_smem(k_op_l2p<PS, GS, HS>, sm);
+    const int g = (int)std::min<int64_t>((n + kL2PThreads - 1) / kL2PThreads, 1024);
+    note_launch();
+    k_op_l2p<PS, GS, HS><<<g, kL2PThreads, sm, st>>>(n, dx, local, p, lh ? 1 : 0, out13);
+    FMM_CUDA_TRY(cudaGetLastError());
+  }
+};
+}  // namespace
+
 void launch_l2p(DevTree& t, int p, bool lh, bool ps, bool gs, bool hs, double* acc13, cudaStream_t st) {
   if (t.n_leaves == 0) return;
-  size_t sm = l2p_smem(p);
-  note_launch();
-  const bool small = t.n_bodies <= 8 * t.n_leaves;
-  const size_t smg = (kL2PGroupThreads / kL2PGroup) * sm;
-  if (small && smg <= 96 * 1024) {
-    // leaves of a few bodies (on average <= 8), low orders: 8 lanes each, 16 per CTA
-    allow_smem(k_l2p_group, smg);
-    const int per = kL2PGroupThreads / kL2PGroup;
-    k_l2p_group<<<(int)((t.n_leaves + per - 1) / per), kL2PGroupThreads, smg, st>>>(
-        t.leaf_index.ptr, (int)t.n_leaves, t.body_start.ptr, t.body_count.ptr, t.tcenter.ptr, t.pos.ptr, t.local.ptr,
-        p, lh ? 1 : 0, ps ? 1 : 0, gs ? 1 : 0, hs ? 1 : 0, acc13);
-  } else {
-    allow_smem(k_l2p, sm);
-    k_l2p<<<(int)t.n_leaves, small ? 32 : kL2PThreads, sm, st>>>(t.leaf_index.ptr, t.body_start.ptr, t.body_count.ptr,
-                                                     t.tcenter.ptr, t.pos.ptr, t.local.ptr, p, lh ? 1 : 0, ps ? 1 : 0,
-                                                     gs ? 1 : 0, hs ? 1 : 0, acc13);
-  }
-  FMM_CUDA_TRY(cudaGetLastError());
+  dispatch_outputs(ps, gs, hs, L2PGo{t, p, lh, acc13, st});
 }
 
 void launch_op_m2m(int64_t n, double* target, const double* tc, const double* src, const double* sc, int p, bool lh,
@@ -1000,12 +982,7 @@ void launch_op_p2m(int kind, const double4* pos, const double4* str, int64_t n, 
 void launch_op_l2p(int64_t n, const double* dx, const double* local, int p, bool lh, bool ps, bool gs, bool hs,
                    double* out13, cudaStream_t st) {
   if (n == 0) return;
-  size_t sm = l2p_smem(p);
-  allow_smem(k_op_l2p, sm);
-  int g = (int)std::min<int64_t>((n + kL2PThreads - 1) / kL2PThreads, 1024);
-  note_launch();
-  k_op_l2p<<<g, kL2PThreads, sm, st>>>(n, dx, local, p, lh ? 1 : 0, ps ? 1 : 0, gs ? 1 : 0, hs ? 1 : 0, out13);
-  FMM_CUDA_TRY(cudaGetLastError());
+  dispatch_outputs(ps, gs, hs, OpL2PGo{n, dx, local, p, lh, out13, st});
 }
 
 }  // namespace fmmb
