@@ -7,8 +7,8 @@
 // passes and the unsort of the target buffer.  The trees, the lists, the near field
 // and the unsort run on the context's stream; the far field (upward pass, M2L,
 // downward pass) runs on a second high-priority stream concurrently with the near
-// field, and the influence estimate's sub-solve on a third; the tree and list
-// builders synchronise with the host once per level (trees) or per build (lists).
+// field, and the influence estimate's sub-solve on a third; the tree and list builders
+// wait for the device once each (large trees once more per four levels).
 #include <algorithm>
 #include <cstring>
 #include <string>

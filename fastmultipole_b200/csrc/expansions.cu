@@ -1,18 +1,12 @@
-// expansions.cu -- far-field kernels: P2M, M2M, M2L (plain and error-controlled),
-// L2L and L2P, FP64, rotation-based ("point-and-shoot") operators.
+// expansions.cu -- far-field kernels: P2M, L2P, the low-order vortex M2L, the routing of
+// the M2L, and the single-operator entry points, FP64.
 //
-// Every translation follows the reference's operator chain
+// The single operators follow the reference's operator chain
 //   rotate about z (e^{i m phi})  ->  rotate about y (Wigner d at theta, built
 //   from the pi/2 table)  ->  coaxial translation along z  ->  [Lamb-Helmholtz
 //   re-centring]  ->  rotate back about y  ->  rotate back about z and accumulate
-// (src/translate.jl:144-174, 519-550, 1896-1926; src/rotate.jl).  One warp
-// owns one output expansion (a target branch for M2L, a parent for M2M, a
-// child for L2L), loops over its inputs, keeps the sum in registers (lane l
-// holds coefficients l, l+32, ...) and writes once: no atomics.  Intermediate
-// expansions, the Wigner matrices and e^{i m phi} live in the warp's slice of
-// shared memory; the lanes split each stage over output coefficients
-// (n, m), or over (m, m') for the Wigner entries, or over m for the
-// column-recursive steps.
+// (src/translate.jl:144-174, 519-550, 1896-1926; src/rotate.jl), one warp per output
+// expansion (engine.cuh).  The tree's translations are in translate_deg.cu and m2l_lane.cu.
 //
 // Expansion layout: 4*Nh doubles per branch, e[4*i + 2*set + reim], i = n(n+1)/2 + m,
 // set 0 = phi, set 1 = chi (Lamb-Helmholtz), as the reference's Tree.expansions.
@@ -54,7 +48,7 @@ __device__ __forceinline__ void acc_store_add(double* dst, const double (&acc)[k
 }
 
 // ---------------------------------------------------------------------------
-// translation kernels (templated on SLOTS = ceil(Nh/32) and Lamb-Helmholtz)
+// translations (the unit operators templated on SLOTS = ceil(Nh/32) and Lamb-Helmholtz)
 
 using eng::Tab;
 using eng::WS;

@@ -72,3 +72,17 @@ def test_max_influence_of_ancestors():
             assert t["max_influence"][k] == t["max_influence"][c0:c0 + nc].max()
     assert t["max_influence"].min() > 0
     ctx.close()
+
+
+def test_traversals_of_changing_size():
+    """One context, systems whose traversals outgrow what the previous build's let expect, and back."""
+    ctx = fm.Context(0)
+    rng = np.random.default_rng(9)
+    for n, ls in ((900, 4), (60, 4), (30000, 4), (2500, 40), (12000, 3), (1, 1), (5000, 2)):
+        b = points(rng.random((n, 3)) ** 2, n)
+        og, oo = opt_pair(expansion_order=1, leaf_size_source=ls, multipole_acceptance=0.4)
+        fm.solve_buffers(b, L.FMM_POINT_SOURCE, og, ctx=ctx)
+        ref = O.fmm(b, O.POINT_SOURCE, oo, want_tree=True)
+        compare_trees(fm.get_tree(ctx, 1), ref["source_tree"])
+        compare_lists(*fm.get_lists(ctx), ref["m2l"], ref["direct"])
+    ctx.close()
