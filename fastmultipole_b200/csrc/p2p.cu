@@ -8,7 +8,7 @@
 // k_p2p (direct list): one CTA per target leaf, source bodies gathered into
 // warp-private shared-memory batches, lanes split between targets and sources
 // by the leaf's size (details at the kernel).  k_direct (all pairs): one CTA
-// per block of targets, sources staged through shared memory.  FP64 is the
+// per block of targets and share of the sources, staged through shared memory.  FP64 is the
 // drop-in arithmetic; the MIXED variant moves every body relative to a nearby
 // centre in FP64, then evaluates the kernel in FP32 (rsqrt on the SFU),
 // summing blocks of sources in FP32 and the block partials in FP64.
