@@ -625,16 +625,19 @@ __device__ __forceinline__ void l2p_coefficients(double* C, const double* __rest
   }
 }
 
-// 1/k for the body-wise recursions (k <= 2 kMaxP + 1): a product with 1/k in place of the
-// division by k in the hot loops (within an ulp of the quotient)
-__constant__ double c_rcp[42] = {
+// 1/k for the body-wise recursions: a product with 1/k in place of the division by k in the hot
+// loops (within an ulp of the quotient)
+__constant__ double c_rcp[] = {
     0.0, 1.0 / 1, 1.0 / 2, 1.0 / 3, 1.0 / 4, 1.0 / 5, 1.0 / 6, 1.0 / 7, 1.0 / 8, 1.0 / 9, 1.0 / 10, 1.0 / 11,
     1.0 / 12, 1.0 / 13, 1.0 / 14, 1.0 / 15, 1.0 / 16, 1.0 / 17, 1.0 / 18, 1.0 / 19, 1.0 / 20, 1.0 / 21,
     1.0 / 22, 1.0 / 23, 1.0 / 24, 1.0 / 25, 1.0 / 26, 1.0 / 27, 1.0 / 28, 1.0 / 29, 1.0 / 30, 1.0 / 31,
-    1.0 / 32, 1.0 / 33, 1.0 / 34, 1.0 / 35, 1.0 / 36, 1.0 / 37, 1.0 / 38, 1.0 / 39, 1.0 / 40, 1.0 / 41};
+    1.0 / 32, 1.0 / 33, 1.0 / 34, 1.0 / 35, 1.0 / 36, 1.0 / 37, 1.0 / 38, 1.0 / 39, 1.0 / 40, 1.0 / 41,
+    1.0 / 42};
 
-// 1 / ((2 m + 2) (2 m + 1)), the step of rho^m / (2 m)! along the diagonal
-__device__ __forceinline__ double rcp_diag(int m) { return c_rcp[2 * m + 2] * c_rcp[2 * m + 1]; }
+// 1 / ((2 m + 2) (2 m + 1)), the step of rho^m / (2 m)! along the diagonal (m up to the order)
+__host__ __device__ constexpr int diag_index(int m) { return 2 * m + 2; }
+static_assert(diag_index(kMaxP) < (int)(sizeof(c_rcp) / sizeof(double)), "the diagonal step reads past 1/k");
+__device__ __forceinline__ double rcp_diag(int m) { return c_rcp[diag_index(m)] * c_rcp[diag_index(m) - 1]; }
 
 // contract one body: regular harmonics by the reference's column recursion.  The requested channels
 // are template arguments, so that the sums stay in registers (as run-time flags they were indexed in

@@ -220,6 +220,25 @@ def test_l2p_matches_oracle(ctx, p, lh):
         np.testing.assert_allclose(out[k], ref, rtol=0, atol=1e-12 * np.abs(ref).max())
 
 
+@pytest.mark.parametrize("lh", [0, 1])
+@pytest.mark.parametrize("ps,gs,hs", [(1, 1, 1), (1, 0, 0), (0, 1, 0), (0, 0, 1)])
+def test_l2p_at_the_highest_order(ctx, lh, ps, gs, hs):
+    """Order 20 uses the recursions' whole table of reciprocals."""
+    p, n = 20, 33
+    rng = np.random.default_rng(20 + lh)
+    Lx = rng.standard_normal(4 * O.nh(p))
+    if not lh:
+        Lx.reshape(-1, 4)[:, 2:] = 0
+    dx = 0.3 * rng.standard_normal((n, 3))
+    out = np.zeros((n, 13))
+    ctx.check(L.lib().fmm_op_l2p(ctx.handle, n, d(dx), d(Lx), p, lh, ps, gs, hs, d(out)))
+    for k in range(n):
+        phi, g, H = np.zeros(1), np.zeros(3), np.zeros(9)
+        O.lib().oracle_l2p(O.dptr(dx[k].copy()), O.dptr(Lx), p, lh, 1, 1, 1, O.dptr(phi), O.dptr(g), O.dptr(H))
+        ref = np.concatenate([phi * ps, g * gs, H * hs])
+        np.testing.assert_allclose(out[k], ref, rtol=0, atol=1e-12 * np.abs(ref).max())
+
+
 def test_measured_fp32_peak_is_plausible():
     # the near field's roofline denominator: independent FMA chains on every SM of a B200
     # (nominal 148 SMs x 128 lanes x 2 flop x ~1.9 GHz = 74 TFLOP/s)
