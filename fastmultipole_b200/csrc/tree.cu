@@ -647,6 +647,7 @@ __global__ void k_leaf_bodies(Branches B, int n_leaves, const int* __restrict__ 
       __threadfence();
     }
     if (!__shfl_sync(mask, last, 0, 8)) break;
+    __syncwarp(mask);  // the other lanes' loads of the children after lane 0's fence (a shuffle orders no memory)
     shrink_branch(geo, mask, lane, k, B.child_start[k], nc);
     __syncwarp(mask);
   }

@@ -74,6 +74,33 @@ def test_max_influence_of_ancestors():
     ctx.close()
 
 
+@pytest.mark.parametrize("n,ls", [(60001, 1), (60001, 3), (200003, 40)])
+def test_ancestors_enclose_finished_children(n, ls):
+    """Every branch's geometry is the one its children's gives, bit for bit, build after build: a
+    parent is formed by whichever child is last to finish, from what other SMs wrote."""
+    b = points(np.random.default_rng(n + ls).random((n, 3)) ** 2)
+    ctx = fm.Context(0)
+    og = fm.make_options(expansion_order=1, leaf_size_source=ls, farfield=False, nearfield=False)
+    for _ in range(5):
+        fm.solve_buffers(b, L.FMM_POINT_SOURCE, og, ctx=ctx)
+        t = fm.get_tree(ctx, 1)
+        parents = np.flatnonzero(t["n_children"])
+        first = t["child_start"][parents]
+        kids = np.concatenate([np.arange(c, c + k) for c, k in zip(first, t["n_children"][parents])])
+        at = np.concatenate([[0], np.cumsum(t["n_children"][parents])[:-1]])
+        rep = np.repeat(np.arange(len(parents)), t["n_children"][parents])
+        for c, w, r in (("target_center", "target_box", "target_radius"), ("source_center", "source_box", "source_radius")):
+            lo = np.minimum.reduceat(np.minimum(t[c][kids], t[c][kids] - t[w][kids]), at)
+            hi = np.maximum.reduceat(np.maximum(t[c][kids], t[c][kids] + t[w][kids]), at)
+            cen = (lo + hi) * 0.5
+            d = t[c][kids] - cen[rep]
+            rad = np.sqrt(d[:, 0] * d[:, 0] + d[:, 1] * d[:, 1] + d[:, 2] * d[:, 2]) + t[r][kids]
+            np.testing.assert_array_equal(t[c][parents], cen)
+            np.testing.assert_array_equal(t[w][parents], hi - cen)
+            np.testing.assert_array_equal(t[r][parents], np.maximum.reduceat(rad, at))
+    ctx.close()
+
+
 def test_traversals_of_changing_size():
     """One context, systems whose traversals outgrow what the previous build's let expect, and back."""
     ctx = fm.Context(0)
