@@ -417,12 +417,12 @@ DevTree view_tree(const DevTree& S, const SysView& v) {
   return t;
 }
 
-// host_out: copy the target buffer there before the call's one wait at its end
+// copy_out: copy the target buffer there (copy_kind) before the call's one wait at its end
 // is_estimate: the influence estimate's sub-solve, whose out16 receives one value per body
 // (get_influence: the scalar potential when influence_potential, else |gradient|)
 void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, double* out16, fmm_result* res,
              bool is_estimate, cudaStream_t st, Scratch& sc, DevBuf<int>& stats, bool influence_potential = false,
-             double* host_out = nullptr) {
+             double* copy_out = nullptr, cudaMemcpyKind copy_kind = cudaMemcpyDeviceToHost) {
   const int p = o.expansion_order;
   const bool multi = in.n_sys > 1;
   // lamb_helmholtz = has_vector_potential(source_systems) (src/fmm.jl:927)
@@ -601,8 +601,7 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
                                                     split ? far13 : nullptr);
   FMM_CUDA_TRY(cudaGetLastError());
   mark(7);
-  if (host_out)
-    FMM_CUDA_TRY(cudaMemcpyAsync(host_out, out16, 16 * T.n_bodies * sizeof(double), cudaMemcpyDeviceToHost, st));
+  if (copy_out) FMM_CUDA_TRY(cudaMemcpyAsync(copy_out, out16, 16 * T.n_bodies * sizeof(double), copy_kind, st));
   if (res) {
     int h[6] = {0, 0, 0, 0, 0, 0};
     FMM_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -676,6 +675,17 @@ const double* stage(fmm_ctx* c, DevBuf<double>& buf, const double* ptr, size_t n
   buf.grow(n_doubles);
   FMM_CUDA_TRY(cudaMemcpyAsync(buf.ptr, ptr, n_doubles * sizeof(double), cudaMemcpyHostToDevice, c->stream));
   return buf.ptr;
+}
+
+// p is memory of this GPU (not managed, not another GPU's, not mapped host memory), which kernels
+// may write wherever a copy may
+bool on_device(const void* p, int device) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return a.type == cudaMemoryTypeDevice && a.device == device;
 }
 
 size_t tree_bytes(const DevTree& t) {
@@ -917,12 +927,14 @@ int fmm_solve(fmm_ctx* c, const fmm_target_system* target, const fmm_source_syst
       in.tpos = stage(c, c->stage_t, target->positions, (size_t)target->stride * target->n_bodies, target->memory);
       in.t_stride = target->stride;
     }
-    // the target buffer (rows 1..3 = positions, 4..16 = phi, gradient, hessian): device memory is
-    // written by the solve's last kernel, which runs after everything that reads the inputs
-    const bool on_device = target->memory == FMM_MEMORY_DEVICE;
-    if (!on_device) c->out16.grow(16 * (size_t)in.n_t);
-    run_fmm(c, c->main, in, *opt, on_device ? target->out : c->out16.ptr, result, false, c->stream, c->sc, c->stats,
-            false, on_device ? nullptr : target->out);
+    // the target buffer (rows 1..3 = positions, 4..16 = phi, gradient, hessian): memory of this GPU is
+    // written by the solve's last kernel, which runs after everything that reads the inputs; other
+    // memory (another GPU's needs no peer access) by a copy
+    const bool direct = target->memory == FMM_MEMORY_DEVICE && on_device(target->out, c->device);
+    if (!direct) c->out16.grow(16 * (size_t)in.n_t);
+    run_fmm(c, c->main, in, *opt, direct ? target->out : c->out16.ptr, result, false, c->stream, c->sc, c->stats,
+            false, direct ? nullptr : target->out,
+            target->memory == FMM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost);
     if (!result) FMM_CUDA_TRY(cudaStreamSynchronize(c->stream));  // (with a result the solve has waited for it)
     c->have_solve = true;
     c->last_p = opt->expansion_order;

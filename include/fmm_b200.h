@@ -94,7 +94,9 @@ typedef struct {
   int64_t stride;          /* >= 3 (use data_per_body to read a source buffer)     */
   double* out;             /* 16 * n_bodies, body-major: rows 1..3 receive the
                               positions, rows 4..16 phi, gradient, hessian          */
-  int memory;              /* fmm_memory of `positions` and `out`                  */
+  int memory;              /* fmm_memory of `positions` and `out`; DEVICE inputs are read by
+                              kernels of the context's GPU, `out` may also be managed
+                              memory or another GPU's                               */
 } fmm_target_system;
 
 /* Keyword arguments of fmm! (src/fmm.jl:862-923). */
