@@ -104,7 +104,7 @@ __device__ __forceinline__ int chan_row(int a) {
 // are cut after e^2, below the rounding of a double.  r^2 = 0 gives y = 0 and all products
 // zero, which skips the pair as the reference does.  Outside the range where y^3 and the
 // products are normal numbers the sums come out non-finite or the caller must not get here
-// (kFarHi): such batches take the general arithmetic (self_batch_f64_*).
+// (kFarHi, tiny_strength): such batches take the general arithmetic (self_batch_f64_*).
 struct InvR {
   double u, e, r3;  // y^2, 1 - r^2 y^2, q r^-3 (q the factor given)
 };
@@ -126,6 +126,10 @@ __device__ __forceinline__ InvR inv_r3(double r2, double q) {
 // arithmetic: r^-5 and the products with it stay normal numbers below
 constexpr int kFarHi = (1023 + 160) << 20;
 __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+// so do, where the potential is asked for, strengths below 2^-536 (not zero): the potential is
+// (q r^-3) r^2, r below 2^162, and q r^-3 would be subnormal where q / r is not
+constexpr int kTinyHi = (1023 - 536) << 20;
+__device__ __forceinline__ bool tiny_strength(double q) { return hi_abs(q) < kTinyHi && q != 0.0; }
 
 // one source body on one target, Laplace, 17 FP64 operations: phi = (q / r^3) r^2
 template <bool PS>
@@ -666,6 +670,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
             const double4 q = sstr[body];
             far = max(far, max(hi_abs(p.x), max(hi_abs(p.y), hi_abs(p.z))));
             if constexpr (KIND == FMM_POINT_SOURCE) {
+              if (PS && tiny_strength(q.x)) far = kFarHi;
               reinterpret_cast<double4*>(B)[idx] = make_double4(p.x, p.y, p.z, q.x);
             } else {
               double2* Bd = reinterpret_cast<double2*>(B) + 3 * idx;
@@ -954,6 +959,7 @@ __global__ void __launch_bounds__(kP2PThreads) k_direct(const double4* __restric
         const double4 p = spos[j];
         const double4 q = sstr[j];
         far = max(far, max(hi_abs(p.x), max(hi_abs(p.y), hi_abs(p.z))));
+        if (SOURCE && PS && tiny_strength(q.x)) far = kFarHi;
         float4* F = reinterpret_cast<float4*>(sh) + (SOURCE ? 2 : 3) * threadIdx.x;
         double2* D = reinterpret_cast<double2*>(F);
         if (MIXED) {

@@ -2,6 +2,8 @@
 coincident bodies, leaf sizes around the lane tiles.  The reference is the plain all-pairs sum in
 extended precision; the bound is the rounding of a sum of n terms of a few ulps each, relative to
 the sum of the terms' magnitudes."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -85,6 +87,29 @@ def test_f64_overflowing_gradient_keeps_the_potential(ctx):
     v, m = sums(b[:, :3], b, False)[0]
     assert np.all(abs(out[:, 3] - v) <= 4 * (80 + 16) * EPS * m)
     assert not np.all(np.isfinite(out[:, 4:7]))
+
+
+@pytest.mark.parametrize("scale,strength", [(1e40, 1e-200), (1e3, 1e-300), (1.0, 1e-307), (1e40, 1e-160)])
+@pytest.mark.parametrize("mix", [False, True])
+def test_f64_potential_of_tiny_strengths(ctx, scale, strength, mix):
+    """q / r is a normal number where q / r^3 is not: the potential keeps all its bits (mix: beside
+    bodies of ordinary strength and of none)."""
+    b = bodies(150, 1, scale, 7)
+    b[:, 4] = (1 + abs(b[:, 4])) * strength
+    if mix:
+        b[::7, 4] = 0.0
+        b[3::50, 4] *= 1e20
+    v, m = sums(b[:, :3], b, False)[0]
+    tol = 4 * (150 + 16) * EPS * m
+    opt = fm.make_options(expansion_order=3, leaf_size_source=20, scalar_potential=True, farfield=False,
+                          multipole_acceptance=1e-9)
+    out, _ = fm.solve_buffers(b, 1, opt, ctx=ctx)
+    assert np.all(abs(out[:, 3] - v) <= tol + 2.0 ** -1073)
+    out = np.zeros((150, 16))
+    src = L.SourceSystem(1, 150, 5, b.ctypes.data, L.FMM_MEMORY_HOST)
+    tgt = L.TargetSystem(150, None, 0, out.ctypes.data, L.FMM_MEMORY_HOST)
+    ctx.check(L.lib().fmm_direct(ctx.handle, C.byref(tgt), C.byref(src), 1, 1, 0, L.FMM_PRECISION_F64))
+    assert np.all(abs(out[:, 3] - v) <= tol + 2.0 ** -1073)
 
 
 @pytest.mark.parametrize("kind,hess", [(1, False), (3, False), (3, True)])
