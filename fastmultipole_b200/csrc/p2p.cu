@@ -144,20 +144,29 @@ __device__ __forceinline__ void source_pair_f64(double tx, double ty, double tz,
   a[3] = fma(dz, q3, a[3]);
 }
 
-// One lane's slice of a packed batch on its two targets.  GUARD skips pairs with
-// r^2 = 0 (coincident bodies); without it such a pair makes the sums non-finite.
-template <bool GUARD, bool PS>
+// How a packed batch treats pairs without r^2 > 0.  kUnguarded: they make the sums non-finite.
+// kCoincident: 1 / r = 0, so that coincident bodies add nothing.  kSkip: they are left out whatever
+// their offsets and strengths (NaN coordinates, infinite strengths) are.
+enum : int { kUnguarded = 0, kCoincident, kSkip };
+__device__ __forceinline__ float2 keep(float2 r2, float2 v) {
+  return make_float2(r2.x > 0.f ? v.x : 0.f, r2.y > 0.f ? v.y : 0.f);
+}
+
+// One lane's slice of a packed batch on its two targets.
+template <int GUARD, bool PS>
 __device__ __forceinline__ void packed_batch(const float4* __restrict__ B4, int j0, int nb, int SS, float2 tx2,
                                              float2 ty2, float2 tz2, float2& ph, float2& gx, float2& gy, float2& gz) {
 #pragma unroll 4
   for (int j = j0; j < nb; j += SS) {
     const float4 u = B4[2 * j], v = B4[2 * j + 1];
-    const float2 dx = __fadd2_rn(tx2, make_float2(u.x, u.y));
-    const float2 dy = __fadd2_rn(ty2, make_float2(u.z, u.w));
-    const float2 dz = __fadd2_rn(tz2, make_float2(v.x, v.y));
+    float2 dx = __fadd2_rn(tx2, make_float2(u.x, u.y));
+    float2 dy = __fadd2_rn(ty2, make_float2(u.z, u.w));
+    float2 dz = __fadd2_rn(tz2, make_float2(v.x, v.y));
+    float2 q = make_float2(v.z, v.w);
     float2 r2 = __fmul2_rn(dx, dx);
     r2 = __ffma2_rn(dy, dy, r2);
     r2 = __ffma2_rn(dz, dz, r2);
+    if (GUARD == kSkip) dx = keep(r2, dx), dy = keep(r2, dy), dz = keep(r2, dz), q = keep(r2, q);
     float2 ri;
     if (GUARD) {
       ri.x = r2.x > 0.f ? rsqrt_ftz(r2.x) : 0.f;
@@ -166,7 +175,7 @@ __device__ __forceinline__ void packed_batch(const float4* __restrict__ B4, int 
       ri = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
     }
     // q / r and q / r^3 = (q / r) (1 / r^2): the two products after the rsqrt are independent
-    const float2 qr = __fmul2_rn(make_float2(v.z, v.w), ri);
+    const float2 qr = __fmul2_rn(q, ri);
     const float2 ri2 = __fmul2_rn(ri, ri);
     if (PS) ph = __fadd2_rn(ph, qr);
     const float2 q3 = __fmul2_rn(qr, ri2);
@@ -267,9 +276,8 @@ __device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y
 // du_j/dx_i = eps_jki G_k / r^3 - 3 d_i (G x d)_j / r^5 is summed as two parts, Q_ij =
 // sum d_i (G x d)_j / r^5 and E_k = sum G_k / r^3, combined once per batch (r^2 / r^5 =
 // 1 / r^3, so the six eps terms need three sums; the trace of Q vanishes, so Q_zz is not
-// summed).  GUARD skips pairs with r^2 = 0
-// (coincident bodies); without it such a pair makes the sums non-finite.
-template <bool GUARD, bool GS, bool HS, int NA>
+// summed).
+template <int GUARD, bool GS, bool HS, int NA>
 __device__ __forceinline__ void packed_vortex_batch(const float4* __restrict__ B4, int j0, int nb, int SS,
                                                     float2 tx2, float2 ty2, float2 tz2, float2 (&acc)[NA]) {
   constexpr int h = GS ? 3 : 0;
@@ -281,13 +289,17 @@ __device__ __forceinline__ void packed_vortex_batch(const float4* __restrict__ B
 #pragma unroll 2
   for (int j = j0; j < nb; j += SS) {
     const float4 p = B4[3 * j], v = B4[3 * j + 1], w = B4[3 * j + 2];
-    const float2 dx = __fadd2_rn(tx2, make_float2(p.x, p.y));
-    const float2 dy = __fadd2_rn(ty2, make_float2(p.z, p.w));
-    const float2 dz = __fadd2_rn(tz2, make_float2(v.x, v.y));
-    const float2 g0 = make_float2(v.z, v.w), g1 = make_float2(w.x, w.y), g2 = make_float2(w.z, w.w);
+    float2 dx = __fadd2_rn(tx2, make_float2(p.x, p.y));
+    float2 dy = __fadd2_rn(ty2, make_float2(p.z, p.w));
+    float2 dz = __fadd2_rn(tz2, make_float2(v.x, v.y));
+    float2 g0 = make_float2(v.z, v.w), g1 = make_float2(w.x, w.y), g2 = make_float2(w.z, w.w);
     float2 r2 = __fmul2_rn(dx, dx);
     r2 = __ffma2_rn(dy, dy, r2);
     r2 = __ffma2_rn(dz, dz, r2);
+    if (GUARD == kSkip) {
+      dx = keep(r2, dx), dy = keep(r2, dy), dz = keep(r2, dz);
+      g0 = keep(r2, g0), g1 = keep(r2, g1), g2 = keep(r2, g2);
+    }
     float2 ri;
     if (GUARD) {
       ri.x = r2.x > 0.f ? rsqrt_ftz(r2.x) : 0.f;
@@ -696,12 +708,12 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
             self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
             self_batch_f64_source<PS, NA>(reinterpret_cast<const double4*>(B), slice, nb, SS, txd, tyd, tzd, tot);
           } else if (self_batch) {
-            packed_batch<true, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+            packed_batch<kCoincident, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
           } else {
-            packed_batch<false, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+            packed_batch<kUnguarded, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
             if (!isfinite(ph.x + ph.y + gx.x + gx.y + gy.x + gy.y + gz.x + gz.y)) {
               ph = gx = gy = gz = make_float2(0.f, 0.f);
-              packed_batch<true, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
+              packed_batch<kCoincident, PS>(B4, slice, nb, SS, tx2, ty2, tz2, ph, gx, gy, gz);
             }
           }
           part[0][0] += (R)ph.x;
@@ -726,13 +738,13 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
             self_targets_f64(tpos, ts + tile, nt, ti, TS, ox, oy, oz, txd, tyd, tzd);
             self_batch_f64_vortex<GS, HS, NA>(reinterpret_cast<const double2*>(B), slice, nb, SS, txd, tyd, tzd, tot);
           } else if (self_batch) {
-            packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+            packed_vortex_batch<kCoincident, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
           } else {
-            packed_vortex_batch<false, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+            packed_vortex_batch<kUnguarded, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
             float sum = 0.f;
 #pragma unroll
             for (int a = 0; a < NA; ++a) sum += acc[a].x + acc[a].y;
-            if (!isfinite(sum)) packed_vortex_batch<true, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
+            if (!isfinite(sum)) packed_vortex_batch<kCoincident, GS, HS, NA>(B4, slice, nb, SS, tx2, ty2, tz2, acc);
           }
 #pragma unroll
           for (int a = 0; a < NA; ++a) {
@@ -982,21 +994,21 @@ __global__ void __launch_bounds__(kP2PThreads) k_direct(const double4* __restric
           const float2 tx2 = make_float2(tx[2 * h], tx[2 * h + 1]), ty2 = make_float2(ty[2 * h], ty[2 * h + 1]);
           const float2 tz2 = make_float2(tz[2 * h], tz[2 * h + 1]);
           float2 a[NA];
-          // unguarded; a chunk with a coincident body again with the r^2 > 0 guard
+          // unguarded; a chunk whose sums are not finite again without the pairs that lack r^2 > 0
 #pragma unroll 1
           for (int guard = 0; guard < 2; ++guard) {
 #pragma unroll
             for (int q = 0; q < NA; ++q) a[q] = make_float2(0.f, 0.f);
             if constexpr (SOURCE) {
               if (guard)
-                packed_batch<true, PS>(B4, 0, m, 1, tx2, ty2, tz2, a[0], a[1 % NA], a[2 % NA], a[3 % NA]);
+                packed_batch<kSkip, PS>(B4, 0, m, 1, tx2, ty2, tz2, a[0], a[1 % NA], a[2 % NA], a[3 % NA]);
               else
-                packed_batch<false, PS>(B4, 0, m, 1, tx2, ty2, tz2, a[0], a[1 % NA], a[2 % NA], a[3 % NA]);
+                packed_batch<kUnguarded, PS>(B4, 0, m, 1, tx2, ty2, tz2, a[0], a[1 % NA], a[2 % NA], a[3 % NA]);
             } else {
               if (guard)
-                packed_vortex_batch<true, GS, HS, NA>(B4, 0, m, 1, tx2, ty2, tz2, a);
+                packed_vortex_batch<kSkip, GS, HS, NA>(B4, 0, m, 1, tx2, ty2, tz2, a);
               else
-                packed_vortex_batch<false, GS, HS, NA>(B4, 0, m, 1, tx2, ty2, tz2, a);
+                packed_vortex_batch<kUnguarded, GS, HS, NA>(B4, 0, m, 1, tx2, ty2, tz2, a);
             }
             float sum = 0.f;
 #pragma unroll

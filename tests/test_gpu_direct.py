@@ -49,3 +49,30 @@ def test_blocks_and_splits(ctx, kind, hess, nt, ns, mixed):
             tol = tol + (rel if got.ndim == 1 else rel[:, None]) * ref[1]
         assert np.all(np.isfinite(got))
         assert np.all(abs(got - ref[0]) <= tol)
+
+
+@pytest.mark.parametrize("kind,hess", [(1, False), (3, False), (3, True)])
+@pytest.mark.parametrize("mixed", [False, True])
+def test_pairs_without_a_distance_are_left_out(ctx, kind, hess, mixed):
+    """A pair counts if r^2 > 0: bodies with a NaN coordinate, and the own infinite or NaN strength of
+    a coincident body, add nothing (to the other targets they do)."""
+    prec = L.FMM_PRECISION_MIXED if mixed else L.FMM_PRECISION_F64
+    b = bodies(700, kind, 1.0, 23)
+    pos = bodies(300, 1, 1.0, 24)[:, :3]
+    rows = slice(3, 16) if hess else slice(3, 7)
+    bad = b.copy()
+    bad[[5, 129, 699], [0, 1, 2]] = np.nan
+    b[[5, 129, 699], 4:] = 0.0
+    got, ref = direct(ctx, bad, kind, pos, hess, prec), direct(ctx, b, kind, pos, hess, prec)
+    tol = 1e-4 if mixed else 1e-12  # another path sums the same terms
+    assert np.all(np.isfinite(got[:, rows]))
+    np.testing.assert_allclose(got[:, rows], ref[:, rows], rtol=0, atol=tol * np.abs(ref[:, rows]).max())
+    # a target without a position: no pair at all
+    pos[17, 1] = np.nan
+    got = direct(ctx, bad, kind, pos, hess, prec)
+    assert np.all(got[17, rows] == 0) and np.all(np.isfinite(np.delete(got, 17, 0)[:, rows]))
+    # a body of infinite strength on a target: only that target leaves it out
+    pos[40] = bad[300, :3]
+    bad[300, 4:] = np.inf
+    got = direct(ctx, bad, kind, pos, hess, prec)
+    assert np.all(np.isfinite(got[40, rows])) and not np.any(np.all(np.isfinite(np.delete(got, [17, 40], 0)[:, 4:7]), 1))
