@@ -48,9 +48,12 @@ struct Workspace {
 // it has its own, the far field: the single addition the L2P makes when it accumulates into the
 // near-field rows itself) after the position.  Bound by the traffic: 1e6 bodies 146 us with a thread
 // per body, whose rows lay 104 and 128 bytes apart.
+// undefined (may be null): a centre of the tree, when the downward pass of the requested rows (mask) was
+// left out because nothing was translated: a position that is not a number gives NaN there too.
 __global__ void k_unsort(const double* __restrict__ acc13, const int* __restrict__ sort_index,
                          const double4* __restrict__ pos, int64_t n, double* __restrict__ out16,
-                         const double* __restrict__ far = nullptr) {
+                         const double* __restrict__ far = nullptr, const double* __restrict__ undefined = nullptr,
+                         unsigned mask = 0) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 16 * n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e >> 4;
     const int r = (int)(e & 15);
@@ -60,6 +63,10 @@ __global__ void k_unsort(const double* __restrict__ acc13, const int* __restrict
     } else {
       v = acc13[13 * i + r - 3];
       if (far) v += far[13 * i + r - 3];
+      if (undefined && ((mask >> r) & 1u)) {
+        const double4 p = pos[i];
+        v += 0.0 * (p.x - undefined[0]) + 0.0 * (p.y - undefined[1]) + 0.0 * (p.z - undefined[2]);
+      }
     }
     out16[16 * (int64_t)(sort_index ? sort_index[i] : i) + r] = v;
   }
@@ -581,8 +588,10 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
                c->tables, o.precision, fs);
   markf(3);
   if (!split) mark(6);
-  // no translation into the locals: they are zero, and so is what the downward pass would add
-  if (o.downward_pass && o.horizontal_pass && W.lists.n_m2l > 0) {
+  // no translation into the locals: they are zero, and so is what the downward pass would add to every
+  // target that has a position
+  const bool translated = o.horizontal_pass && W.lists.n_m2l > 0;
+  if (o.downward_pass && translated) {
     launch_l2l(T, p, lh, fs);
     launch_l2p(T, p, lh, ps, gs, hs, far13, fs);
   }
@@ -597,8 +606,10 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
     k_unsort_gradnorm<<<grid_for(T.n_bodies), 256, 0, st>>>(W.acc13.ptr, T.sort_index.ptr, T.n_bodies, out16,
                                                              influence_potential ? 1 : 0);
   else
-    k_unsort<<<grid_for(16 * T.n_bodies), 256, 0, st>>>(W.acc13.ptr, T.sort_index.ptr, T.pos.ptr, T.n_bodies, out16,
-                                                    split ? far13 : nullptr);
+    k_unsort<<<grid_for(16 * T.n_bodies), 256, 0, st>>>(
+        W.acc13.ptr, T.sort_index.ptr, T.pos.ptr, T.n_bodies, out16, split ? far13 : nullptr,
+        o.downward_pass && !translated ? T.tcenter.ptr : nullptr,
+        (ps ? 0x8u : 0u) | (gs ? 0x70u : 0u) | (hs ? 0xff80u : 0u));
   FMM_CUDA_TRY(cudaGetLastError());
   mark(7);
   if (copy_out) FMM_CUDA_TRY(cudaMemcpyAsync(copy_out, out16, 16 * T.n_bodies * sizeof(double), copy_kind, st));
