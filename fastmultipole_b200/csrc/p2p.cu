@@ -1227,7 +1227,8 @@ __global__ void k_p2p_sum(const int4* __restrict__ items, const int* __restrict_
     if (KIND == FMM_POINT_SOURCE && ch == 0 && !PS) continue;
     double v = 0.0;
     for (int c = 0; c < b.y; ++c) v += sums[b.x + c * b.z * NA + e];
-    acc13[13 * (int64_t)(first + i) + chan_row<KIND, GS>(ch)] += v * kOneOver4Pi;  // the tile's only writer
+    // atomic: under SelfTuning the rows of nested branches add to the same targets
+    atomicAdd(acc13 + 13 * (int64_t)(first + i) + chan_row<KIND, GS>(ch), v * kOneOver4Pi);
   }
 }
 
@@ -1258,9 +1259,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   constexpr int NA = n_chan<KIND, GS, HS>();
   const double est_pairs = (double)L.n_direct * ((double)stt.n_bodies / std::max<int64_t>(1, stt.n_leaves)) *
                            ((double)tt.n_bodies / std::max<int64_t>(1, tt.n_leaves));
-  // rows that are not leaves (SelfTuning) can be nested, their targets' other rows adding at the
-  // same time: they keep whole rows, added with atomics
-  if (est_pairs > kItemPairs && rows <= kItemRowsPerSM * n_sm && L.rule_method != FMM_LIST_SELF_TUNING) {
+  if (est_pairs > kItemPairs && rows <= kItemRowsPerSM * n_sm) {
     if (smem > 48 * 1024)
       FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1269,8 +1268,10 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
                                                                kWarps * 32, smem));
     const int goal = kItemWaves * std::max(1, per_sm) * n_sm;
     // a tile per 64 targets begun (up to three with sub-tiles), a share more per 1 / goal of the work;
-    // at most twice the goal of them in tiles that are cut
-    const int64_t most = 3 * (int64_t)rows + tt.n_bodies / (32 * kTPT) + goal + 1;
+    // at most twice the goal of them in tiles that are cut.  The targets of rows that are not leaves
+    // (SelfTuning) can be those of other rows too, one of them per level
+    const int64_t nest = L.rule_method == FMM_LIST_SELF_TUNING ? tt.n_levels : 1;
+    const int64_t most = 3 * (int64_t)rows + nest * tt.n_bodies / (32 * kTPT) + goal + 1;
     const int64_t sums = (int64_t)2 * goal * 32 * kTPT * NA;
     L.p2p_items.grow(2 * (size_t)most);
     L.p2p_meta.grow((size_t)rows + 1);

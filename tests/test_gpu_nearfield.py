@@ -134,3 +134,28 @@ def test_items_cover_every_pair(ctx, kind, hess, leaf, ls_t):
         # few thousand bodies in a unit cube (about 1e-2), order 5
         mixed = res["mixed"][:, cols].reshape(np.shape(ref[0]))
         assert np.linalg.norm(mixed - got) <= 1e-4 * np.linalg.norm(got)
+
+
+@pytest.mark.parametrize("kind,hess", [(1, False), (3, True)])
+@pytest.mark.parametrize("leaf,ls_t", [(16, 3), (60, 47), (300, 150)])
+def test_items_of_nested_rows(ctx, kind, hess, leaf, ls_t):
+    """SelfTuning: target branches that are not leaves have rows too, of several tiles, and share their
+    targets with the rows of their descendants."""
+    b = bodies(8111, kind, 1.0, 35)
+    pos = np.concatenate([bodies(3000, kind, 0.4, 36)[:, :3], bodies(201, kind, 3.0, 37)[:, :3]])
+    some = np.arange(0, len(pos), 19)
+    ref = sums(pos[some], b, hess)
+    for prec, eps in (("f64", None), ("mixed", 1e-4)):
+        opt = fm.make_options(expansion_order=3, leaf_size_source=leaf, leaf_size_target=ls_t, scalar_potential=kind == 1,
+                              hessian=hess, farfield=False, multipole_acceptance=1e-9, precision=prec,
+                              interaction_list_method=fm.SelfTuning())
+        out, res = fm.solve_buffers(b, kind, opt, pos, ctx=ctx)
+        assert res.n_p2p_pairs == len(b) * len(pos)
+        for cols, r in zip((slice(3, 4), slice(4, 7), slice(7, 16)), ref):
+            if r is None:
+                continue
+            got = out[some, cols].reshape(np.shape(r[0]))
+            if eps is None:  # (rows of a branch and its ancestors: a few more additions)
+                assert np.all(abs(got - r[0]) <= 4 * (len(b) + 32) * EPS * r[1])
+            else:
+                assert np.linalg.norm((got - r[0]).astype(float)) <= eps * np.linalg.norm(r[0].astype(float))
