@@ -527,7 +527,6 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   }
   stats.grow(8);
   FMM_CUDA_TRY(cudaMemsetAsync(stats.ptr, 0, 8 * sizeof(int), st));
-  if (res) count_p2p_pairs(T, S, W.lists, reinterpret_cast<unsigned long long*>(stats.ptr + 4), st);
   // trees, lists and zeroed accumulators are ready: fork the rest of the far field and the estimate
   if (estimate || split) FMM_CUDA_TRY(cudaEventRecord(fork_event(c), st));
   if (split) FMM_CUDA_TRY(cudaStreamWaitEvent(fs, fork_event(c), 0));
@@ -614,12 +613,11 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   mark(7);
   if (copy_out) FMM_CUDA_TRY(cudaMemcpyAsync(copy_out, out16, 16 * T.n_bodies * sizeof(double), copy_kind, st));
   if (res) {
-    int h[6] = {0, 0, 0, 0, 0, 0};
-    FMM_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 6 * sizeof(int), cudaMemcpyDeviceToHost, st));
+    int h[4] = {0, 0, 0, 0};
+    FMM_CUDA_TRY(cudaMemcpyAsync(h, stats.ptr, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
     FMM_CUDA_TRY(cudaStreamSynchronize(st));
-    unsigned long long fl, pairs;
+    unsigned long long fl;
     std::memcpy(&fl, &h[2], 8);
-    std::memcpy(&pairs, &h[4], 8);
     res->p_max = h[0] + (h[1] ? 1 : 0);
     res->error_success = h[1] ? 0 : 1;
     res->n_target_branches = T.n_branches;
@@ -629,7 +627,7 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
     res->n_m2l = W.lists.n_m2l;
     res->n_direct = W.lists.n_direct;
     res->m2l_flops = (int64_t)fl;
-    res->n_p2p_pairs = (int64_t)pairs;
+    res->n_p2p_pairs = W.lists.n_pairs;
     res->n_kernel_launches = g_launches - launches0;
     if (timing) {
       float ms[3], tot = 0.0f, fup = 0.0f, fh = 0.0f, fd = 0.0f;

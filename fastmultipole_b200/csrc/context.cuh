@@ -38,6 +38,7 @@ struct DevTree {
 // per-target CSR used by the target-owned kernels.
 struct DevLists {
   int64_t n_m2l = 0, n_direct = 0;
+  int64_t n_pairs = 0, n_source_bodies = 0;  // body pairs of the direct list; bodies of its source tree
   DevBuf<int> m2l_t, m2l_s, dir_t, dir_s;
   int64_t n_m2l_targets = 0, n_dir_targets = 0;
   DevBuf<int> m2l_tgt, m2l_off;   // unique targets, offsets (n+1)
@@ -108,9 +109,6 @@ void export_lists_reference_order(const DevLists& L, const DevTree& stt, Scratch
 // exact_self: on the mixed path, evaluate the batch holding the target's own leaf in FP64
 void launch_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, int kind, bool ps,
                 bool gs, bool hs, int precision, cudaStream_t st, bool exact_self = true);
-// sum over the direct list of n_target * n_source (atomically added to *out)
-void count_p2p_pairs(const DevTree& tt, const DevTree& stt, const DevLists& L, unsigned long long* out,
-                     cudaStream_t st);
 // All pairs (direct!): targets in pos order, sources; accumulates into acc13.
 // part (may be null): buffer for the sums of source splits; without it nothing is allocated and
 // every target block goes through all the sources

@@ -20,6 +20,7 @@
 // Both lists go through each stage in one launch, and the host synchronises once per build:
 // after the row compaction (totals, capacity check, row counts).
 #include <climits>
+#include <cstring>
 
 #include <cub/cub.cuh>
 #include <cub/block/block_merge_sort.cuh>
@@ -123,7 +124,8 @@ __global__ void k_pack_nodes(NodeIn T, NodeIn S, int2* front, int* ctr) {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxSteps = 64;  // frontier counters; a traversal takes levels_t + levels_s - 1 steps
-enum : int { C_DIR = kMaxSteps, C_M2L, C_FLAG, C_ROWS_DIR, C_ROWS_M2L = C_ROWS_DIR + 8, C_N = 128 };
+enum : int { C_DIR = kMaxSteps, C_M2L, C_FLAG, C_ROWS_DIR, C_ROWS_M2L = C_ROWS_DIR + 8, C_PAIRS = C_ROWS_M2L + 9, C_N = 128 };
+static_assert(C_PAIRS % 2 == 0, "the body pairs of the direct list are a 64-bit counter");
 constexpr int kStepThreads = 128;
 constexpr int kStepMaxBlocks = 148 * 16;
 
@@ -161,6 +163,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
   const int n = min(ctr[k], cap_f);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   bool bad = false;
+  unsigned long long pairs = 0;  // body pairs of this thread's direct pairs
   // a frontier that the launch's threads cover takes one pair per thread
   const int items = n > (int)gridDim.x * kStepThreads ? kStepItems : 1, chunk = items * kStepThreads;
   for (int c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
@@ -204,6 +207,7 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
 #pragma unroll
     for (int r = 0; r < kStepItems; ++r) {
       if (a[r] == A_DIRECT) {
+        pairs += (unsigned long long)T.info[p[r].x].z * (unsigned long long)S.info[p[r].y].z;
         if (od < cap_d)
           rdir[od] = p[r];
         else
@@ -233,6 +237,9 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
     __syncthreads();  // wsum / bbase are rewritten by the next chunk
   }
   if (bad) atomicOr(ctr + C_FLAG, 1);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
+  if (lane == 0 && pairs) atomicAdd(reinterpret_cast<unsigned long long*>(ctr + C_PAIRS), pairs);
 }
 
 // per target: (count << 32) | (count > 0), so that one exclusive scan gives both the
@@ -615,6 +622,8 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
   const int rows[2] = {h_d[0], h_m[0]};
   L.n_direct = n_dir;
   L.n_m2l = n_m2l;
+  std::memcpy(&L.n_pairs, h.data() + C_PAIRS, sizeof(L.n_pairs));
+  L.n_source_bodies = stt.n_bodies;
   L.n_dir_targets = rows[0];
   L.n_m2l_targets = rows[1];
   L.rule_method = method;

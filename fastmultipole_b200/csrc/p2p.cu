@@ -53,7 +53,8 @@ constexpr int kWarps = 4;
 // field 273 -> 113 us and 50 us to cut and to add; 300k vortex ring FP64: 28.2 -> 25.5 ms (whole
 // solves).  More rows than that fill the GPU by themselves (1e6 bodies: 62.0 ms either way).
 constexpr int kItemRowsPerSM = 64, kItemWaves = 4, kItemSources = 256;
-constexpr double kItemPairs = 4e6;  // below this many pairs the extra launches cost more than they save
+constexpr double kItemPairs = 4e6;  // below this many pairs the extra launches cost more than they save,
+constexpr double kItemRowPairs = 1e5;  // but for rows that would keep one CTA busy for some 0.1 ms each
 constexpr int kTPT = 2;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -1108,16 +1109,22 @@ __global__ void k_direct_sum(const double* __restrict__ part, int n_split, int64
   }
 }
 
-// source bodies of every row, one warp each
-__global__ void k_p2p_row_sources(const int* __restrict__ off, int rows, const int* __restrict__ src_of,
+// source bodies of every row, one block each (eight loads of a thread in flight: the 32,000 leaves of
+// one row of probes took a warp 1 ms)
+__global__ void k_p2p_row_sources(const int* __restrict__ off, const int* __restrict__ src_of,
                                   const int* __restrict__ s_count, int* __restrict__ n_src) {
-  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (row >= rows) return;
+  __shared__ int sum;
+  if (threadIdx.x == 0) sum = 0;
+  __syncthreads();
   int v = 0;
-  for (int i = off[row] + lane; i < off[row + 1]; i += 32) v += s_count[src_of[i]];
+  const int e = off[blockIdx.x + 1];
+#pragma unroll 8
+  for (int i = off[blockIdx.x] + threadIdx.x; i < e; i += blockDim.x) v += s_count[src_of[i]];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(kAll, v, o);
-  if (lane == 0) n_src[row] = v;
+  if ((threadIdx.x & 31) == 0) atomicAdd(&sum, v);
+  __syncthreads();
+  if (threadIdx.x == 0) n_src[blockIdx.x] = sum;
 }
 
 // target slots that a tile of nt targets occupies (three: the FP64 kernels' choice of targets per lane)
@@ -1200,9 +1207,10 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       const int c = cut(nt);
       // (the bound on the items leaves room for every row's sums)
       const bool split = c > 1 && ex.y + c * nt * na <= max_sums;
+      const int q = nl / c, more = nl - q * c;  // leaves per share, shares with one more
       for (int j = 0; j < c; ++j) {
-        const int lo = split ? a + (int)((long long)nl * j / c) : a;
-        const int hi = split ? a + (int)((long long)nl * (j + 1) / c) : (j == 0 ? a + nl : a);
+        const int lo = split ? a + j * q + min(j, more) : a;
+        const int hi = split ? lo + q + (j < more) : (j == 0 ? a + nl : a);
         items[2 * (ex.x + j)] = make_int4(r, t, lo, hi);
         items[2 * (ex.x + j) + 1] = make_int4(split ? ex.y + j * nt * na : -1, split && j == 0 ? c : 0, nt, 0);
       }
@@ -1213,23 +1221,45 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
   if (threadIdx.x == 0) *n_items = run.x;
 }
 
-// the shares of every tile that was cut, added in order
+// the shares of every tile that was cut, added in order; those of a tile of few sums and many shares in
+// several interleaved groups (a thread per sum alone took 0.2 ms for the 592 shares of a row of probes)
+constexpr int kSumThreads = 128, kSumManyShares = 32;
 template <int KIND, bool PS, bool GS, int NA>
-__global__ void k_p2p_sum(const int4* __restrict__ items, const int* __restrict__ n_items,
-                          const double* __restrict__ sums, const int* __restrict__ tgt_list,
-                          const int* __restrict__ t_start, double* __restrict__ acc13) {
+__global__ void __launch_bounds__(kSumThreads) k_p2p_sum(const int4* __restrict__ items,
+                                                         const int* __restrict__ n_items,
+                                                         const double* __restrict__ sums,
+                                                         const int* __restrict__ tgt_list,
+                                                         const int* __restrict__ t_start, double* __restrict__ acc13) {
+  __shared__ double part[kSumThreads];
   if ((int)blockIdx.x >= *n_items) return;
   const int4 a = items[2 * blockIdx.x], b = items[2 * blockIdx.x + 1];
   if (b.y == 0) return;
-  const int first = t_start[tgt_list[a.x]] + a.y;
-  for (int e = threadIdx.x; e < b.z * NA; e += blockDim.x) {
-    const int i = e / NA, ch = e - i * NA;
-    if (KIND == FMM_POINT_SOURCE && ch == 0 && !PS) continue;
+  const int first = t_start[tgt_list[a.x]] + a.y, n = b.z * NA;
+  // sum e of the shares from c0 in steps of dc
+  auto add = [&](int e, int c0, int dc) {
     double v = 0.0;
-    for (int c = 0; c < b.y; ++c) v += sums[b.x + c * b.z * NA + e];
-    // atomic: under SelfTuning the rows of nested branches add to the same targets
+#pragma unroll 8
+    for (int c = c0; c < b.y; c += dc) v += sums[b.x + c * n + e];
+    return v;
+  };
+  // atomic: under SelfTuning the rows of nested branches add to the same targets
+  auto put = [&](int e, double v) {
+    const int i = e / NA, ch = e - i * NA;
+    if (KIND == FMM_POINT_SOURCE && ch == 0 && !PS) return;
     atomicAdd(acc13 + 13 * (int64_t)(first + i) + chan_row<KIND, GS>(ch), v * kOneOver4Pi);
+  };
+  const int groups = b.y >= kSumManyShares ? kSumThreads / n : 1;
+  if (groups > 1) {
+    const int g = threadIdx.x / n, e = threadIdx.x - g * n;
+    if (g < groups) part[threadIdx.x] = add(e, g, groups);
+    __syncthreads();
+    if (g != 0) return;
+    double v = part[e];
+    for (int q = 1; q < groups; ++q) v += part[q * n + e];
+    put(e, v);
+    return;
   }
+  for (int e = threadIdx.x; e < n; e += kSumThreads) put(e, add(e, 0, 1));
 }
 
 template <class R, int KIND, bool PS, bool GS, bool HS>
@@ -1257,9 +1287,9 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   FMM_CUDA_TRY(cudaGetDevice(&dev));
   FMM_CUDA_TRY(cudaDeviceGetAttribute(&n_sm, cudaDevAttrMultiProcessorCount, dev));
   constexpr int NA = n_chan<KIND, GS, HS>();
-  const double est_pairs = (double)L.n_direct * ((double)stt.n_bodies / std::max<int64_t>(1, stt.n_leaves)) *
-                           ((double)tt.n_bodies / std::max<int64_t>(1, tt.n_leaves));
-  if (est_pairs > kItemPairs && rows <= kItemRowsPerSM * n_sm) {
+  // body pairs (of a tuple's system: its part by the number of bodies)
+  const double pairs = (double)L.n_pairs * ((double)stt.n_bodies / (double)L.n_source_bodies);
+  if (rows <= kItemRowsPerSM * n_sm && (pairs > kItemPairs || pairs > kItemRowPairs * rows)) {
     if (smem > 48 * 1024)
       FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -1277,8 +1307,9 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     L.p2p_meta.grow((size_t)rows + 1);
     L.p2p_part.grow((size_t)sums);
     note_launch();
-    k_p2p_row_sources<<<(int)((rows * 32ll + 255) / 256), 256, 0, st>>>(L.dir_off.ptr, rows, L.dir_s.ptr,
-                                                                        stt.body_count.ptr, L.p2p_meta.ptr + 1);
+    const int64_t per_row = L.n_direct / rows;
+    k_p2p_row_sources<<<rows, per_row <= 64 ? 32 : per_row <= 1024 ? 128 : 1024, 0, st>>>(
+        L.dir_off.ptr, L.dir_s.ptr, stt.body_count.ptr, L.p2p_meta.ptr + 1);
     note_launch();
     k_p2p_plan<sub_tiles<R, KIND, true>() && max_targets_per_lane<R, KIND, HS>() == kTPT><<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
                                            goal, NA, (int)sums, max_targets_per_lane<R, KIND, HS>() == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
@@ -1288,7 +1319,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
         stt.body_start.ptr, stt.body_count.ptr, tt.pos.ptr, stt.pos.ptr, stt.str.ptr, acc13, L.p2p_items.ptr,
         L.p2p_meta.ptr, L.p2p_part.ptr, exact_self);
     note_launch();
-    k_p2p_sum<KIND, PS, GS, NA><<<(int)most, 128, 0, st>>>(L.p2p_items.ptr, L.p2p_meta.ptr, L.p2p_part.ptr,
+    k_p2p_sum<KIND, PS, GS, NA><<<(int)most, kSumThreads, 0, st>>>(L.p2p_items.ptr, L.p2p_meta.ptr, L.p2p_part.ptr,
                                                           L.dir_tgt.ptr, tt.body_start.ptr, acc13);
   } else {
     if (smem > 48 * 1024)
@@ -1394,26 +1425,7 @@ struct DirectLaunch {
   }
 };
 
-__global__ void k_pair_count(const int* __restrict__ dt, const int* __restrict__ ds, int64_t n,
-                             const int* __restrict__ tcount, const int* __restrict__ scount,
-                             unsigned long long* __restrict__ out) {
-  unsigned long long v = 0;
-  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x)
-    v += (unsigned long long)tcount[dt[k]] * (unsigned long long)scount[ds[k]];
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) atomicAdd(out, v);
-}
-
 }  // namespace
-
-void count_p2p_pairs(const DevTree& tt, const DevTree& stt, const DevLists& L, unsigned long long* out,
-                     cudaStream_t st) {
-  if (L.n_direct == 0) return;
-  int g = (int)std::min<int64_t>((L.n_direct + 255) / 256, 148 * 8);
-  note_launch();
-  k_pair_count<<<g, 256, 0, st>>>(L.dir_t.ptr, L.dir_s.ptr, L.n_direct, tt.body_count.ptr, stt.body_count.ptr, out);
-  FMM_CUDA_TRY(cudaGetLastError());
-}
 
 void launch_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, int kind, bool ps, bool gs,
                 bool hs, int precision, cudaStream_t st, bool exact_self) {
