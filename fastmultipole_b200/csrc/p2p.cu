@@ -45,16 +45,19 @@ __device__ __forceinline__ double rsq(double x) { return rsqrt(x); }
 // of small target leaves (at most 8 bodies on average) take one warp each instead of
 // a CTA, so that the per-row setup and the cross-warp sum do not dominate their work.
 constexpr int kWarps = 4;
-// Launches of up to kItemRowsPerSM rows per SM are cut into items of about equal work, some
-// kItemWaves for every CTA that the SMs hold at a time: one tile of a row's targets x a share of the
-// row's source leaves (at least kItemSources bodies), whose sums are added in order by k_p2p_sum.
+// Launches of up to kItemRowsPerSM rows per SM whose rows are long are cut into items of about equal
+// work, some kItemWaves for every CTA that the SMs hold at a time: one tile of a row's targets x a share
+// of the row's source leaves (at least kItemSources bodies), whose sums are added in order by k_p2p_sum.
 // With a CTA of 4 or 16 warps per row the few rows of large leaves (up to three tiles) and the long
 // rows of probe leaves were still running when the others had finished.  10,000 bodies FP64: near
 // field 273 -> 113 us and 50 us to cut and to add; 300k vortex ring FP64: 28.2 -> 25.5 ms (whole
 // solves).  More rows than that fill the GPU by themselves (1e6 bodies: 62.0 ms either way).
 constexpr int kItemRowsPerSM = 64, kItemWaves = 4, kItemSources = 256;
-constexpr double kItemPairs = 4e6;  // below this many pairs the extra launches cost more than they save,
-constexpr double kItemRowPairs = 1e5;  // but for rows that would keep one CTA busy for some 0.1 ms each
+// Body pairs per row (on average) from which rows are cut; to cut and to add takes some 40 us.  Near field
+// whole / cut: 4,096 rows of 3,000 pairs FP64 0.07 / 0.13 ms; 64 rows of 15,600 0.036 / 0.055; 407 uneven rows
+// of 20,000 (up to 210,000) 0.129 / 0.082; 512 even rows of 27,000 0.070 / 0.091, mixed 0.100 / 0.095; 64 rows of
+// 62,000, vortex particles, 0.10 / 0.07; 574 rows of 80,000 0.24 / 0.16; one row of 1.6e6 1.28 / 0.09.
+constexpr double kItemRowPairs = 1.6e4;
 constexpr int kTPT = 2;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -443,11 +446,12 @@ __host__ __device__ __forceinline__ int next_tile(int rem) {
   }
   return rem;
 }
-// (300k ring FP64 25.1 -> 23.8 ms, 2e6 ring mixed 210.4 -> 205.8 ms; mixed point sources only in whole
-// rows, 1e6 bodies 34.7 -> 34.5 ms: as items of the gradient of 2e5 sources 2.99 -> 3.22 ms)
+// (300k ring FP64 25.1 -> 23.8 ms, 2e6 ring mixed 210.4 -> 205.8 ms, 1e6 clustered bodies mixed 34.7 -> 34.5 ms.
+// Not in mixed items, whose pairs cost less than gathering far-off sources twice: gradient of 2e5 sources
+// 2.99 -> 3.22 ms; 1e4 probes around 2e5 vortex particles, near field 2.97 -> 4.03 ms)
 template <class R, int KIND, bool ITEMS>
 __host__ __device__ constexpr bool sub_tiles() {
-  return KIND == FMM_POINT_VORTEX || (sizeof(R) == 4 && !ITEMS);
+  return sizeof(R) == 4 ? !ITEMS : KIND == FMM_POINT_VORTEX;
 }
 
 // Targets per lane of a tile of nt targets on the FP64 path: three where 3 x a power of two lanes
@@ -1109,8 +1113,9 @@ __global__ void k_direct_sum(const double* __restrict__ part, int n_split, int64
   }
 }
 
-// source bodies of every row, one block each (eight loads of a thread in flight: the 32,000 leaves of
-// one row of probes took a warp 1 ms)
+// source bodies of every row, one block each, eight loads of a thread in flight (a warp per row and a
+// thread per sum in k_p2p_sum: 300 targets x 1e6 sources, 32,000 leaves a row, mixed, near field 1.03 ms;
+// 0.57 now)
 __global__ void k_p2p_row_sources(const int* __restrict__ off, const int* __restrict__ src_of,
                                   const int* __restrict__ s_count, int* __restrict__ n_src) {
   __shared__ int sum;
@@ -1221,8 +1226,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
   if (threadIdx.x == 0) *n_items = run.x;
 }
 
-// the shares of every tile that was cut, added in order; those of a tile of few sums and many shares in
-// several interleaved groups (a thread per sum alone took 0.2 ms for the 592 shares of a row of probes)
+// the shares of every tile that was cut, added in order; those of a tile of few sums and many shares
+// (rows of few targets and thousands of leaves) in several interleaved groups
 constexpr int kSumThreads = 128, kSumManyShares = 32;
 template <int KIND, bool PS, bool GS, int NA>
 __global__ void __launch_bounds__(kSumThreads) k_p2p_sum(const int4* __restrict__ items,
@@ -1289,7 +1294,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
   constexpr int NA = n_chan<KIND, GS, HS>();
   // body pairs (of a tuple's system: its part by the number of bodies)
   const double pairs = (double)L.n_pairs * ((double)stt.n_bodies / (double)L.n_source_bodies);
-  if (rows <= kItemRowsPerSM * n_sm && (pairs > kItemPairs || pairs > kItemRowPairs * rows)) {
+  if (rows <= kItemRowsPerSM * n_sm && pairs > kItemRowPairs * rows) {
     if (smem > 48 * 1024)
       FMM_CUDA_TRY(cudaFuncSetAttribute(k_p2p<R, KIND, PS, GS, HS, false, true>,
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
