@@ -583,8 +583,8 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   markf(2);
   if (!split) mark(5);
   if (o.horizontal_pass)
-    launch_m2l(T, S, W.lists, p, lh, o.error_method, o.error_tolerance, o.bonus_expansion, nullptr, stats.ptr,
-               c->tables, o.precision, fs);
+    launch_m2l(T, S, W.lists, p, lh, o.error_method, o.error_tolerance, o.bonus_expansion, stats.ptr, c->tables,
+               o.precision, fs);
   markf(3);
   if (!split) mark(6);
   // no translation into the locals: they are zero, and so is what the downward pass would add to every

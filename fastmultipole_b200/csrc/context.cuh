@@ -119,13 +119,12 @@ void launch_direct(const double4* tpos, int64_t nt, const double4* spos, const d
 // ---- expansions.cu ----
 void upload_tables(DevTables& dt, int p, cudaStream_t st);
 void launch_p2m(DevTree& s, int p, int kind, const DevTables& tb, cudaStream_t st);
-// per-pair orders go to p_used (device, one per m2l entry) when non-null; stats (device,
-// 4 ints, zeroed by the caller) receives the max order, a failure flag and the flop count
-// lane-per-pair M2L (m2l_lane.cu): point sources, orders 1..12; false = not handled
+// M2L: stats (device, 4 ints, zeroed by the caller) receives the max order, a failure flag and the
+// flop count.  launch_m2l_lane (m2l_lane.cu): orders 1..12 by lanes; false = not handled
 bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
-                     int* p_used, int* stats, int precision, cudaStream_t st);
+                     int* stats, int precision, cudaStream_t st);
 void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int error_method, double eps,
-                int be, int* p_used, int* stats, const DevTables& tb, int precision, cudaStream_t st);
+                int be, int* stats, const DevTables& tb, int precision, cudaStream_t st);
 void launch_l2p(DevTree& t, int p, bool lh, bool ps, bool gs, bool hs, double* acc13, cudaStream_t st);
 // unit operators over explicit pair lists (device arrays)
 void launch_op_m2m(int64_t n, double* target, const double* tc, const double* src, const double* sc, int p,

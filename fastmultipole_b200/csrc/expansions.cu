@@ -80,8 +80,7 @@ __global__ void __launch_bounds__(32 * kWarps) k_m2l_pair(const int* __restrict_
                                                           int n_targets, double* __restrict__ local,
                                                           const double* __restrict__ multipole,
                                                           const double* __restrict__ tcen,
-                                                          const double* __restrict__ scen, int* __restrict__ p_used,
-                                                          Tab tb, M2LStats stats) {
+                                                          const double* __restrict__ scen, Tab tb, M2LStats stats) {
   using K = eng::PairM2L<P, LH>;
   constexpr int NV = K::NH * K::NC;
   const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -97,7 +96,6 @@ __global__ void __launch_bounds__(32 * kWarps) k_m2l_pair(const int* __restrict_
   for (int l = l0 + lane; l < l1; l += 32) {
     const int s = src_of[l];
     K::run(acc, multipole + NH4 * s, tx - scen[3 * s], ty - scen[3 * s + 1], tz - scen[3 * s + 2], tb);
-    if (p_used) p_used[l] = P;
   }
 #pragma unroll
   for (int v = 0; v < NV; ++v)
@@ -858,7 +856,7 @@ struct OpM2LLaunch {
 }  // namespace
 
 void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
-                int* p_used, int* stats, const DevTables& tb, int precision, cudaStream_t st) {
+                int* stats, const DevTables& tb, int precision, cudaStream_t st) {
   if (L.n_m2l_targets == 0) return;
   // stats: [0] = max order used, [1] = any tolerance missed, [2..3] = flop count (u64)
   M2LStats S{stats, stats + 1, reinterpret_cast<unsigned long long*>(stats + 2)};
@@ -868,7 +866,7 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
     note_launch();
 #define FMM_M2L_PAIR(PP, LL)                                                                                   \
   k_m2l_pair<PP, LL><<<g, 32 * kWarps, 0, st>>>(L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, (int)L.n_m2l_targets, \
-                                                t.local.ptr, s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, p_used, T, S)
+                                                t.local.ptr, s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, T, S)
     if (lh) {
       if (p == 1) FMM_M2L_PAIR(1, true);
       else if (p == 2) FMM_M2L_PAIR(2, true);
@@ -882,7 +880,7 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
     FMM_CUDA_TRY(cudaGetLastError());
     return;
   }
-  if (launch_m2l_lane(t, s, L, p, lh, em, eps, be, p_used, stats, precision, st)) return;
+  if (launch_m2l_lane(t, s, L, p, lh, em, eps, be, stats, precision, st)) return;
   // higher orders, and vortex particles with error control
   launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, precision, st);
 }

@@ -668,8 +668,7 @@ __global__ void __launch_bounds__(32 * W) k_m2l_lane(const int* __restrict__ tgt
                                                  const double* __restrict__ tcen, const double* __restrict__ tbox,
                                                  const double* __restrict__ trad, const double* __restrict__ maxinf,
                                                  const double* __restrict__ scen, int em, double eps_in, int be,
-                                                 int* __restrict__ p_used, int* __restrict__ st_pmax,
-                                                 int* __restrict__ st_fail,
+                                                 int* __restrict__ st_pmax, int* __restrict__ st_fail,
                                                  unsigned long long* __restrict__ st_flops) {
   constexpr int NH = hi(PMAX + 1, 0);
   constexpr bool F32 = sizeof(V) == 4;
@@ -790,7 +789,6 @@ __global__ void __launch_bounds__(32 * W) k_m2l_lane(const int* __restrict__ tgt
         back_degree<PMAX>(n, un, q, Ms, stage, acc, lane);
     }
     if (q.valid) {
-      if (p_used) p_used[l] = q.P;
       pmax = max(pmax, q.P);
       fail = fail || !q.ok;
       fl += lane_pair_flops(q.P);
@@ -834,7 +832,7 @@ int sm_count() {
 }
 
 template <int PMAX, class V>
-void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double eps, int be, int* p_used, int* stats,
+void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double eps, int be, int* stats,
                 cudaStream_t st) {
   const size_t sm = lane_smem_bytes<PMAX, V>();
   note_launch();
@@ -846,7 +844,7 @@ void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double 
                                         (int)(WW * sm)));
       k_m2l_lane<PMAX, V, WW><<<(int)L.n_m2l_targets, 32 * WW, WW * sm, st>>>(
           L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-          t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
+          t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, stats, stats + 1,
           reinterpret_cast<unsigned long long*>(stats + 2));
       FMM_CUDA_TRY(cudaGetLastError());
       return;
@@ -856,18 +854,18 @@ void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double 
     FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
   k_m2l_lane<PMAX, V><<<(int)L.n_m2l_targets, 32, sm, st>>>(
       L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-      t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, p_used, stats, stats + 1,
+      t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, stats, stats + 1,
       reinterpret_cast<unsigned long long*>(stats + 2));
   FMM_CUDA_TRY(cudaGetLastError());
 }
 
 template <int PMAX>
-void run_lane(DevTree& t, const DevTree& s, const DevLists& L, int em, double eps, int be, int* p_used, int* stats,
+void run_lane(DevTree& t, const DevTree& s, const DevLists& L, int em, double eps, int be, int* stats,
               int precision, cudaStream_t st) {
   if (precision == FMM_PRECISION_MIXED)
-    run_lane_v<PMAX, float>(t, s, L, em, eps, be, p_used, stats, st);
+    run_lane_v<PMAX, float>(t, s, L, em, eps, be, stats, st);
   else
-    run_lane_v<PMAX, double>(t, s, L, em, eps, be, p_used, stats, st);
+    run_lane_v<PMAX, double>(t, s, L, em, eps, be, stats, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -938,7 +936,7 @@ __global__ void __launch_bounds__(128) k_m2l_small(const int* __restrict__ tgt_l
                                                    const int* __restrict__ src_of, int n_targets,
                                                    double* __restrict__ local, const double* __restrict__ multipole,
                                                    const double* __restrict__ tcen, const double* __restrict__ scen,
-                                                   int* __restrict__ p_used, int* __restrict__ st_pmax,
+                                                   int* __restrict__ st_pmax,
                                                    unsigned long long* __restrict__ st_flops) {
   constexpr int NH = hi(P + 1, 0);
   const int lane = threadIdx.x & 31;
@@ -998,7 +996,6 @@ __global__ void __launch_bounds__(128) k_m2l_small(const int* __restrict__ tgt_l
         acci[hi(n, m)] += Yi[m];
       }
     }
-    if (p_used) p_used[l] = P;
   }
 #pragma unroll
   for (int i = 0; i < NH; ++i)
@@ -1031,7 +1028,7 @@ __global__ void __launch_bounds__(128) k_m2l_small_f(const int* __restrict__ tgt
                                                      const int* __restrict__ src_of, int n_targets,
                                                      double* __restrict__ local, const double* __restrict__ multipole,
                                                      const double* __restrict__ tcen, const double* __restrict__ scen,
-                                                     int* __restrict__ p_used, int* __restrict__ st_pmax,
+                                                     int* __restrict__ st_pmax,
                                                      unsigned long long* __restrict__ st_flops) {
   constexpr int NH = hi(P + 1, 0);
   const int lane = threadIdx.x & 31;
@@ -1124,7 +1121,6 @@ __global__ void __launch_bounds__(128) k_m2l_small_f(const int* __restrict__ tgt
         ei = tt * sph + ei * cph;
       }
     }
-    if (p_used) p_used[l] = P;
   }
 #pragma unroll
   for (int i = 0; i < NH; ++i)
@@ -1155,24 +1151,24 @@ __global__ void __launch_bounds__(128) k_m2l_small_f(const int* __restrict__ tgt
 }
 
 template <int P>
-void run_m2l_small(DevTree& t, const DevTree& s, const DevLists& L, int* p_used, int* stats, int precision,
+void run_m2l_small(DevTree& t, const DevTree& s, const DevLists& L, int* stats, int precision,
                    cudaStream_t st) {
   note_launch();
   const int g = (int)((L.n_m2l_targets + 3) / 4);
   auto* fl = reinterpret_cast<unsigned long long*>(stats + 2);
   if (precision == FMM_PRECISION_MIXED)
     k_m2l_small_f<P><<<g, 128, 0, st>>>(L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, (int)L.n_m2l_targets, t.local.ptr,
-                                        s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, p_used, stats, fl);
+                                        s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, stats, fl);
   else
     k_m2l_small<P><<<g, 128, 0, st>>>(L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, (int)L.n_m2l_targets, t.local.ptr,
-                                      s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, p_used, stats, fl);
+                                      s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, stats, fl);
   FMM_CUDA_TRY(cudaGetLastError());
 }
 
 }  // namespace
 
 bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
-                     int* p_used, int* stats, int precision, cudaStream_t st) {
+                     int* stats, int precision, cudaStream_t st) {
   if (p < 1 || p > kLaneMaxP) return false;
   // vortex particles (order <= 3 the thread-per-pair kernel, else translate_deg.cu), and the mixed
   // path's fixed orders above 3 with many target rows (translate_deg.cu: 300k clustered bodies, order
@@ -1185,11 +1181,11 @@ bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, boo
   ensure_lane_tables(st);
   if (em == FMM_ERROR_NONE && p <= 3) {
     if (p == 1)
-      run_m2l_small<1>(t, s, L, p_used, stats, precision, st);
+      run_m2l_small<1>(t, s, L, stats, precision, st);
     else if (p == 2)
-      run_m2l_small<2>(t, s, L, p_used, stats, precision, st);
+      run_m2l_small<2>(t, s, L, stats, precision, st);
     else
-      run_m2l_small<3>(t, s, L, p_used, stats, precision, st);
+      run_m2l_small<3>(t, s, L, stats, precision, st);
     return true;
   }
   // FP64 with few target rows: the degrees of a pair spread over warps shorten the chain (1e4 bodies,
@@ -1197,18 +1193,18 @@ bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, boo
   // here and 11.7 there)
   if (precision != FMM_PRECISION_MIXED && L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) return false;
   switch (p) {
-    case 1: run_lane<1>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 2: run_lane<2>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 3: run_lane<3>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 4: run_lane<4>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 5: run_lane<5>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 6: run_lane<6>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 7: run_lane<7>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 8: run_lane<8>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 9: run_lane<9>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 10: run_lane<10>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    case 11: run_lane<11>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
-    default: run_lane<12>(t, s, L, em, eps, be, p_used, stats, precision, st); break;
+    case 1: run_lane<1>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 2: run_lane<2>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 3: run_lane<3>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 4: run_lane<4>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 5: run_lane<5>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 6: run_lane<6>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 7: run_lane<7>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 8: run_lane<8>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 9: run_lane<9>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 10: run_lane<10>(t, s, L, em, eps, be, stats, precision, st); break;
+    case 11: run_lane<11>(t, s, L, em, eps, be, stats, precision, st); break;
+    default: run_lane<12>(t, s, L, em, eps, be, stats, precision, st); break;
   }
   return true;
 }
