@@ -41,6 +41,7 @@ struct DevLists {
   int64_t n_pairs = 0, n_source_bodies = 0;  // body pairs of the direct list; bodies of its source tree
   DevBuf<int> m2l_t, m2l_s, dir_t, dir_s;
   int64_t n_m2l_targets = 0, n_dir_targets = 0;
+  int64_t m2l_longest = 0;  // pairs of the longest M2L row
   DevBuf<int> m2l_tgt, m2l_off;   // unique targets, offsets (n+1)
   DevBuf<int> dir_tgt, dir_off;
   // near field of launches of few rows: their items (p2p.cu), number of items and sources per

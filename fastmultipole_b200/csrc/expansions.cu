@@ -881,7 +881,7 @@ void launch_m2l(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh,
     return;
   }
   if (launch_m2l_lane(t, s, L, p, lh, em, eps, be, stats, precision, st)) return;
-  // higher orders, and vortex particles with error control
+  // what the lanes do not take (lanes_take in m2l_lane.cu)
   launch_m2l_deg(t, s, L, p, lh, em, eps, be, stats, precision, st);
 }
 

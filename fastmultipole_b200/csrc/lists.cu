@@ -255,6 +255,8 @@ __global__ void k_pack_counts(const int* __restrict__ cnt, int n, unsigned long 
 constexpr int kSmallRow = 256;  // rows up to this length: one warp each (merge sort in registers)
 constexpr int kMidRow = 4096;   // up to this length: one block each; longer: segmented radix sort
 constexpr int kMidClasses = 4;  // block sorts of 512, 1024, 2048 and 4096 keys
+constexpr int kLongestSlot = 2 + kMidClasses;
+static_assert(C_ROWS_DIR + kLongestSlot < C_ROWS_M2L, "counters of a list");
 
 __host__ __device__ constexpr int mid_class(int c) { return c <= 512 ? 0 : c <= 1024 ? 1 : c <= 2048 ? 2 : 3; }
 
@@ -264,7 +266,7 @@ struct Rows {
   const int2* raw;       // pairs in arrival order
   int n;                 // pairs
   int *off, *tgt, *roff; // offsets of all targets, the CSR of the non-empty ones
-  int* ctr;              // rows, rows per block class, big rows
+  int* ctr;              // rows, rows per block class, big rows, longest row
   int *mid, *big_b, *big_e, *big_r;  // rows per block class (n_targets + 1 each), longer rows
   int *cursor, *tmp;     // slots taken per target, rows before their sort
   int *out_t, *out_s;
@@ -281,6 +283,7 @@ __global__ void k_rows(RowsPair P, const unsigned long long* __restrict__ scan, 
   const Rows& L = P.l[blockIdx.y];
   const unsigned long long* ex = scan + (size_t)blockIdx.y * (n + 1);
   const unsigned long long base = ex[0];
+  int longest = 0;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t <= n; t += gridDim.x * blockDim.x) {
     const unsigned long long e = ex[t] - base;
     const int o = (int)(e >> 32), r = (int)(e & 0xffffffffu);
@@ -288,6 +291,7 @@ __global__ void k_rows(RowsPair P, const unsigned long long* __restrict__ scan, 
     if (t < n) {
       L.cursor[t] = 0;
       const int c = L.cnt[t];
+      longest = max(longest, c);
       if (c > 0) {
         L.tgt[r] = t;
         L.roff[r] = o;
@@ -306,6 +310,8 @@ __global__ void k_rows(RowsPair P, const unsigned long long* __restrict__ scan, 
       L.ctr[0] = r;
     }
   }
+  longest = __reduce_max_sync(kFull, longest);
+  if ((threadIdx.x & 31) == 0 && longest > 0) atomicMax(L.ctr + kLongestSlot, longest);
 }
 
 // raw pairs into their target's row, sources only (order inside a row fixed by the
@@ -626,6 +632,7 @@ void build_lists(DevLists& L, const DevTree& tt, const DevTree& stt, Scratch& sc
   L.n_source_bodies = stt.n_bodies;
   L.n_dir_targets = rows[0];
   L.n_m2l_targets = rows[1];
+  L.m2l_longest = h_m[kLongestSlot];
   L.rule_method = method;
 }
 

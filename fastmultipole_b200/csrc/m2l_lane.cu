@@ -1,5 +1,5 @@
-// m2l_lane.cu -- lane-per-pair M2L for point sources, orders 1..kLaneMaxP,
-// plain and error-controlled.
+// m2l_lane.cu -- lane-per-pair M2L for point sources, orders 1..kLaneMaxP, plain and
+// error-controlled, and with two lanes per pair for vortex particles, plain, orders 4..10.
 //
 // One warp owns one target branch and takes its M2L sources 32 at a time, one
 // (target, source) pair per lane.  Each lane runs the reference's chain
@@ -836,19 +836,17 @@ void run_lane_v(DevTree& t, const DevTree& s, const DevLists& L, int em, double 
                 cudaStream_t st) {
   const size_t sm = lane_smem_bytes<PMAX, V>();
   note_launch();
-  if constexpr (sizeof(V) == 4) {
-    if (L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) {
-      // few target rows (small problems, probe trees): kWideM2LWarps warps share each row
-      constexpr int WW = kWideM2LWarps;
-      FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V, WW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)(WW * sm)));
-      k_m2l_lane<PMAX, V, WW><<<(int)L.n_m2l_targets, 32 * WW, WW * sm, st>>>(
-          L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
-          t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, stats, stats + 1,
-          reinterpret_cast<unsigned long long*>(stats + 2));
-      FMM_CUDA_TRY(cudaGetLastError());
-      return;
-    }
+  if (L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) {
+    // few target rows (small problems, probe trees): kWideM2LWarps warps share each row
+    constexpr int WW = kWideM2LWarps;
+    FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V, WW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)(WW * sm)));
+    k_m2l_lane<PMAX, V, WW><<<(int)L.n_m2l_targets, 32 * WW, WW * sm, st>>>(
+        L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, t.tbox.ptr,
+        t.tradius.ptr, t.max_influence.ptr, s.scenter.ptr, em, eps, be, stats, stats + 1,
+        reinterpret_cast<unsigned long long*>(stats + 2));
+    FMM_CUDA_TRY(cudaGetLastError());
+    return;
   }
   if (sm > 48 * 1024)
     FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
@@ -1165,21 +1163,260 @@ void run_m2l_small(DevTree& t, const DevTree& s, const DevLists& L, int* stats, 
   FMM_CUDA_TRY(cudaGetLastError());
 }
 
+// ---- Lamb-Helmholtz (vortex particle) plain M2L ---------------------------------
+// One warp per target branch, two lanes per (target, source) pair: lanes 0-15 carry set 0
+// (phi) and lanes 16-31 set 1 (chi) of the same 16 pairs, so each lane rotates, translates
+// and rotates back one set.  Before the rotations (in V: FP32 on the mixed path, FP64 on the
+// drop-in path) set 0 of the multipole is scaled by t^-n and set 1 by t^(1-n); the coaxial
+// translation with (n+n')! then gives the local sets times t^(n+1) and t^(n+2), on which the
+// Lamb-Helmholtz coupling of transform_lamb_helmholtz_local! (src/translate.jl:98-142) needs no
+// power of t:
+//   phi(n, m) -= i (m / n) chi(n, m),  chi(n, m) -= chi(n + 1, m) / (n + 1).
+// The chi lane translates one degree ahead (it needs chi(n + 1)) and keeps chi(n) from the
+// step before, which the phi lane reads across the warp (xor 16).  The rotated-back degrees are
+// staged in shared memory unscaled (in V) with each lane's t^-(n+1) (phi) or t^-(n+2) (chi),
+// and summed over the 16 pairs in FP64, value times power, into the warp's FP64 accumulator.
+// One set per lane halves the registers and the shared memory a pair holds on a lane
+// (order 12, FP32: 30 KB per warp, 7 warps per SM instead of 4 with a pair per lane).
+template <int PMAX, class V>
+constexpr size_t lane_lh_smem_bytes() {
+  return ((size_t)4 * hi(PMAX + 1, 0) + 32) * sizeof(double) +
+         ((size_t)4 * (PMAX + 1) * 17 + (size_t)2 * hi(PMAX + 1, 0) * 32) * sizeof(V);
+}
+
+// coaxial translation of the lane's set, degree n, orders m <= mmax, scaled:
+// sum_{n'} (n+n')! M(n', m) (source degrees outer, orders inner: one degree's loads and FMAs
+// are independent, each sum keeps its n'-ascending order)
+template <int PMAX, class V>
+__device__ __forceinline__ void coax_lh(int n, int mmax, int P, const V* Ms, int lane, V (&Xr)[PMAX + 1],
+                                        V (&Xi)[PMAX + 1]) {
+#pragma unroll
+  for (int m = 0; m <= PMAX; ++m) Xr[m] = Xi[m] = V(0);
+#pragma unroll 2
+  for (int np = 0; np <= P; ++np) {
+    const V c = sizeof(V) == 4 ? (V)c_factF[n + np] : (V)c_fact[n + np];
+    const int base = hi(np, 0);
+#pragma unroll
+    for (int m = 0; m <= PMAX; ++m) {
+      if (m > mmax || m > np) break;
+      Xr[m] += c * Ms[(2 * (base + m)) * 32 + lane];
+      Xi[m] += c * Ms[(2 * (base + m) + 1) * 32 + lane];
+    }
+  }
+}
+
+// resident warps that the registers have to allow, 0: as the compiler chooses.  (FP64 order 7 takes 186
+// registers by itself: 6.3e6 pairs in 13.2 ms, held to 160 10.5; order 4 125, 3.37 ms, held to 120 3.09)
+template <int PMAX, class V>
+constexpr int lane_lh_min_blocks() {
+  return sizeof(V) == 8 && PMAX == 7 ? 12 : sizeof(V) == 8 && PMAX == 4 ? 16 : 0;
+}
+
+template <int PMAX, class V>
+__global__ void __launch_bounds__(32, lane_lh_min_blocks<PMAX, V>())
+    k_m2l_lane_lh(const int* __restrict__ tgt_list, const int* __restrict__ off, const int* __restrict__ src_of,
+                  double* __restrict__ local, const double* __restrict__ multipole, const double* __restrict__ tcen,
+                  const double* __restrict__ scen, int P, int* __restrict__ st_pmax,
+                  unsigned long long* __restrict__ st_flops) {
+  constexpr int NH = hi(PMAX + 1, 0);
+  extern __shared__ double lane_smem[];
+  double* acc = lane_smem;                    // [4 NH]
+  double* tsc = acc + 4 * NH;                 // per pair t^-(n+1) (set 0), t^-(n+2) (set 1): [2][16]
+  V* stage = reinterpret_cast<V*>(tsc + 32);  // unscaled rotated-back values [4 (PMAX+1)][17]
+  V* Ms = stage + 4 * (PMAX + 1) * 17;        // rotated multipole of the lane's set [2 NH][32]
+  const int lane = threadIdx.x;
+  const int set = lane >> 4, slot = lane & 15;
+  const int b = blockIdx.x;
+  const int t = tgt_list[b];
+  const double tc0 = tcen[3 * t], tc1 = tcen[3 * t + 1], tc2 = tcen[3 * t + 2];
+  for (int i = lane; i < 4 * NH; i += 32) acc[i] = 0.0;
+  const int l0 = off[b], l1 = off[b + 1];
+  for (int lb = l0; lb < l1; lb += 16) {
+    const int l = lb + slot;
+    const bool valid = l < l1;
+    const double* src = multipole;
+    double cph = 1.0, sph = 0.0, cth = 1.0, sth = 0.0, r = 1.0, rinv = 1.0;
+    if (valid) {
+      const int s = src_of[l];
+      src = multipole + (int64_t)4 * NH * s;
+      const double x = tc0 - scen[3 * s], y = tc1 - scen[3 * s + 1], z = tc2 - scen[3 * s + 2];
+      const double x2y2 = x * x + y * y;
+      r = sqrt(x2y2 + z * z);
+      if (x2y2 > 0) {
+        const double rho = sqrt(x2y2);
+        cph = x / rho;
+        sph = y / rho;
+        cth = z / r;
+        sth = rho / r;
+      } else {
+        cth = z < 0 ? -1.0 : 1.0;
+      }
+      rinv = 1 / r;
+    }
+    const V fcph = (V)cph, fsph = (V)sph, fcth = (V)cth, fsth = (V)sth;
+    // forward: the lane's set of every degree, scaled (t^-n, t^(1-n)) and rotated
+    double sc = set ? r : 1.0;
+#pragma unroll 1
+    for (int n = 0; n <= P; ++n) {
+      if (n > 0) sc *= rinv;
+      V Xr[PMAX + 1], Xi[PMAX + 1];
+      double er = 1.0, ei = 0.0;
+      const int base = hi(n, 0);
+#pragma unroll
+      for (int a = 0; a <= PMAX; ++a) {
+        Xr[a] = Xi[a] = V(0);
+        if (a > n || !valid) continue;
+        const double2 u = __ldg(reinterpret_cast<const double2*>(src) + 2 * (base + a) + set);
+        Xr[a] = (V)((u.x * er - u.y * ei) * sc);
+        Xi[a] = (V)((u.x * ei + u.y * er) * sc);
+        const double tt = er;
+        er = er * cph - ei * sph;
+        ei = tt * sph + ei * cph;
+      }
+      V Yr[PMAX + 1], Yi[PMAX + 1];
+      rot_y<PMAX, false, V>(n, Xr, Xi, fcth, fsth, Yr, Yi);
+#pragma unroll
+      for (int m = 0; m <= PMAX; ++m) {
+        if (m > n) break;
+        Ms[(2 * (base + m)) * 32 + lane] = Yr[m];
+        Ms[(2 * (base + m) + 1) * 32 + lane] = Yi[m];
+      }
+    }
+    __syncwarp();
+    // back: the chi lane carries chi(n) (Cr, Ci) and translates chi(n + 1); the phi lane
+    // translates phi(n) and reads chi(n) from its chi lane
+    V Cr[PMAX + 1], Ci[PMAX + 1];
+    coax_lh<PMAX, V>(0, 0, P, Ms, lane, Cr, Ci);
+    double tn1 = rinv;  // t^-(n+1)
+#pragma unroll 1
+    for (int n = 0; n <= P; ++n) {
+      if (n > 0) tn1 *= rinv;
+      const int nd = n + set;  // degree the lane translates
+      V Nr[PMAX + 1], Ni[PMAX + 1];
+      if (nd <= P) {
+        coax_lh<PMAX, V>(nd, n + 1, P, Ms, lane, Nr, Ni);
+      } else {
+#pragma unroll
+        for (int m = 0; m <= PMAX; ++m) Nr[m] = Ni[m] = V(0);
+      }
+      V Xr[PMAX + 1], Xi[PMAX + 1], Yr[PMAX + 1], Yi[PMAX + 1];
+      const V inv_n = n > 0 ? V(1) / (V)n : V(0);
+      const V inv_n1 = V(1) / (V)(n + 1);
+#pragma unroll
+      for (int m = 0; m <= PMAX; ++m) {
+        Xr[m] = Xi[m] = V(0);
+        if (m > n) continue;
+        const V pr = __shfl_xor_sync(kAll, Cr[m], 16), pi = __shfl_xor_sync(kAll, Ci[m], 16);
+        if (set == 0) {  // phi(n, m) - i (m / n) chi(n, m)
+          const V a = (V)m * inv_n;
+          Xr[m] = Nr[m] - a * pi;
+          Xi[m] = Ni[m] + a * pr;
+        } else {  // chi(n, m) - chi(n + 1, m) / (n + 1)
+          Xr[m] = Cr[m] - inv_n1 * Nr[m];
+          Xi[m] = Ci[m] - inv_n1 * Ni[m];
+        }
+      }
+      if (set) {  // chi(n + 1) is the next step's chi(n)
+#pragma unroll
+        for (int m = 0; m <= PMAX; ++m) {
+          Cr[m] = Nr[m];
+          Ci[m] = Ni[m];
+        }
+      }
+      rot_y<PMAX, true, V>(n, Xr, Xi, fcth, fsth, Yr, Yi);
+      V er = 1, ei = 0;
+#pragma unroll
+      for (int m = 0; m <= PMAX; ++m) {
+        if (m > n) break;
+        const V vr = Yr[m] * er + Yi[m] * ei;  // times e^{-i m phi}
+        const V vi = Yi[m] * er - Yr[m] * ei;
+        stage[(4 * m + 2 * set) * 17 + slot] = valid ? vr : V(0);
+        stage[(4 * m + 2 * set + 1) * 17 + slot] = valid ? vi : V(0);
+        const V tt = er;
+        er = er * fcph - ei * fsph;
+        ei = tt * fsph + ei * fcph;
+      }
+      tsc[lane] = set ? tn1 * rinv : tn1;
+      __syncwarp();
+      // 4 (n + 1) staged rows (order m, set, re/im), each value times its pair's power of t
+      // in FP64 (set 0: t^-(n+1), set 1: t^-(n+2))
+      for (int row = lane; row < 4 * (n + 1); row += 32) {
+        const double* ts = tsc + ((row & 2) ? 16 : 0);
+        double v = 0.0;
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v += (double)stage[row * 17 + k] * ts[k];
+        acc[4 * hi(n, 0) + row] += v;
+      }
+      __syncwarp();
+    }
+    __syncwarp();
+  }
+  double* dst = local + (int64_t)4 * NH * t;
+  for (int i = lane; i < 4 * NH; i += 32) dst[i] += acc[i];
+  if (lane == 0) {
+    atomicMax(st_pmax, P);
+    atomicAdd(st_flops, (unsigned long long)(l1 - l0) * 2ull * lane_pair_flops(P));
+  }
+}
+
+struct LaneLHGo {
+  DevTree& t;
+  const DevTree& s;
+  const DevLists& L;
+  int* stats;
+  int precision;
+  cudaStream_t st;
+  template <int PMAX, class V>
+  void run() {
+    constexpr size_t sm = lane_lh_smem_bytes<PMAX, V>();
+    if (sm > 48 * 1024)
+      FMM_CUDA_TRY(cudaFuncSetAttribute(k_m2l_lane_lh<PMAX, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm));
+    note_launch();
+    k_m2l_lane_lh<PMAX, V><<<(int)L.n_m2l_targets, 32, sm, st>>>(
+        L.m2l_tgt.ptr, L.m2l_off.ptr, L.m2l_s.ptr, t.local.ptr, s.multipole.ptr, t.tcenter.ptr, s.scenter.ptr, PMAX,
+        stats, reinterpret_cast<unsigned long long*>(stats + 2));
+    FMM_CUDA_TRY(cudaGetLastError());
+  }
+  template <int PMAX>
+  void go() {
+    if (precision == FMM_PRECISION_MIXED)
+      run<PMAX, float>();
+    else
+      run<PMAX, double>();
+  }
+};
+
+// Whether the lanes of this file take a launch, or the degrees spread over warps of translate_deg.cu (deg).
+// A pass of a warp's lanes is the longer chain, so that the longest row decides where the GPU would
+// wait for it: rows count as even when they hold the pairs of kEvenRowsPerSM of the longest per SM.
+// Measured, ms here / deg, rows given with the longest:
+//   vortex particles, fixed order.  6,845 rows, 655,000 pairs (even, up to 472): FP64 order 4 0.37 / 1.08, 8 1.70 /
+//     2.80, 10 3.85 / 4.04, 12 6.19 / 5.82; mixed 8 1.19 / 1.49, 10 1.84 / 2.12, 12 3.62 / 3.04.  4,631 rows, 442,000
+//     pairs (uneven, up to 1,407): FP64 8 2.93 / 2.02, mixed 3.05 / 1.56.
+//   point sources, mixed, fixed order, the same rows: even 4 0.22 / 0.29, 8 0.69 / 0.72, 10 1.18 / 1.00; uneven 4 0.55 /
+//     0.33, 8 1.50 / 0.72.  Few rows, which four warps share here: 0.43 / 0.57 (gradient of 2e5 sources).
+//   point sources, FP64.  24,000 rows, order 10: 10.5 / 11.7.  64 rows up to 871: 4 0.09 / 0.18, 12 0.63 / 0.84,
+//     tolerance 0.46 / 0.81.  571 up to 202: 4 0.039 / 0.053, 10 0.28 / 0.16, tolerance 0.24 / 0.17.  576 up to 2,808:
+//     8 1.33 / 2.02, 10 2.88 / 2.73, tolerance 1.89 / 2.61.  351 up to 76: 8 0.086 / 0.057.
+constexpr int64_t kEvenRowsPerSM = 5, kLongRow = 128;
+bool lanes_take(const DevLists& L, int p, bool lh, int em, int precision) {
+  const int64_t n_sm = sm_count(), rows = L.n_m2l_targets, longest = L.m2l_longest;
+  const bool mixed = precision == FMM_PRECISION_MIXED, fixed = em == FMM_ERROR_NONE;
+  const bool even = L.n_m2l >= kEvenRowsPerSM * n_sm * longest;
+  if (lh) return fixed && p >= 4 && p <= 10 && even;
+  if (rows >= kWideM2LRowsPerSM * n_sm) return !(mixed && fixed) || (even && p <= 8);
+  if (mixed) return true;
+  return longest >= kLongRow && ((fixed && p <= 8) || rows <= 2 * n_sm || (!fixed && longest >= 4 * kLongRow));
+}
+
 }  // namespace
 
 bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, bool lh, int em, double eps, int be,
                      int* stats, int precision, cudaStream_t st) {
   if (p < 1 || p > kLaneMaxP) return false;
-  // vortex particles (order <= 3 the thread-per-pair kernel, else translate_deg.cu), and the mixed
-  // path's fixed orders above 3 with many target rows (translate_deg.cu: 300k clustered bodies, order
-  // 10, 1.0 ms where this kernel took 2.0; few rows of many pairs are faster here, where four warps
-  // share a row: 0.43 and 0.57 ms of the gradient of 2e5 sources)
-  if (lh || (precision == FMM_PRECISION_MIXED && em == FMM_ERROR_NONE && p > 3 &&
-             L.n_m2l_targets >= (int64_t)kWideM2LRowsPerSM * sm_count()))
-    return false;
   if (L.n_m2l_targets == 0) return true;
-  ensure_lane_tables(st);
-  if (em == FMM_ERROR_NONE && p <= 3) {
+  if (!lh && em == FMM_ERROR_NONE && p <= 3) {
+    ensure_lane_tables(st);
     if (p == 1)
       run_m2l_small<1>(t, s, L, stats, precision, st);
     else if (p == 2)
@@ -1188,10 +1425,21 @@ bool launch_m2l_lane(DevTree& t, const DevTree& s, const DevLists& L, int p, boo
       run_m2l_small<3>(t, s, L, stats, precision, st);
     return true;
   }
-  // FP64 with few target rows: the degrees of a pair spread over warps shorten the chain (1e4 bodies,
-  // order 6, 59 us here with four warps per row; the 24,000 rows of 1e6 bodies, order 10, take 10.5 ms
-  // here and 11.7 there)
-  if (precision != FMM_PRECISION_MIXED && L.n_m2l_targets < (int64_t)kWideM2LRowsPerSM * sm_count()) return false;
+  if (!lanes_take(L, p, lh, em, precision)) return false;
+  ensure_lane_tables(st);
+  if (lh) {
+    LaneLHGo f{t, s, L, stats, precision, st};
+    switch (p) {
+      case 4: f.go<4>(); break;
+      case 5: f.go<5>(); break;
+      case 6: f.go<6>(); break;
+      case 7: f.go<7>(); break;
+      case 8: f.go<8>(); break;
+      case 9: f.go<9>(); break;
+      default: f.go<10>(); break;
+    }
+    return true;
+  }
   switch (p) {
     case 1: run_lane<1>(t, s, L, em, eps, be, stats, precision, st); break;
     case 2: run_lane<2>(t, s, L, em, eps, be, stats, precision, st); break;
