@@ -59,13 +59,15 @@ __device__ __forceinline__ bool mac_accept(const double4& tg, const double4& sg,
 
 // one step of build_interaction_lists! for the three rule sets
 // (src/interaction_list.jl:23-64, 66-120, 122-166); for a split, n_next children
-// starting at child0 (of the target for A_SPLIT_T, of the source for A_SPLIT_S)
-__device__ int decide(const TreeRef& T, int t, const TreeRef& S, int s, const Rule& R, int& n_next, int& child0) {
+// starting at child0 (of the target for A_SPLIT_T, of the source for A_SPLIT_S); pairs: the body pairs
+__device__ int decide(const TreeRef& T, int t, const TreeRef& S, int s, const Rule& R, int& n_next, int& child0,
+                      unsigned long long& pairs) {
   n_next = 0;
   child0 = 0;
   const int4 ti = T.info[t], si = S.info[s];
   const int nct = ti.x, ncs = si.x;
   const int bt = ti.z, bs = si.z;
+  pairs = (unsigned long long)bt * (unsigned)bs;
   bool both_leaves = (nct == 0) && (ncs == 0);
   bool dir_ok = (R.nf || (t == s && R.si)) && (t != s || R.si);
   if (R.method == FMM_LIST_BARBA) {
@@ -153,23 +155,24 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
   __shared__ int wsum[3][NW];
   __shared__ int bbase[3];
   __shared__ int stop;
+  __shared__ unsigned long long bpairs;
   // after an overflow the frontier holds unwritten slots: the steps that follow do
   // nothing, and the host grows the buffers and repeats the traversal.  Another block
   // of this step may raise the flag meanwhile, so one thread reads it for the block:
   // the block leaves or stays as a whole (its barriers and block sums need every warp)
-  if (threadIdx.x == 0) stop = *reinterpret_cast<volatile int*>(ctr + C_FLAG);
+  if (threadIdx.x == 0) stop = *reinterpret_cast<volatile int*>(ctr + C_FLAG), bpairs = 0;
   __syncthreads();
   if (stop) return;
   const int n = min(ctr[k], cap_f);
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   bool bad = false;
-  unsigned long long pairs = 0;  // body pairs of this thread's direct pairs
   // a frontier that the launch's threads cover takes one pair per thread
   const int items = n > (int)gridDim.x * kStepThreads ? kStepItems : 1, chunk = items * kStepThreads;
   for (int c0 = blockIdx.x * chunk; c0 < n; c0 += gridDim.x * chunk) {
     int2 p[kStepItems];
     int a[kStepItems], nn[kStepItems], ch[kStepItems];
     int cd = 0, cm = 0, cf = 0;
+    unsigned long long pairs = 0;  // body pairs of this thread's direct pairs
 #pragma unroll
     for (int r = 0; r < kStepItems; ++r) {
       const int i = c0 + r * kStepThreads + threadIdx.x;
@@ -179,7 +182,9 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
       ch[r] = 0;
       if (r < items && i < n) {
         p[r] = fin[i];
-        a[r] = decide(T, p[r].x, S, p[r].y, R, nn[r], ch[r]);
+        unsigned long long v;
+        a[r] = decide(T, p[r].x, S, p[r].y, R, nn[r], ch[r], v);
+        if (a[r] == A_DIRECT) pairs += v;
       }
       if (a[r] != A_SPLIT_T && a[r] != A_SPLIT_S) nn[r] = 0;
       cd += a[r] == A_DIRECT;
@@ -207,7 +212,6 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
 #pragma unroll
     for (int r = 0; r < kStepItems; ++r) {
       if (a[r] == A_DIRECT) {
-        pairs += (unsigned long long)T.info[p[r].x].z * (unsigned long long)S.info[p[r].y].z;
         if (od < cap_d)
           rdir[od] = p[r];
         else
@@ -234,12 +238,16 @@ __global__ void __launch_bounds__(kStepThreads) k_step(const int2* __restrict__ 
         count_targets(a[r] == A_M2L, p[r].x, lane, cm2l);
       }
     }
-    __syncthreads();  // wsum / bbase are rewritten by the next chunk
+    if (__any_sync(kFull, cd > 0)) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
+      if (lane == 0) atomicAdd(&bpairs, pairs);
+    }
+    __syncthreads();  // wsum / bbase are rewritten by the next chunk, bpairs is complete
   }
   if (bad) atomicOr(ctr + C_FLAG, 1);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) pairs += __shfl_xor_sync(kFull, pairs, o);
-  if (lane == 0 && pairs) atomicAdd(reinterpret_cast<unsigned long long*>(ctr + C_PAIRS), pairs);
+  // one addition per block to the launch's counter
+  if (threadIdx.x == 0 && bpairs) atomicAdd(reinterpret_cast<unsigned long long*>(ctr + C_PAIRS), bpairs);
 }
 
 // per target: (count << 32) | (count > 0), so that one exclusive scan gives both the

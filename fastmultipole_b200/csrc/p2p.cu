@@ -133,7 +133,10 @@ __device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7
 // so do, where the potential is asked for, strengths below 2^-536 (not zero): the potential is
 // (q r^-3) r^2, r below 2^162, and q r^-3 would be subnormal where q / r is not
 constexpr int kTinyHi = (1023 - 536) << 20;
-__device__ __forceinline__ bool tiny_strength(double q) { return hi_abs(q) < kTinyHi && q != 0.0; }
+__device__ __forceinline__ bool tiny_strength(double q) {
+  const int h = hi_abs(q);
+  return h < kTinyHi && (h | __double2loint(q)) != 0;
+}
 
 // one source body on one target, Laplace, 17 FP64 operations: phi = (q / r^3) r^2
 template <bool PS>
