@@ -126,7 +126,15 @@ __global__ void k_pack_nodes(NodeIn T, NodeIn S, int2* front, int* ctr) {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kMaxSteps = 64;  // frontier counters; a traversal takes levels_t + levels_s - 1 steps
-enum : int { C_DIR = kMaxSteps, C_M2L, C_FLAG, C_ROWS_DIR, C_ROWS_M2L = C_ROWS_DIR + 8, C_PAIRS = C_ROWS_M2L + 9, C_N = 128 };
+enum : int {
+  C_DIR = kMaxSteps,
+  C_M2L,
+  C_FLAG,
+  C_ROWS_DIR,
+  C_ROWS_M2L = C_ROWS_DIR + 8,
+  C_PAIRS = C_ROWS_M2L + 9,
+  C_N = 128
+};
 static_assert(C_PAIRS % 2 == 0, "the body pairs of the direct list are a 64-bit counter");
 constexpr int kStepThreads = 128;
 constexpr int kStepMaxBlocks = 148 * 16;

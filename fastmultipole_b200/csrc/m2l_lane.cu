@@ -1149,8 +1149,7 @@ __global__ void __launch_bounds__(128) k_m2l_small_f(const int* __restrict__ tgt
 }
 
 template <int P>
-void run_m2l_small(DevTree& t, const DevTree& s, const DevLists& L, int* stats, int precision,
-                   cudaStream_t st) {
+void run_m2l_small(DevTree& t, const DevTree& s, const DevLists& L, int* stats, int precision, cudaStream_t st) {
   note_launch();
   const int g = (int)((L.n_m2l_targets + 3) / 4);
   auto* fl = reinterpret_cast<unsigned long long*>(stats + 2);
@@ -1393,8 +1392,8 @@ struct LaneLHGo {
 //   vortex particles, fixed order.  6,845 rows, 655,000 pairs (even, up to 472): FP64 order 4 0.37 / 1.08, 8 1.70 /
 //     2.80, 10 3.85 / 4.04, 12 6.19 / 5.82; mixed 8 1.19 / 1.49, 10 1.84 / 2.12, 12 3.62 / 3.04.  4,631 rows, 442,000
 //     pairs (uneven, up to 1,407): FP64 8 2.93 / 2.02, mixed 3.05 / 1.56.
-//   point sources, mixed, fixed order, the same rows: even 4 0.22 / 0.29, 8 0.69 / 0.72, 10 1.18 / 1.00; uneven 4 0.55 /
-//     0.33, 8 1.50 / 0.72.  Few rows, which four warps share here: 0.43 / 0.57 (gradient of 2e5 sources).
+//   point sources, mixed, fixed order, the same rows: even 4 0.22 / 0.29, 8 0.69 / 0.72, 10 1.18 / 1.00; uneven 4
+//     0.55 / 0.33, 8 1.50 / 0.72.  Few rows, which four warps share here: 0.43 / 0.57 (gradient of 2e5 sources).
 //   point sources, FP64.  24,000 rows, order 10: 10.5 / 11.7.  64 rows up to 871: 4 0.09 / 0.18, 12 0.63 / 0.84,
 //     tolerance 0.46 / 0.81.  571 up to 202: 4 0.039 / 0.053, 10 0.28 / 0.16, tolerance 0.24 / 0.17.  576 up to 2,808:
 //     8 1.33 / 2.02, 10 2.88 / 2.73, tolerance 1.89 / 2.61.  351 up to 76: 8 0.086 / 0.057.

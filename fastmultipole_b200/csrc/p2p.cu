@@ -486,21 +486,20 @@ __device__ __forceinline__ double pick(const float (&v)[N], int) { return v[0]; 
 // 28.6 ms, 28.8 with 2 CTAs, and 49.3 with 4, whose 128 registers spill inside the loop)
 template <class R, int KIND, bool HS, bool RW>
 __host__ __device__ constexpr int p2p_min_blocks() {
-  constexpr int regs = (KIND == FMM_POINT_VORTEX && HS) ? (RW ? 168 : 128) : (RW ? 72 : 64);
-  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS && !RW) ? 3 : 4;
+  static_assert(!RW || packed<R, KIND>(), "a warp per row: packed point sources only");
+  if (sizeof(R) != 4) return (KIND == FMM_POINT_VORTEX && HS) ? 3 : 4;
+  constexpr int regs = (KIND == FMM_POINT_VORTEX && HS) ? 128 : (RW ? 72 : 64);
   return 65536 / (regs * kWarps * 32);
 }
 
 template <class R, int KIND, bool PS, bool GS, bool HS, bool RW, bool ITEMS>
-__global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()) k_p2p(const int* __restrict__ tgt_list, const int* __restrict__ off,
-                                                     int n_rows, const int* __restrict__ src_of,
-                                                     const int* __restrict__ t_start, const int* __restrict__ t_count,
-                                                     const double* __restrict__ t_center,
-                                                     const int* __restrict__ s_start, const int* __restrict__ s_count,
-                                                     const double4* __restrict__ tpos, const double4* __restrict__ spos,
-                                                     const double4* __restrict__ sstr, double* __restrict__ acc13,
-                                                     const int4* __restrict__ items, const int* __restrict__ n_items,
-                                                     double* __restrict__ item_sums, int exact_self) {
+__global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>())
+    k_p2p(const int* __restrict__ tgt_list, const int* __restrict__ off, int n_rows, const int* __restrict__ src_of,
+          const int* __restrict__ t_start, const int* __restrict__ t_count, const double* __restrict__ t_center,
+          const int* __restrict__ s_start, const int* __restrict__ s_count, const double4* __restrict__ tpos,
+          const double4* __restrict__ spos, const double4* __restrict__ sstr, double* __restrict__ acc13,
+          const int4* __restrict__ items, const int* __restrict__ n_items, double* __restrict__ item_sums,
+          int exact_self) {
   // items (ITEMS, CTA path only), two int4 each: row, first target of the tile, source leaves [z, w); and the place of
   // the item's sums (unscaled) in item_sums, or -1 to add them to the targets
   constexpr int W = kWarps;
@@ -779,7 +778,7 @@ __global__ void __launch_bounds__(kWarps * 32, p2p_min_blocks<R, KIND, HS, RW>()
                   for (int a = 0; a < NA; ++a) tot[k][a] += g2[k == q ? 0 : 1][a];
             }
           } else {
-auto pairs = [&](auto n) {
+            auto pairs = [&](auto n) {
 #pragma unroll 2
               for (int j = slice; j < nb; j += SS) {
                 const double4 b = Bd[j];
@@ -1319,8 +1318,10 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     k_p2p_row_sources<<<rows, per_row <= 64 ? 32 : per_row <= 1024 ? 128 : 1024, 0, st>>>(
         L.dir_off.ptr, L.dir_s.ptr, stt.body_count.ptr, L.p2p_meta.ptr + 1);
     note_launch();
-    k_p2p_plan<sub_tiles<R, KIND, true>() && max_targets_per_lane<R, KIND, HS>() == kTPT><<<1, kPlanThreads, 0, st>>>(L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1,
-                                           goal, NA, (int)sums, max_targets_per_lane<R, KIND, HS>() == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
+    constexpr int KT = max_targets_per_lane<R, KIND, HS>();
+    k_p2p_plan<sub_tiles<R, KIND, true>() && KT == kTPT><<<1, kPlanThreads, 0, st>>>(
+        L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1, goal, NA, (int)sums,
+        KT == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
     note_launch();
     k_p2p<R, KIND, PS, GS, HS, false, true><<<(int)most, kWarps * 32, smem, st>>>(
         L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,

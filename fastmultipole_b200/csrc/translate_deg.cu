@@ -10,10 +10,10 @@
 // after another with its Wigner matrices built per pair: a few hundred warps whose chains of
 // dependent stages set the time.  Whole solves, before -> after: 150k clustered point sources,
 // order 16, tolerance 1e-7: 98.4 -> 10.2 ms; 48k vortex particles, order 16, tolerance 1e-6: 18.0 ->
-// 4.45 ms; 30k vortex ring, order 8: 2.17 -> 1.49 ms (M2M and L2L alone).  Bound now by the FP64 pipe
-// and, at orders above 12, by the shared memory of the rotated degrees (two CTAs per SM).  In FP32
-// (fixed orders of the mixed path) against a kernel with a lane per pair, seven warps per SM: 300k
-// clustered bodies, order 10, M2L 2.04 -> 1.02 ms; 200k vortex ring, order 12, 1.42 -> 0.67 ms.
+// 4.45 ms; 30k vortex ring, order 8: 2.17 -> 1.49 ms (M2M and L2L alone).  The M2L's shared memory
+// lets an SM hold two CTAs up to order 16 and one above.  In FP32 (fixed orders of the mixed path)
+// against a lane per pair: 300k clustered bodies, order 10, M2L 2.04 -> 1.02 ms; 200k vortex ring, order
+// 12, 1.42 -> 0.67 ms.  Rows that are long and even are faster by lanes: m2l_lane.cu has the rule.
 //
 // Rotations about y are factorised as in m2l_lane.cu, with the magnitudes applied outside
 // the two matrix products, so that one constant table of the Wigner matrix at pi/2 serves both
