@@ -141,14 +141,6 @@ __global__ void k_branch_ranges(const int* __restrict__ body_start, const int* _
 
 int grid_for(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 148 * 32)); }
 
-// out += in on rows 4..16 of the target buffer (rows 1..3 are the positions)
-__global__ void k_add_rows(int64_t n, const double* __restrict__ in, double* __restrict__ out) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < 13 * n; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t b = i / 13, r = 3 + i % 13;
-    out[16 * b + r] += in[16 * b + r];
-  }
-}
-
 // adjoint sources: at the targets (or the sources themselves), strengths = cotangents
 __global__ void k_adj_sources(int64_t n, const double* __restrict__ pos, int64_t stride, bool radius_from_pos,
                               const double* __restrict__ dout16, int kind, double* __restrict__ buf) {

@@ -1309,7 +1309,9 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     // (SelfTuning) can be those of other rows too, one of them per level
     const int64_t nest = L.rule_method == FMM_LIST_SELF_TUNING ? tt.n_levels : 1;
     const int64_t most = 3 * (int64_t)rows + nest * tt.n_bodies / (32 * kTPT) + goal + 1;
-    const int64_t sums = (int64_t)2 * goal * 32 * kTPT * NA;
+    // the sums: 64 targets of each of those, and (a share has kItemSources bodies or more) no more than the
+    // pairs allow: 0.5 MB for 2,000 bodies instead of 10
+    const int64_t sums = std::min((int64_t)2 * goal * 32 * kTPT, L.n_pairs / kItemSources + 1) * NA;
     L.p2p_items.grow(2 * (size_t)most);
     L.p2p_meta.grow((size_t)rows + 1);
     L.p2p_part.grow((size_t)sums);
