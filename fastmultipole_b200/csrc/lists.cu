@@ -137,7 +137,7 @@ enum : int {
 };
 static_assert(C_PAIRS % 2 == 0, "the body pairs of the direct list are a 64-bit counter");
 constexpr int kStepThreads = 128;
-constexpr int kStepMinBlocks = 9;  // per SM: 56 registers (62 left alone, eight blocks: 150,001 bodies 459 -> 442 us of traversal)
+constexpr int kStepMinBlocks = 9;  // per SM, 56 registers (62 left alone: 150,001 bodies 459 -> 442 us)
 constexpr int kStepMaxBlocks = 148 * 16;
 
 // Add one to cnt[t] for the lanes that pass, one atomic per distinct target of the warp.
@@ -155,11 +155,10 @@ constexpr int kStepChunk = kStepThreads * kStepItems;      // pairs per block an
 // takes the slots of a whole chunk with one atomic per counter.  Slots past a
 // capacity are not written and raise the flag, which stops the later steps (the
 // host grows the buffers and repeats).
-__global__ void __launch_bounds__(kStepThreads, kStepMinBlocks) k_step(const int2* __restrict__ fin, int2* __restrict__ fout, int k,
-                                                      TreeRef T, TreeRef S, Rule R, int2* __restrict__ rdir,
-                                                      int2* __restrict__ rm2l, int* __restrict__ cdir,
-                                                      int* __restrict__ cm2l, int* __restrict__ ctr, int cap_f,
-                                                      int cap_d, int cap_m) {
+__global__ void __launch_bounds__(kStepThreads, kStepMinBlocks)
+    k_step(const int2* __restrict__ fin, int2* __restrict__ fout, int k, TreeRef T, TreeRef S, Rule R,
+           int2* __restrict__ rdir, int2* __restrict__ rm2l, int* __restrict__ cdir, int* __restrict__ cm2l,
+           int* __restrict__ ctr, int cap_f, int cap_d, int cap_m) {
   constexpr int NW = kStepThreads / 32;
   __shared__ int wsum[3][NW];
   __shared__ int bbase[3];

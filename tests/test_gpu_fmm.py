@@ -107,12 +107,12 @@ CASES = [
                  interaction_list_method=fm.SelfTuning())),
     dict(name="clustered20k_p10", gen=lambda: clustered(20000, 2),
          kw=dict(expansion_order=10, leaf_size_source=64, multipole_acceptance=0.5)),
-    # ~4,000 target rows: the near field's 4-warp CTAs and the one-warp M2L rows (launches of fewer
-    # rows than 4 per SM take wider CTAs, which the smaller cases here exercise)
+    # ~4,000 target rows: one-warp M2L rows (launches of fewer rows than 4 per SM take other kernels)
     dict(name="uniform60k_p4_ls20", gen=lambda: uniform(60000, 31), kw=dict(expansion_order=4, leaf_size_source=20,
                                                                            multipole_acceptance=0.5,
                                                                            scalar_potential=True)),
-    # the lane kernel's highest order
+    # nothing is well separated in leaves of this size: order 12 of the upward pass, near field (the
+    # translations of every order and kind of launch are in test_gpu_translations.py)
     dict(name="uniform6k_p12", gen=lambda: uniform(6000, 8), kw=dict(expansion_order=12, leaf_size_source=40,
                                                                      multipole_acceptance=0.5,
                                                                      scalar_potential=True)),
@@ -170,8 +170,8 @@ def test_vortex_low_order_and_large_leaves(ctx, p, ls):
 
 @pytest.mark.parametrize("p", [4, 6, 9, 10])
 def test_vortex_lane_m2l_orders_match_oracle(ctx, p):
-    # plain vortex M2L from order 4 runs the lane-per-pair Lamb-Helmholtz kernel, one template
-    # instance per order; degrees >= 8 stage more rows than a warp has lanes
+    # plain vortex M2L from order 4, uneven rows (the degree-parallel kernel); degrees >= 8 stage more
+    # rows than a warp has lanes
     buf = ring(8000, 10 + p)
     og, oo = opt_pair(expansion_order=p, leaf_size_source=30, multipole_acceptance=0.5, hessian=True)
     out, res = fm.solve_buffers(buf, L.FMM_POINT_VORTEX, og, ctx=ctx)
@@ -204,7 +204,7 @@ def test_many_rows_vortex_and_mixed(ctx):
 
 def test_chunked_near_field_probes_match_oracle(ctx):
     # 10,000 probes around 200,000 sources: 456 target rows, a few of them with most of the pairs,
-    # so the near field cuts the rows into chunks of source leaves (summed in chunk order)
+    # so the near field cuts the rows into items of a tile's targets and a share of the source leaves
     rng = np.random.default_rng(4)
     buf = uniform(200000, 41)
     probes = np.ascontiguousarray(-0.5 + 2.0 * rng.random((10000, 3)))
@@ -235,9 +235,8 @@ def test_mixed_vortex_matches_f64(ctx):
 
 @pytest.mark.parametrize("p", [4, 12])
 def test_mixed_vortex_far_field_matches_f64(ctx, p):
-    # far field only: the mixed path's lane-per-pair Lamb-Helmholtz M2L (FP32 rotations of
-    # scaled multipoles) against its FP64 instance (pinned to the oracle above), velocity and
-    # velocity gradient
+    # far field only: the mixed path's Lamb-Helmholtz M2L (FP32 rotations of scaled multipoles) against
+    # its FP64 form (pinned to the oracle above), velocity and velocity gradient
     buf = ring(30000, 9)
     outs = {}
     for prec in ("f64", "mixed"):

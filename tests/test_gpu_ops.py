@@ -1,6 +1,7 @@
 """GPU single-operator parity: the reference test suite's golden vectors through the
 C ABI's fmm_op_* entry points (device kernels), plus agreement with the FP64 oracle
-on random inputs at the orders the configurations use."""
+on random inputs at the orders the configurations use.  (These operators have kernels of their
+own; the translations of a solve are compared in test_gpu_translations.py.)"""
 import ctypes as C
 import json
 import os
