@@ -48,11 +48,12 @@ struct Workspace {
 // it has its own, the far field: the single addition the L2P makes when it accumulates into the
 // near-field rows itself) after the position.  Bound by the traffic: 1e6 bodies 146 us with a thread
 // per body, whose rows lay 104 and 128 bytes apart.
-// undefined (may be null): a centre of the tree, when the downward pass of the requested rows (mask) was
-// left out because nothing was translated: a position that is not a number gives NaN there too.
+// LEFT_OUT: the downward pass of the requested rows (mask) was left out because nothing was translated; a
+// position that is not a number (centre: one of the tree) gives NaN there too.
+template <bool LEFT_OUT = false>
 __global__ void k_unsort(const double* __restrict__ acc13, const int* __restrict__ sort_index,
                          const double4* __restrict__ pos, int64_t n, double* __restrict__ out16,
-                         const double* __restrict__ far = nullptr, const double* __restrict__ undefined = nullptr,
+                         const double* __restrict__ far = nullptr, const double* __restrict__ centre = nullptr,
                          unsigned mask = 0) {
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < 16 * n; e += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = e >> 4;
@@ -63,9 +64,9 @@ __global__ void k_unsort(const double* __restrict__ acc13, const int* __restrict
     } else {
       v = acc13[13 * i + r - 3];
       if (far) v += far[13 * i + r - 3];
-      if (undefined && ((mask >> r) & 1u)) {
+      if (LEFT_OUT && ((mask >> r) & 1u)) {
         const double4 p = pos[i];
-        v += 0.0 * (p.x - undefined[0]) + 0.0 * (p.y - undefined[1]) + 0.0 * (p.z - undefined[2]);
+        v += 0.0 * (p.x - centre[0]) + 0.0 * (p.y - centre[1]) + 0.0 * (p.z - centre[2]);
       }
     }
     out16[16 * (int64_t)(sort_index ? sort_index[i] : i) + r] = v;
@@ -596,11 +597,13 @@ void run_fmm(fmm_ctx* c, Workspace& W, const SolveIn& in, const fmm_options& o, 
   if (is_estimate)  // out16 receives |grad| per body (n doubles)
     k_unsort_gradnorm<<<grid_for(T.n_bodies), 256, 0, st>>>(W.acc13.ptr, T.sort_index.ptr, T.n_bodies, out16,
                                                              influence_potential ? 1 : 0);
-  else
-    k_unsort<<<grid_for(16 * T.n_bodies), 256, 0, st>>>(
-        W.acc13.ptr, T.sort_index.ptr, T.pos.ptr, T.n_bodies, out16, split ? far13 : nullptr,
-        o.downward_pass && !translated ? T.tcenter.ptr : nullptr,
+  else if (o.downward_pass && !translated)
+    k_unsort<true><<<grid_for(16 * T.n_bodies), 256, 0, st>>>(
+        W.acc13.ptr, T.sort_index.ptr, T.pos.ptr, T.n_bodies, out16, split ? far13 : nullptr, T.tcenter.ptr,
         (ps ? 0x8u : 0u) | (gs ? 0x70u : 0u) | (hs ? 0xff80u : 0u));
+  else
+    k_unsort<><<<grid_for(16 * T.n_bodies), 256, 0, st>>>(W.acc13.ptr, T.sort_index.ptr, T.pos.ptr, T.n_bodies, out16,
+                                                          split ? far13 : nullptr);
   FMM_CUDA_TRY(cudaGetLastError());
   mark(7);
   if (copy_out) FMM_CUDA_TRY(cudaMemcpyAsync(copy_out, out16, 16 * T.n_bodies * sizeof(double), copy_kind, st));
@@ -1167,7 +1170,7 @@ int fmm_direct(fmm_ctx* c, const fmm_target_system* target, const fmm_source_sys
     (void)ps;
     c->out16.grow(16 * (size_t)nt + 1);
     note_launch();
-    k_unsort<<<grid_for(16 * nt), 256, 0, c->stream>>>(c->main.acc13.ptr, nullptr, T.pos.ptr, nt, c->out16.ptr);
+    k_unsort<><<<grid_for(16 * nt), 256, 0, c->stream>>>(c->main.acc13.ptr, nullptr, T.pos.ptr, nt, c->out16.ptr);
     FMM_CUDA_TRY(cudaGetLastError());
     auto kind = target->memory == FMM_MEMORY_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
     FMM_CUDA_TRY(cudaMemcpyAsync(target->out, c->out16.ptr, 16 * nt * sizeof(double), kind, c->stream));
