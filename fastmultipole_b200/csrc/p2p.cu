@@ -58,6 +58,10 @@ constexpr int kItemRowsPerSM = 64, kItemWaves = 4, kItemSources = 256;
 // of 20,000 (up to 210,000) 0.129 / 0.082; 512 even rows of 27,000 0.070 / 0.091, mixed 0.100 / 0.095; 64 rows of
 // 62,000, vortex particles, 0.10 / 0.07; 574 rows of 80,000 0.24 / 0.16; one row of 1.6e6 1.28 / 0.09.
 constexpr double kItemRowPairs = 1.6e4;
+// A body's gathering into a batch, in target slots of its pairs.  Without it the second tile of a row of 68
+// targets got a sixteenth of the shares of the first and took the longest: 4,333 probes and 189,460 vortex
+// particles, mixed, near field 2.25 ms, 1.42 with it (1.41 and 1.45 with two and four times as many slots)
+constexpr int kGatherSlotsF32 = 16, kGatherSlotsF64 = 4;
 constexpr int kTPT = 2;
 constexpr unsigned kAll = 0xffffffffu;
 
@@ -1134,12 +1138,13 @@ __global__ void k_p2p_row_sources(const int* __restrict__ off, const int* __rest
   if (threadIdx.x == 0) n_src[blockIdx.x] = sum;
 }
 
-// target slots that a tile of nt targets occupies (three: the FP64 kernels' choice of targets per lane)
-__device__ __forceinline__ int tile_slots(int nt, bool three) {
+// what a source body costs a tile of nt targets, in target slots: those that the tile occupies (three: the
+// FP64 kernels' choice of targets per lane) and its gathering (gather)
+__device__ __forceinline__ int tile_cost(int nt, bool three, int gather) {
   const int tpt = three ? targets_per_lane(nt) : kTPT;
   int ts = 1;
   while (ts * tpt < nt) ts <<= 1;
-  return ts * tpt;
+  return ts * tpt + gather;
 }
 
 // The items of a launch, one block: every tile of a row is cut into shares of about the launch's
@@ -1151,7 +1156,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
                                                            const int* __restrict__ off, int rows,
                                                            const int* __restrict__ t_count,
                                                            const int* __restrict__ n_src, int goal, int na,
-                                                           int max_sums, int three, int4* __restrict__ items,
+                                                           int max_sums, int three, int gather, int4* __restrict__ items,
                                                            int* __restrict__ n_items) {
   __shared__ unsigned long long tot[kPlanThreads / 32];
   __shared__ int2 sh[kPlanThreads / 32];
@@ -1162,7 +1167,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
     int slots = 0;
     for (int t = 0, nt; t < tc; t += nt) {
       nt = next_tile<SUB>(tc - t);
-      slots += tile_slots(nt, three != 0);
+      slots += tile_cost(nt, three != 0, gather);
     }
     work += (unsigned long long)slots * (unsigned)n_src[r];
   }
@@ -1184,7 +1189,7 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       nl = off[r + 1] - a;
     }
     auto cut = [&](int nt) {
-      const unsigned long long c = ((unsigned long long)tile_slots(nt, three != 0) * (unsigned)ns + share - 1) / share;
+      const unsigned long long c = ((unsigned long long)tile_cost(nt, three != 0, gather) * (unsigned)ns + share - 1) / share;
       return (int)max(1ull, min(c, (unsigned long long)min(nl, ns / kItemSources)));
     };
     int2 v = make_int2(0, 0);
@@ -1323,7 +1328,7 @@ void run_p2p(const DevTree& tt, const DevTree& stt, DevLists& L, double* acc13, 
     constexpr int KT = max_targets_per_lane<R, KIND, HS>();
     k_p2p_plan<sub_tiles<R, KIND, true>() && KT == kTPT><<<1, kPlanThreads, 0, st>>>(
         L.dir_tgt.ptr, L.dir_off.ptr, rows, tt.body_count.ptr, L.p2p_meta.ptr + 1, goal, NA, (int)sums,
-        KT == 3 ? 1 : 0, L.p2p_items.ptr, L.p2p_meta.ptr);
+        KT == 3 ? 1 : 0, sizeof(R) == 4 ? kGatherSlotsF32 : kGatherSlotsF64, L.p2p_items.ptr, L.p2p_meta.ptr);
     note_launch();
     k_p2p<R, KIND, PS, GS, HS, false, true><<<(int)most, kWarps * 32, smem, st>>>(
         L.dir_tgt.ptr, L.dir_off.ptr, rows, L.dir_s.ptr, tt.body_start.ptr, tt.body_count.ptr, tt.tcenter.ptr,
