@@ -1152,12 +1152,10 @@ __device__ __forceinline__ int tile_cost(int nt, bool three, int gather) {
 // cut, and with it the order of every sum, depends on the tree and the lists alone.
 constexpr int kPlanThreads = 1024;
 template <bool SUB>
-__global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict__ tgt_list,
-                                                           const int* __restrict__ off, int rows,
-                                                           const int* __restrict__ t_count,
-                                                           const int* __restrict__ n_src, int goal, int na,
-                                                           int max_sums, int three, int gather, int4* __restrict__ items,
-                                                           int* __restrict__ n_items) {
+__global__ void __launch_bounds__(kPlanThreads)
+    k_p2p_plan(const int* __restrict__ tgt_list, const int* __restrict__ off, int rows, const int* __restrict__ t_count,
+               const int* __restrict__ n_src, int goal, int na, int max_sums, int three, int gather,
+               int4* __restrict__ items, int* __restrict__ n_items) {
   __shared__ unsigned long long tot[kPlanThreads / 32];
   __shared__ int2 sh[kPlanThreads / 32];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -1189,7 +1187,8 @@ __global__ void __launch_bounds__(kPlanThreads) k_p2p_plan(const int* __restrict
       nl = off[r + 1] - a;
     }
     auto cut = [&](int nt) {
-      const unsigned long long c = ((unsigned long long)tile_cost(nt, three != 0, gather) * (unsigned)ns + share - 1) / share;
+      const unsigned long long cost = (unsigned long long)tile_cost(nt, three != 0, gather) * (unsigned)ns;
+      const unsigned long long c = (cost + share - 1) / share;
       return (int)max(1ull, min(c, (unsigned long long)min(nl, ns / kItemSources)));
     };
     int2 v = make_int2(0, 0);
