@@ -60,7 +60,8 @@ constexpr int kItemRowsPerSM = 64, kItemWaves = 4, kItemSources = 256;
 constexpr double kItemRowPairs = 1.6e4;
 // A body's gathering into a batch, in target slots of its pairs.  Without it the second tile of a row of 68
 // targets got a sixteenth of the shares of the first and took the longest: 4,333 probes and 189,460 vortex
-// particles, mixed, near field 2.25 ms, 1.42 with it (1.41 and 1.45 with two and four times as many slots)
+// particles, gradients on, mixed: near field 2.25 ms, 1.42 with it (1.41 and 1.45 with two and four times as
+// many slots); gradients off 1.13 and 0.78
 constexpr int kGatherSlotsF32 = 16, kGatherSlotsF64 = 4;
 constexpr int kTPT = 2;
 constexpr unsigned kAll = 0xffffffffu;
